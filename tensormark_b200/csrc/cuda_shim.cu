@@ -241,7 +241,7 @@ bool tm_cuda_gemv_q(const float* x, const void* W, float* y, unsigned N, unsigne
     // then copies that image instead of staging x in every CTA. Pageable x takes the copy.
     {
         cudaPointerAttributes ax;
-        const size_t img = xq_bytes(K, dtype);
+        const size_t img = wb / N % 16 == 0 ? xq_bytes(K, dtype) : 0;      // rows off the 16-byte grid are multiplied by a finer image, made in the CTAs
         if (img && cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost && ax.devicePointer &&
             (uintptr_t)ax.devicePointer % 16 == 0) {
             uint32_t* xq = (uint32_t*)s.io_xq.get(img);

@@ -15,7 +15,8 @@
 //     the grid or on whether it was reached through a segment table: the segmented launch is bit-identical to separate
 //     launches (the property tensormark/metal.h:504-510 requires).
 //   * Rows that start on any even address are served: a row's copy starts at the 16-byte boundary below it and the
-//     lanes read from the remainder on (AL = false). Odd addresses and TQ2 take gemv_generic, a plain byte-granular
+//     lanes read from the remainder on (AL = false). Such rows used to be multiplied by x in fp32; here x keeps four
+//     planes for them, which holds an fp32 x to its last bits. Odd addresses and TQ2 take gemv_generic, a plain byte-granular
 //     kernel with the same per-row arithmetic contract (tolerance-level, not bitwise, agreement).
 #include "common.cuh"
 #include "gemv_tile.cuh"
@@ -68,7 +69,7 @@ template <int CDT>
 __device__ __forceinline__ void stage_vector(uint32_t* out, const float* x, const float* x2, uint32_t x_op, float eps, uint32_t K, float* red) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const uint32_t ngroups = (K + 255u) / 256u;
-    float ss = stage_groups<CDT>(out + kXqHeaderWords, x, x2, x_op, K, (uint32_t)warp, ngroups, (uint32_t)nwarps, lane);
+    float ss = stage_groups<CDT>(out + kXqHeaderWords, nullptr, x, x2, x_op, K, (uint32_t)warp, ngroups, (uint32_t)nwarps, lane);
     if (x_op == 1u) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -100,13 +101,13 @@ __global__ void __launch_bounds__(512) xprep_kernel(uint32_t* out, const float* 
     if (gridDim.x == 1) { stage_vector<CDT>(out, x, x2, x_op, eps, K, red); return; }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const uint32_t ngroups = (K + 255u) / 256u, g = blockIdx.x * nwarps + warp;
-    if (g < ngroups) (void)stage_groups<CDT>(out + kXqHeaderWords, x, x2, x_op, K, g, g + 1, 1u, lane);
+    if (g < ngroups) (void)stage_groups<CDT>(out + kXqHeaderWords, nullptr, x, x2, x_op, K, g, g + 1, 1u, lane);
     if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = __float_as_uint(1.0f);
 }
 
 
 // Shared memory: [x image and a group of zeros][the ring's barriers][ring].
-inline uint32_t fixed_smem(const TileGeom& g) { return x_image_bytes(g.ngroups) + kRingBarBytes; }
+__host__ __device__ inline uint32_t x_smem(const TileGeom& g, bool aligned) { return x_image_bytes(g.ngroups) * (aligned ? 1u : 2u); }
 static_assert(kRingBarBytes % 128 == 0, "the ring starts on a 128-byte boundary");
 
 template <int DT, bool AL>
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
     const TileGeom ge = p.ge;
     uint32_t* img = reinterpret_cast<uint32_t*>(smem);
     Ring rg;
-    rg.bars = smem_base(smem) + x_image_bytes(ge.ngroups);
+    rg.bars = smem_base(smem) + x_smem(ge, AL);
     rg.at = rg.bars + kRingBarBytes;
     rg.slots = p.slots; rg.slot_bytes = ge.slot_bytes; rg.gone = &gone;
     const uint32_t cta_lo = min(p.N, blockIdx.x * p.rows_per_cta), rows = min(p.N, cta_lo + p.rows_per_cta) - cta_lo;
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
                 ok = mbar_wait(xb, 0, &gone);
             }
         } else {
-            float ss = stage_groups<DT>(img, p.x, p.x2, p.x_op, p.K, (uint32_t)warp, ge.ngroups, (uint32_t)kConsumers, lane);
+            float ss = stage_groups<DT, !AL>(img, img + x_image_bytes(ge.ngroups) / 4u, p.x, p.x2, p.x_op, p.K, (uint32_t)warp, ge.ngroups, (uint32_t)kConsumers, lane);
             if (p.x_op == 1u) {
 #pragma unroll
                 for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -436,8 +437,10 @@ template <int DT> bool launch_generic_only(GemvParams p, cudaStream_t st);
 template <int DT>
 bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st) {
     p.ge = tile_geom(DT, p.K, aligned);
-    const uint32_t fixed = fixed_smem(p.ge);
-    // a slot per producer at least: a longer x than that (some 40000 activations) leaves no room for the ring
+    const uint32_t fixed = x_smem(p.ge, aligned) + kRingBarBytes;
+    if (!aligned) p.xq = nullptr;                           // such an image has two planes
+    // a slot per producer at least: a longer x than that (some 40000 activations, half as many where x has four planes)
+    // leaves no room for the ring
     if (even && fixed + p.ge.producers * p.ge.slot_bytes <= kSmemLimit) {
         const unsigned sms = (unsigned)device_sm_count();
         // as many CTAs as SMs, rows spread evenly: with one CTA per SM the longest range is the launch's time

@@ -139,6 +139,13 @@ __device__ __forceinline__ void quantize_quad(float x, float y, float z, float w
     const uint32_t f = (__byte_perm(p01, p23, 0x6420) & 0x7F7F7F7Fu) ^ 0x40404040u;      // a2 in seven bits, two's complement
     q2 = f | ((f & 0x40404040u) << 1);
 }
+// Two more planes: what rounding to multiples of s / 128 left, in multiples of s / 2^21: x ~= s (a1 + a2/128 + a3/2^14 +
+// a4/2^21), as close as fp32 holds x.
+__device__ __forceinline__ void quantize_rest(float x, float y, float z, float w, float inv, uint32_t& q3, uint32_t& q4) {
+    const float s = inv * 128.0f, magic = 12582912.0f;
+    auto rest = [&](float v) { const float t = __fmul_rn(v, s); return __fmul_rn(__fadd_rn(t, -__fadd_rn(__fadd_rn(t, magic), -magic)), 128.0f); };   // exact, |rest| <= 64
+    quantize_quad(rest(x), rest(y), rest(z), rest(w), 1.0f, q3, q4);
+}
 #endif
 
 // Loads of weight bytes. On the GPU the bytes lie in shared memory and an address is the 32-bit one (SPtr): generic
@@ -276,8 +283,8 @@ template <> struct Lane<0> : LanePairs<272, false> {
     static constexpr TM_HD int xw(int k) { return 8 * k; }
     static TM_HD void merge(const int (&c)[2], int, int (&S)[2]) { S[0] = c[0]; S[1] = c[1]; }
     static TM_HD void mask(Meta& m, int nvalid) { mask_d(m.d, nvalid); }
-    static TM_HD float combine(const int (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
-        return fma1(m.d[1], xs.y * (float)S[1], fma1(m.d[0], xs.x * (float)S[0], acc));
+    static TM_HD float combine(const float (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
+        return fma1(m.d[1], xs.y * S[1], fma1(m.d[0], xs.x * S[0], acc));
     }
     TM_LANE_HOST(0)
 };
@@ -311,8 +318,8 @@ template <> struct Lane<1> : LanePairs<144, true> {
     static constexpr TM_HD int xw(int k) { return 4 * k; }
     static TM_HD void merge(const int (&c)[4], int, int (&S)[2]) { S[0] = c[0] * 16 + c[1]; S[1] = c[2] * 16 + c[3]; }
     static TM_HD void mask(Meta& m, int nvalid) { mask_d(m.d, nvalid); }
-    static TM_HD float combine(const int (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
-        return fma1(m.d[1], fma1(xs.y, (float)S[1], xs.w), fma1(m.d[0], fma1(xs.x, (float)S[0], xs.z), acc));
+    static TM_HD float combine(const float (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
+        return fma1(m.d[1], fma1(xs.y, S[1], xs.w), fma1(m.d[0], fma1(xs.x, S[0], xs.z), acc));
     }
     TM_LANE_HOST(1)
 };
@@ -353,9 +360,9 @@ template <> struct Lane<4> : LanePairs<160, true> {
     static constexpr TM_HD int xw(int k) { return 4 * k; }
     static TM_HD void merge(const int (&c)[4], int, int (&S)[2]) { S[0] = c[0] * 16 + c[1]; S[1] = c[2] * 16 + c[3]; }
     static TM_HD void mask(Meta& m, int nvalid) { mask_d(m.d, nvalid); mask_d(m.m, nvalid); }
-    static TM_HD float combine(const int (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
-        acc += fma1(m.d[0] * xs.x, (float)S[0], m.m[0] * xs.z);
-        return acc + fma1(m.d[1] * xs.y, (float)S[1], m.m[1] * xs.w);
+    static TM_HD float combine(const float (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
+        acc += fma1(m.d[0] * xs.x, S[0], m.m[0] * xs.z);
+        return acc + fma1(m.d[1] * xs.y, S[1], m.m[1] * xs.w);
     }
     TM_LANE_HOST(4)
 };
@@ -411,9 +418,9 @@ template <> struct Lane<5> : LanePairs<176, true> {
         S[1] = c[1] + (c[3] >> (2 * t + 1)) * 256;
     }
     static TM_HD void mask(Meta&, int) {}                    // rows are whole super-blocks
-    static TM_HD float combine(const int (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
-        acc = fma1(m.d[0] * xs.x, (float)S[0], fma1(-m.m[0], xs.z, acc));
-        return fma1(m.d[1] * xs.y, (float)S[1], fma1(-m.m[1], xs.w, acc));
+    static TM_HD float combine(const float (&S)[2], const Meta& m, const float4 xs, const float4, float acc) {
+        acc = fma1(m.d[0] * xs.x, S[0], fma1(-m.m[0], xs.z, acc));
+        return fma1(m.d[1] * xs.y, S[1], fma1(-m.m[1], xs.w, acc));
     }
     TM_LANE_HOST(5)
 };
@@ -486,11 +493,11 @@ template <> struct Lane<6> {
         S[0] = c[0] + c[1] * 16; S[1] = c[2] + c[3] * 4; S[2] = c[4] + c[5] * 16; S[3] = c[6] + c[7] * 4;
     }
     static TM_HD void mask(Meta&, int) {}
-    static TM_HD float combine(const int (&S)[4], const Meta& m, const float4 xs, const float4 xz, float acc) {
-        float v = m.s[0] * fma1(xs.x, (float)S[0], xz.x);
-        v = fma1(m.s[1], fma1(xs.y, (float)S[1], xz.y), v);
-        v = fma1(m.s[2], fma1(xs.z, (float)S[2], xz.z), v);
-        v = fma1(m.s[3], fma1(xs.w, (float)S[3], xz.w), v);
+    static TM_HD float combine(const float (&S)[4], const Meta& m, const float4 xs, const float4 xz, float acc) {
+        float v = m.s[0] * fma1(xs.x, S[0], xz.x);
+        v = fma1(m.s[1], fma1(xs.y, S[1], xz.y), v);
+        v = fma1(m.s[2], fma1(xs.z, S[2], xz.z), v);
+        v = fma1(m.s[3], fma1(xs.w, S[3], xz.w), v);
         return fma1(m.d, v, acc);
     }
     TM_LANE_HOST(6)
@@ -521,42 +528,55 @@ __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, ui
 // column's quarter is this thread's k range, a group of zeros otherwise; xf: its quarter's eight floats.
 struct XRegs { uint4 b[4]; float4 xs, xz; };
 __device__ __forceinline__ float4 ld_f4(SPtr p) { const uint4 v = ld16(p); return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
-template <int DT> __device__ __forceinline__ void load_x(XRegs& x, SPtr xb, SPtr xf) {
+template <int DT, bool FINE> __device__ __forceinline__ void load_x(XRegs& x, SPtr xb, SPtr xf) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x.b[k] = ld16(xb + 128 * k);
+    for (int k = 0; k < 4; ++k) if (!FINE) x.b[k] = ld16(xb + 128 * k);
     x.xs = ld_f4(xf);
     if (Lane<DT>::NR == 4) x.xz = ld_f4(xf + 16);
 }
 // Quarter t of rows g (r0: the quarter's bytes, quarter_off) and g + 8 (r1) of the tile times one group: their two
 // partial sums. nvalid: 32-blocks of this quarter that exist (2, but for the last group of a row that is no multiple of
-// 256).
-template <int DT, bool AL>
-__device__ __forceinline__ void group_dot(SPtr r0, SPtr r1, const XRegs& x, int t, int nvalid,
-                                          float& acc0, float& acc1) {
+// 256). FINE: four planes of x, the B operands at xb and, of the second pair, at fine (registers are too few to hold them).
+template <int DT, bool AL, bool FINE>
+__device__ __forceinline__ void group_dot(SPtr r0, SPtr r1, const XRegs& x, SPtr xb, SPtr fine, int t, int nvalid, float& acc0, float& acc1) {
     using L = Lane<DT>;
     uint32_t w0[L::NRAW], w1[L::NRAW];
     typename L::Meta m0, m1;
     L::template load<AL>(r0, t, w0, m0);
     L::template load<AL>(r1, t, w1, m1);
-    int s0[L::NACC], s1[L::NACC], S0[L::NR], S1[L::NR];
+    float f0[L::NR], f1[L::NR];
+    auto planes = [&](auto operand, bool rest) {             // operand(i): B words of MMA pair i (two MMAs)
+        int s0[L::NACC], s1[L::NACC], S0[L::NR], S1[L::NR];
 #pragma unroll
-    for (int k = 0; k < L::NACC; ++k) {
-        int c[4];
+        for (int k = 0; k < L::NACC; ++k) {
+            int c[4];
 #pragma unroll
-        for (int i = 0; i < L::MPA; ++i) {
-            const uint4 b = x.b[(L::xw(k) + 2 * i) / 4];
-            const uint32_t b0 = i & 1 ? b.z : b.x, b1 = i & 1 ? b.w : b.y;      // xw(k) is a multiple of 4
-            const uint32_t p = L::code(w0, k, 2 * i, t), q = L::code(w1, k, 2 * i, t), r = L::code(w0, k, 2 * i + 1, t), s = L::code(w1, k, 2 * i + 1, t);
-            if (i == 0) mma_i8<L::SIGNED, true>(c, p, q, r, s, b0, b1);
-            else mma_i8<L::SIGNED, false>(c, p, q, r, s, b0, b1);
+            for (int i = 0; i < L::MPA; ++i) {
+                const uint4 b = operand((L::xw(k) + 2 * i) / 4);
+                const uint32_t b0 = i & 1 ? b.z : b.x, b1 = i & 1 ? b.w : b.y;      // xw(k) is a multiple of 4
+                const uint32_t p = L::code(w0, k, 2 * i, t), q = L::code(w1, k, 2 * i, t), r = L::code(w0, k, 2 * i + 1, t), s = L::code(w1, k, 2 * i + 1, t);
+                if (i == 0) mma_i8<L::SIGNED, true>(c, p, q, r, s, b0, b1);
+                else mma_i8<L::SIGNED, false>(c, p, q, r, s, b0, b1);
+            }
+            s0[k] = c[0] * 128 + c[1]; s1[k] = c[2] * 128 + c[3];
         }
-        s0[k] = c[0] * 128 + c[1]; s1[k] = c[2] * 128 + c[3];
+        L::merge(s0, t, S0);
+        L::merge(s1, t, S1);
+#pragma unroll
+        for (int r = 0; r < L::NR; ++r) {
+            f0[r] = rest ? fmaf((float)S0[r], 1.0f / 16384.0f, f0[r]) : (float)S0[r];
+            f1[r] = rest ? fmaf((float)S1[r], 1.0f / 16384.0f, f1[r]) : (float)S1[r];
+        }
+    };
+    if constexpr (FINE) {
+        planes([&](int i) { return ld16(xb + 128 * i); }, false);
+        planes([&](int i) { return ld16(fine + 128 * i); }, true);
+    } else {
+        planes([&](int i) { return x.b[i]; }, false);
     }
-    L::merge(s0, t, S0);
-    L::merge(s1, t, S1);
     if (nvalid < 2) { L::mask(m0, nvalid); L::mask(m1, nvalid); }
-    acc0 = L::combine(S0, m0, x.xs, x.xz, 0.f);
-    acc1 = L::combine(S1, m1, x.xs, x.xz, 0.f);
+    acc0 = L::combine(f0, m0, x.xs, x.xz, 0.f);
+    acc1 = L::combine(f1, m1, x.xs, x.xz, 0.f);
 }
 #else
 // What thread t of a row computes, without the tensor core.
@@ -575,9 +595,11 @@ template <int DT> float LaneHost<DT>::dot(const uint8_t* quarter, const uint32_t
         }
     }
     L::merge(c, t, S);
+    float f[L::NR];
+    for (int r = 0; r < L::NR; ++r) f[r] = (float)S[r];
     const float4 xs = {as_float(w[32]), as_float(w[33]), as_float(w[34]), as_float(w[35])};
     const float4 xz = {as_float(w[36]), as_float(w[37]), as_float(w[38]), as_float(w[39])};
-    return L::combine(S, m, xs, xz, 0.f);
+    return L::combine(f, m, xs, xz, 0.f);
 }
 // The x words of quarter u % 4 of group u / 4 in MMA order: plane 0, plane 1, then the eight floats.
 template <int DT> void load_x_unit(typename Lane<DT>::X& x, const uint32_t* units, uint32_t u) {

@@ -158,10 +158,10 @@ __device__ __forceinline__ void row_sum(SPtr pa, SPtr pb, uint32_t n, float& a, 
 // shuffle stages, the plane bytes leave as packed stores. A warp stages eight blocks (one group) per pass; it takes
 // groups g_first, g_first + g_step, ... below g_end. `units` is shared memory (a CTA staging for itself) or global
 // memory (staging once for every CTA of a later launch). Blocks past K inside the last group are staged as zeros.
-// Returns this lane's share of sum(x^2) for x_op 1 (RMSNorm: x * w is staged, the factor rsqrt(mean(x^2) + eps) is one
+// FINE: two more planes, into an image of their own at `fine`. Returns this lane's share of sum(x^2) for x_op 1 (RMSNorm: x * w is staged, the factor rsqrt(mean(x^2) + eps) is one
 // number for the whole vector and multiplies the finished row sums instead); x_op 2 stages silu(x) * x2.
-template <int DT>
-__device__ __forceinline__ float stage_groups(uint32_t* units, const float* x, const float* x2, uint32_t x_op, uint32_t K,
+template <int DT, bool FINE = false>
+__device__ __forceinline__ float stage_groups(uint32_t* units, uint32_t* fine, const float* x, const float* x2, uint32_t x_op, uint32_t K,
                                               uint32_t g_first, uint32_t g_end, uint32_t g_step, int lane) {
     using L = Lane<DT>;
     constexpr int B = 2;
@@ -223,6 +223,11 @@ __device__ __forceinline__ float stage_groups(uint32_t* units, const float* x, c
             quantize_quad(v[j].x, v[j].y, v[j].z, v[j].w, inv, q1, q2);
             L::store_quad(units, b * 32 + 4 * li, 0, q1);
             L::store_quad(units, b * 32 + 4 * li, 1, q2);
+            if constexpr (FINE) {
+                quantize_rest(v[j].x, v[j].y, v[j].z, v[j].w, inv, q1, q2);
+                L::store_quad(fine, b * 32 + 4 * li, 0, q1);
+                L::store_quad(fine, b * 32 + 4 * li, 1, q2);
+            }
             L::scalars(units, b, (int)(4 * li), (int)li, sc, 0.f, s16[j], s32[j]);
         }
     }
@@ -298,8 +303,8 @@ __device__ __forceinline__ void drain(const Ring& rg) {
     for (uint32_t s = 0; s < rg.slots; ++s) (void)mbar_wait(rg.full(s), 0, rg.gone, 50000000ull), (void)mbar_wait(rg.full(s), 1, rg.gone, 50000000ull);
 }
 
-// Consumer warp: multiplies its groups by x (image at shared address img). mis(row): the low four address bits of a row's
-// first byte (AL = false). The loop is short of issue slots on the 4-bit formats (41 weights per clock and SM at the HBM
+// Consumer warp: multiplies its groups by x (image at shared address img). AL = false: rows on any even address; mis(row)
+// gives the low four bits of a row's first byte, and x has four planes (a second image behind the first). The loop is short of issue slots on the 4-bit formats (41 weights per clock and SM at the HBM
 // rate), so what it needs is in registers and its control is warp-uniform: a wait, the group, an arrival.
 // ONE: a row is one chunk, so a warp multiplies by the same group throughout and keeps it in registers.
 template <int DT, bool AL, bool ONE, typename Mis>
@@ -309,6 +314,7 @@ __device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, cons
     const uint32_t ngroups = ge.ngroups, nchunks = ONE ? 1u : ge.nchunks, rw = ge.rw, stride8 = 8u * ge.stride, prow8 = 32u * ge.prow;
     const bool column = (g >> 1) == t;                      // this thread's B column belongs to its own k range
     const uint32_t xb0 = img + (column ? wk * kXGroupWords + 4u * g : ngroups * kXGroupWords) * 4u, xb_step = column ? kw * kXGroupWords * 4u : 0u;
+    const uint32_t fine_off = column ? x_image_bytes(ngroups) : 0u;        // AL = false: the second pair of planes
     const uint32_t xf0 = img + (wk * kXGroupWords + 128u + 8u * t) * 4u;
     const uint32_t short_last = L::LANE_UNITS == 2 && (K & 255u) ? ngroups - 1u : ~0u;     // the group with missing blocks
     const uint32_t src0 = rg.at + g * ge.stride + wk * (uint32_t)L::GB + quarter_off<DT>(t);
@@ -316,7 +322,7 @@ __device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, cons
     const uint32_t tiles = (rows + kTileRows - 1) / kTileRows;
     bool ok = true;
     XRegs x;
-    if (ONE) load_x<DT>(x, xb0, xf0);
+    if (ONE) load_x<DT, !AL>(x, xb0, xf0);
     uint32_t tg = 0, c = 0, r = 0, gi = wk, rr = min(rw, tiles);
 #pragma unroll 1
     for (uint32_t left = tiles * nchunks; left; --left) {
@@ -331,9 +337,9 @@ __device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, cons
             }
             int nvalid = 2;
             if (gi == short_last) { const uint32_t nblk = (K & 255u) / 32u; nvalid = (int)min(2u, max(nblk, 2u * t) - 2u * t); }
-            if (!ONE) load_x<DT>(x, xb0 + c * xb_step, xf0 + c * (kw * kXGroupWords * 4u));
+            if (!ONE) load_x<DT, !AL>(x, xb0 + c * xb_step, xf0 + c * (kw * kXGroupWords * 4u));
             float acc0, acc1;
-            group_dot<DT, AL>(r0, r1, x, (int)t, nvalid, acc0, acc1);
+            group_dot<DT, AL, !AL>(r0, r1, x, xb0 + c * xb_step, xb0 + c * xb_step + fine_off, (int)t, nvalid, acc0, acc1);
             st_f(dst0 + at, acc0);
             st_f(dst0 + at + prow8, acc1);
         }
