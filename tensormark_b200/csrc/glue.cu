@@ -4,8 +4,7 @@
 // rmsnorm_row 2408-2434, add_inplace 2444-2449, silu_mul 2450-2455, rope_inplace
 // 2460-2475, rope_k_cache(_h) 2478-2508, v_to_cache(_h) 2509-2528, argmax_f32
 // 2323-2343, sample_gumbel_f32 2349-2379, embed_q4_row 2380-2395, embed_kq_row
-// 1086-1132, tok_bias_qkv 1566-1573, probe_copy 2437-2443, and the GQA split-K
-// decode attention attn_decode_gqa(_h) + attn_decode_combine 2739-2859.
+// 1086-1132, tok_bias_qkv 1566-1573, probe_copy 2437-2443 (the decode attention is in attn_decode.cu).
 // All arithmetic is fp32; K/V rows are rounded to half once, when written.
 #include "common.cuh"
 #include "glue.h"
@@ -278,113 +277,6 @@ __global__ void __launch_bounds__(256) choose_shard_kernel(const float* x, uint3
     }
 }
 
-// ---- GQA split-K decode attention -------------------------------------------------
-// grid (KVH, nsplit), 4 warps. A CTA serves the REP query heads that share one KV
-// head over positions [split*chunk, min(allow, (split+1)*chunk)). Each warp walks
-// its positions with an online softmax; a lane owns dh/32 consecutive dims, so one
-// K or V row is a single coalesced read. The four warps' states are merged in
-// shared memory and the CTA writes one unnormalised partial per query head:
-// part[(split*H + head)*dh + d] and stat[(split*H + head)*2] = (max, sum).
-template <typename T, int DPL, int REP>
-__global__ void __launch_bounds__(128) attn_split_kernel(const float* q, const T* kc,
-                                                          const T* vc, float* part,
-                                                          float* stat, uint32_t H, uint32_t ctx,
-                                                          uint32_t allow, uint32_t chunk, float scale,
-                                                          const int* st) {
-    pdl_enter();
-    constexpr int dh = DPL * 32;
-    if (st) {                                               // chain: attend [0, position] with the grid's fixed split count
-        allow = min((uint32_t)st[0] + 1u, ctx);
-        chunk = (allow + gridDim.y - 1) / gridDim.y;
-    }
-    const uint32_t kv = blockIdx.x, split = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t p0 = split * chunk, p1 = min(allow, p0 + chunk);
-    __shared__ float sm_acc[4][REP][dh];
-    __shared__ float sm_m[4][REP], sm_l[4][REP];
-
-    float qr[REP][DPL];
-#pragma unroll
-    for (int r = 0; r < REP; ++r)
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) qr[r][d] = q[(size_t)(kv * REP + r) * dh + lane * DPL + d] * scale;
-
-    float m[REP], l[REP], acc[REP][DPL];
-#pragma unroll
-    for (int r = 0; r < REP; ++r) {
-        m[r] = -CUDART_INF_F; l[r] = 0.f;
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) acc[r][d] = 0.f;
-    }
-    const T* kbase = kc + (size_t)kv * ctx * dh + lane * DPL;
-    const T* vbase = vc + (size_t)kv * ctx * dh + lane * DPL;
-    for (uint32_t p = p0 + warp; p < p1; p += 4) {
-        float kf[DPL], vf[DPL];
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) { kf[d] = (float)kbase[(size_t)p * dh + d]; vf[d] = (float)vbase[(size_t)p * dh + d]; }
-#pragma unroll
-        for (int r = 0; r < REP; ++r) {
-            float s = 0.f;
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) s = fmaf(qr[r][d], kf[d], s);
-            s = warp_sum(s);
-            const float mn = fmaxf(m[r], s);
-            const float corr = __expf(m[r] - mn), pw = __expf(s - mn);
-            l[r] = l[r] * corr + pw;
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) acc[r][d] = fmaf(acc[r][d], corr, pw * vf[d]);
-            m[r] = mn;
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < REP; ++r) {
-        if (lane == 0) { sm_m[warp][r] = m[r]; sm_l[warp][r] = l[r]; }
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) sm_acc[warp][r][lane * DPL + d] = acc[r][d];
-    }
-    __syncthreads();
-    // merge the four warps: thread t handles dims t, t+128, ... of every head
-    for (int r = 0; r < REP; ++r) {
-        float M = -CUDART_INF_F;
-#pragma unroll
-        for (int w = 0; w < 4; ++w) M = fmaxf(M, sm_m[w][r]);
-        float Lsum = 0.f;
-        float f[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) { f[w] = sm_m[w][r] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][r] - M); Lsum += f[w] * sm_l[w][r]; }
-        const uint32_t head = kv * REP + r;
-        for (int d = threadIdx.x; d < dh; d += 128) {
-            float o = 0.f;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) o += f[w] * sm_acc[w][r][d];
-            part[((size_t)split * H + head) * dh + d] = o;
-        }
-        if (threadIdx.x == 0) { stat[((size_t)split * H + head) * 2] = M; stat[((size_t)split * H + head) * 2 + 1] = Lsum; }
-    }
-}
-
-// out[head][d] = sum_s e^(m_s - M) part_s[d] / sum_s e^(m_s - M) l_s
-__global__ void attn_combine_kernel(const float* part, const float* stat, float* out,
-                                    uint32_t H, uint32_t dh, uint32_t nsplit) {
-    pdl_enter();
-    const uint32_t head = blockIdx.x;
-    float M = -CUDART_INF_F;
-    for (uint32_t s = 0; s < nsplit; ++s) M = fmaxf(M, stat[((size_t)s * H + head) * 2]);
-    float L = 0.f;
-    for (uint32_t s = 0; s < nsplit; ++s) {
-        const float ms = stat[((size_t)s * H + head) * 2];
-        if (ms != -CUDART_INF_F) L += __expf(ms - M) * stat[((size_t)s * H + head) * 2 + 1];
-    }
-    const float invL = 1.0f / L;
-    for (uint32_t d = threadIdx.x; d < dh; d += blockDim.x) {
-        float o = 0.f;
-        for (uint32_t s = 0; s < nsplit; ++s) {
-            const float ms = stat[((size_t)s * H + head) * 2];
-            if (ms != -CUDART_INF_F) o += __expf(ms - M) * part[((size_t)s * H + head) * dh + d];
-        }
-        out[(size_t)head * dh + d] = o * invL;
-    }
-}
-
 // Chain form of rope(q) + rope(k) -> cache + v -> cache in one launch, position read from the chain state.
 // qkv = [q: H*dh | k: KVH*dh | v: KVH*dh]; thread t < (H+KVH)*dh/2 rotates one pair, the rest copy V.
 template <typename T>
@@ -416,22 +308,6 @@ __global__ void qkv_post_kernel(float* qkv, T* kcache, T* vcache, uint32_t H,
 __global__ void advance_kernel(int* st) { pdl_enter(); st[0] += 1; st[1] += 1; st[3] += 1; }   // position, token index, exchange epoch
 
 inline unsigned cdiv(unsigned a, unsigned b) { return (a + b - 1) / b; }
-
-template <typename T, int DPL>
-bool launch_attn_rep(const float* q, const T* kc, const T* vc, float* part, float* stat, unsigned H, unsigned KVH,
-                     unsigned ctx, unsigned allow, unsigned chunk, unsigned nsplit, float scale, unsigned REP,
-                     const int* state, cudaStream_t st) {
-    const dim3 grid(KVH, nsplit);
-    switch (REP) {
-        case 1: launch_pdl(attn_split_kernel<T, DPL, 1>, grid, dim3(128), st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state); break;
-        case 2: launch_pdl(attn_split_kernel<T, DPL, 2>, grid, dim3(128), st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state); break;
-        case 4: launch_pdl(attn_split_kernel<T, DPL, 4>, grid, dim3(128), st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state); break;
-        case 8: launch_pdl(attn_split_kernel<T, DPL, 8>, grid, dim3(128), st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state); break;
-        default: return fail("attention: REP=%u unsupported (1, 2, 4 or 8)", REP);
-    }
-    note_launch();
-    return check_launch("attn_split");
-}
 
 }  // namespace
 
@@ -553,47 +429,6 @@ bool launch_advance(int* state, cudaStream_t st) {
     launch_pdl(advance_kernel, dim3(1), dim3(1), st, state);
     note_launch();
     return check_launch("advance");
-}
-
-AttnPlan plan_attention(unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t probs_bytes) {
-    return plan_attention_sms((unsigned)device_sm_count(), H, KVH, dh, ctx, allow, probs_bytes);
-}
-AttnPlan plan_attention_sms(unsigned sms, unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t probs_bytes) {
-    AttnPlan pl{};
-    // Enough (kv head, split) CTAs to cover the machine; every split at least 32
-    // positions; the partials must fit the caller's probs buffer.
-    unsigned nsplit = cdiv(sms, KVH);
-    nsplit = nsplit < cdiv(allow, 32u) ? nsplit : cdiv(allow, 32u);
-    const size_t per_split = (size_t)H * (dh + 2) * sizeof(float);
-    const unsigned fit = (unsigned)(probs_bytes / per_split);
-    if (fit == 0) { pl.nsplit = 0; return pl; }
-    if (nsplit > fit) nsplit = fit;
-    if (nsplit == 0) nsplit = 1;
-    pl.chunk = cdiv(allow, nsplit);
-    pl.nsplit = cdiv(allow, pl.chunk);
-    pl.part_floats = (size_t)pl.nsplit * H * dh;
-    (void)ctx;
-    return pl;
-}
-
-bool launch_attention(const float* q, const void* kc, const void* vc, bool half_cache, float* scratch, float* out,
-                      unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, float scale, unsigned REP,
-                      const AttnPlan& pl, cudaStream_t st, const int* state) {
-    if (dh != 64 && dh != 128) return fail("attention: head dim %u unsupported (64 or 128)", dh);
-    float* part = scratch;
-    float* stat = scratch + pl.part_floats;
-    bool ok;
-    if (half_cache) {
-        ok = dh == 128 ? launch_attn_rep<__half, 4>(q, (const __half*)kc, (const __half*)vc, part, stat, H, KVH, ctx, allow, pl.chunk, pl.nsplit, scale, REP, state, st)
-                       : launch_attn_rep<__half, 2>(q, (const __half*)kc, (const __half*)vc, part, stat, H, KVH, ctx, allow, pl.chunk, pl.nsplit, scale, REP, state, st);
-    } else {
-        ok = dh == 128 ? launch_attn_rep<float, 4>(q, (const float*)kc, (const float*)vc, part, stat, H, KVH, ctx, allow, pl.chunk, pl.nsplit, scale, REP, state, st)
-                       : launch_attn_rep<float, 2>(q, (const float*)kc, (const float*)vc, part, stat, H, KVH, ctx, allow, pl.chunk, pl.nsplit, scale, REP, state, st);
-    }
-    if (!ok) return false;
-    launch_pdl(attn_combine_kernel, dim3(H), dim3(dh < 128 ? 64 : 128), st, part, stat, out, H, dh, pl.nsplit);
-    note_launch();
-    return check_launch("attn_combine");
 }
 
 }  // namespace tmc

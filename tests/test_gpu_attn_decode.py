@@ -1,0 +1,57 @@
+"""Decode attention over its whole dispatch: heads per K/V head, head dims, cache types, ranges that end inside a stage,
+caches off the 16-byte grid."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tensormark_b200 import lib
+from tests.gpu_util import dev_f32, ptr, stream_ptr
+
+pytestmark = pytest.mark.gpu
+
+
+def run(cuda, torch, orc, KVH, rep, dh, ctx, allow, half, off=0):
+    rng = np.random.default_rng(allow + rep)
+    H, scale = KVH * rep, 1.0 / np.sqrt(dh)
+    q = rng.standard_normal((H, dh)).astype(np.float32) * 2
+    kv = rng.standard_normal((2, KVH, ctx, dh)).astype(np.float16 if half else np.float32)
+    qd = dev_f32(torch, q)
+    flat = [torch.zeros(kv[0].size + 8, dtype=torch.float16 if half else torch.float32, device="cuda") for _ in range(2)]
+    for t, a in zip(flat, kv):
+        t[off:off + a.size] = torch.from_numpy(a.reshape(-1)).cuda()
+    at = [C.c_void_p(t.data_ptr() + off * t.element_size()) for t in flat]
+    need = cuda.tm_cuda_attn_decode_scratch(H, KVH, dh, ctx, allow)
+    scratch = torch.empty(need // 4 + 1, dtype=torch.float32, device="cuda")
+    out = torch.empty(H * dh, dtype=torch.float32, device="cuda")
+    lib.check(cuda.tm_cuda_attn_decode_dev(ptr(qd), at[0], at[1], ptr(scratch), need, ptr(out), H, KVH, dh, ctx, allow, scale,
+                                           int(half), stream_ptr(torch)), "attn_decode_dev")
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(H, dh)
+    K, V = kv[0].astype(np.float32), kv[1].astype(np.float32)
+    for g in range(KVH):
+        want = orc.attn_group(q[g * rep:(g + 1) * rep], K[g, :allow], V[g, :allow], scale)
+        assert np.allclose(got[g * rep:(g + 1) * rep], want, rtol=1e-3, atol=2e-5), (g, np.abs(got[g * rep:(g + 1) * rep] - want).max())
+
+
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("dh", [64, 128])
+@pytest.mark.parametrize("rep", [1, 2, 4, 8])
+def test_heads_dims_types(cuda, torch_mod, orc, rep, dh, half):
+    for allow in (1, 33, 1000):
+        run(cuda, torch_mod, orc, 2, rep, dh, 1024, allow, half)
+
+
+@pytest.mark.parametrize("KVH,rep,allow", [
+    (148, 1, 127), (148, 1, 128), (148, 1, 129), (149, 2, 300), (37, 4, 95), (37, 4, 97), (74, 8, 57), (1, 4, 8191), (8, 4, 8192),
+])
+def test_ranges_around_a_stage(cuda, torch_mod, orc, KVH, rep, allow):
+    run(cuda, torch_mod, orc, KVH, rep, 128, max(allow, 256), allow, True)
+
+
+@pytest.mark.parametrize("half", [False, True])
+def test_caches_off_the_grid(cuda, torch_mod, orc, half):
+    run(cuda, torch_mod, orc, 2, 4, 128, 300, 257, half, off=1)
+    run(cuda, torch_mod, orc, 3, 8, 64, 300, 300, half, off=3)
