@@ -24,7 +24,7 @@
 // rows, one coalesced 128-byte store). The in-kernel dequantizing form keeps one TMA producer and adds
 // eight converting warps.
 //
-// Two forms. The default (gemm_f16_tn, and gemm_f16_tn_pair on CTA pairs for calls of many tiles) takes both
+// Up to 512 tokens the call goes to gemm_blocks.cu, which reads the blocks themselves. The rest has two forms. The default (gemm_f16_tn, and gemm_f16_tn_pair on CTA pairs for calls of many tiles) takes both
 // operands by TMA from an fp16 copy that one pre-pass launch writes to the workspace (weights dequantized
 // exactly and rounded once, activations rounded once). The other (gemm_q4_tn, TM_GEMM_FUSED=1, Q4_0 only) never materialises the fp16 weights: eight
 // producer warps take the rows' 18-byte blocks from a bulk-copied raw ring, turn the nibbles into
@@ -834,102 +834,180 @@ __device__ __forceinline__ void round_activations(const float* __restrict__ A, _
     }
 }
 
-// Both operand conversions of the Q4_0 pre-pass form in one launch. Blocks [0, blocks_w) turn weights into fp16:
-// one item per 32-bit word of codes = eight consecutive weights = one 16-byte store, consecutive threads consecutive
-// words, with the same two-instruction-per-pair arithmetic as the producer warps of gemm_q4_tn (the exact (n - 8) * d
-// rounded once to fp16). The remaining blocks round the activations.
-__global__ void __launch_bounds__(256) prepass_q4_f16(const uint8_t* __restrict__ W, uint32_t row_bytes, __half* __restrict__ Wh,
-                                                      uint32_t N, uint32_t K, const float* __restrict__ A, __half* __restrict__ Ah,
-                                                      size_t n4, uint32_t blocks_w) {
+// Eight consecutive weights of a row (item t of it): the bytes they come from, requested as 16-bit words since blocks are
+// only that aligned, and the fp32 value of each rounded once to fp16. Products of a code and its scale are exact in fp32,
+// and where the code times one half scale is all there is, half arithmetic rounds the same exact product.
+__device__ __forceinline__ uint32_t ld16(const uint8_t* p) { return __ldg(reinterpret_cast<const unsigned short*>(p)); }
+__device__ __forceinline__ uint32_t ld32(const uint8_t* p) { return ld16(p) | (ld16(p + 2) << 16); }
+__device__ __forceinline__ float half_bits(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
+__device__ __forceinline__ uint32_t half_pair(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// (code - BIAS) * d for the four codes in the bytes of q
+template <int BIAS> __device__ __forceinline__ void half_quad(uint32_t q, uint32_t dbits, uint32_t& o01, uint32_t& o23) {
+    const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits)), bias = __half2half2(__ushort_as_half((unsigned short)(0x6400 + BIAS)));
+    uint32_t a = __byte_perm(q, 0x64646464u, 0x5140), b = __byte_perm(q, 0x64646464u, 0x7362);      // 1024 + code in each half
+    __half2 ha = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&a), bias), d2), hb = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&b), bias), d2);
+    o01 = *reinterpret_cast<uint32_t*>(&ha); o23 = *reinterpret_cast<uint32_t*>(&hb);
+}
+template <int DT> struct Eight;
+template <> struct Eight<DT_Q4_0> {
+    uint32_t d, q;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) { const uint8_t* b = row + (size_t)(t >> 2) * 18u; d = ld16(b); q = ld32(b + 2 + 4 * (t & 3u)); }
+    __device__ __forceinline__ uint4 halves() const {
+        const uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;                            // byte j: weights 2j and 2j + 1
+        uint4 o;
+        half_quad<8>(__byte_perm(lo, hi, 0x5140), d, o.x, o.y);
+        half_quad<8>(__byte_perm(lo, hi, 0x7362), d, o.z, o.w);
+        return o;
+    }
+};
+template <> struct Eight<DT_GGUF_Q4_0> {
+    uint32_t d, q0, q1, up;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint8_t* b = row + (size_t)(t >> 2) * 18u;
+        d = ld16(b); q0 = ld32(b + 2 + 8 * (t & 1u)); q1 = ld32(b + 6 + 8 * (t & 1u)); up = 2u * (t & 2u);
+    }
+    __device__ __forceinline__ uint4 halves() const {
+        uint4 o;
+        half_quad<8>((q0 >> up) & 0x0F0F0F0Fu, d, o.x, o.y);
+        half_quad<8>((q1 >> up) & 0x0F0F0F0Fu, d, o.z, o.w);
+        return o;
+    }
+};
+template <> struct Eight<DT_Q8_0> {
+    uint32_t d, q0, q1;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint8_t* b = row + (size_t)(t >> 2) * 34u;
+        d = ld16(b); q0 = ld32(b + 2 + 8 * (t & 3u)); q1 = ld32(b + 6 + 8 * (t & 3u));
+    }
+    __device__ __forceinline__ uint4 halves() const {
+        uint4 o;
+        half_quad<128>(q0 ^ 0x80808080u, d, o.x, o.y);
+        half_quad<128>(q1 ^ 0x80808080u, d, o.z, o.w);
+        return o;
+    }
+};
+__device__ __forceinline__ float byte_float(uint32_t q, int i) { return __uint2float_rn((q >> (8 * i)) & 255u); }
+template <> struct Eight<DT_Q4_1> {
+    uint32_t dm, q0, q1, up;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint8_t* b = row + (size_t)(t >> 2) * 20u;
+        dm = ld32(b); q0 = ld32(b + 4 + 8 * (t & 1u)); q1 = ld32(b + 8 + 8 * (t & 1u)); up = 2u * (t & 2u);
+    }
+    __device__ __forceinline__ uint4 halves() const {
+        const float d = half_bits(dm & 0xffffu), m = half_bits(dm >> 16);
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t c = ((i < 2 ? q0 : q1) >> up) & 0x0F0F0F0Fu;
+            o[i] = half_pair(__fadd_rn(__fmul_rn(byte_float(c, 2 * (i & 1)), d), m), __fadd_rn(__fmul_rn(byte_float(c, 2 * (i & 1) + 1), d), m));
+        }
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    }
+};
+template <bool FIVE> struct EightK {                                     // Q4_K and Q5_K: 32 items per super-block, four per sub-block
+    uint32_t dm, s, m, q0, q1, h0, h1, j;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint8_t* b = row + (size_t)(t >> 5) * (FIVE ? 176u : 144u);
+        j = (t >> 2) & 7u;
+        const uint32_t l = 8u * (t & 3u), hi = j & 4u ? 4u : 0u;
+        dm = ld32(b);
+        s = ld16(b + 4 + ((j + hi) & ~1u));                              // byte j, or byte j + 4 whose low nibble it is
+        m = ld16(b + 4 + ((j + 4u) & ~1u));
+        if (hi) { h0 = ld16(b + 4 + ((j - 4u) & ~1u)); h1 = ld16(b + 4 + (j & ~1u)); }
+        else h0 = h1 = 0;
+        s = (s >> (8 * (j & 1u))) & 255u; m = (m >> (8 * (j & 1u))) & 255u;
+        if (hi) {
+            const uint32_t a = (h0 >> (8 * (j & 1u))) & 255u, c = (h1 >> (8 * (j & 1u))) & 255u;
+            m = (s >> 4) | ((c >> 6) << 4);
+            s = (s & 15u) | ((a >> 6) << 4);
+        } else { s &= 63u; m &= 63u; }
+        const uint8_t* q = b + (FIVE ? 48 : 16) + 32 * (j >> 1) + l;
+        q0 = ld32(q); q1 = ld32(q + 4);
+        if (FIVE) { h0 = ld32(b + 16 + l); h1 = ld32(b + 20 + l); }
+    }
+    __device__ __forceinline__ uint4 halves() const {
+        const float d1 = __fmul_rn(half_bits(dm & 0xffffu), __uint2float_rn(s)), m1 = __fmul_rn(half_bits(dm >> 16), __uint2float_rn(m));
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t c = ((i < 2 ? q0 : q1) >> (4u * (j & 1u))) & 0x0F0F0F0Fu;
+            if (FIVE) c |= (((i < 2 ? h0 : h1) >> j) & 0x01010101u) << 4;
+            o[i] = half_pair(__fsub_rn(__fmul_rn(d1, byte_float(c, 2 * (i & 1))), m1), __fsub_rn(__fmul_rn(d1, byte_float(c, 2 * (i & 1) + 1)), m1));
+        }
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    }
+};
+template <> struct Eight<DT_Q4_K> : EightK<false> {};
+template <> struct Eight<DT_Q5_K> : EightK<true> {};
+template <> struct Eight<DT_Q6_K> {                                      // eight weights share both scales, the nibble half and the high bits' place
+    uint32_t q0, q1, h0, h1, j;
+    float ds;
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint32_t e = 8u * (t & 31u), h = e >> 7, l = e & 31u;
+        const uint8_t* b = row + (size_t)(t >> 5) * 210u;
+        j = (e >> 5) & 3u;
+        const uint8_t *ql = b + 64 * h + 32 * (j & 1u) + l, *qh = b + 128 + 32 * h + l;
+        q0 = ld32(ql); q1 = ld32(ql + 4); h0 = ld32(qh); h1 = ld32(qh + 4);
+        ds = __fmul_rn(half_bits(ld16(b + 208)), __int2float_rn((int)(int8_t)__ldg(b + 192 + 8 * h + 2 * j + (l >> 4))));
+    }
+    __device__ __forceinline__ uint4 halves() const {
+        uint32_t o[4];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const uint32_t nib = ((w ? q1 : q0) >> (2u * (j & 2u))) & 0x0F0F0F0Fu, code = nib | ((((w ? h1 : h0) >> (2 * j)) & 0x03030303u) << 4);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                o[2 * w + i] = half_pair(__fmul_rn(ds, __int2float_rn((int)((code >> (16 * i)) & 255u) - 32)),
+                                         __fmul_rn(ds, __int2float_rn((int)((code >> (16 * i + 8)) & 255u) - 32)));
+        }
+        return make_uint4(o[0], o[1], o[2], o[3]);
+    }
+};
+
+// Both operand conversions of the pre-pass form in one launch: blocks [0, blocks_w) turn weights into fp16, consecutive
+// threads consecutive sixteen-byte words; the remaining blocks round the activations. (The K-quants, Q8_0 and Q4_1 went
+// through the byte-wise fp32 dequantizer and a launch for the activations before: 2000 tokens x 4096 x 4096 Q5_K 120 us,
+// now 77; Q8_0 91, now 72.)
+template <int DT>
+__global__ void __launch_bounds__(256) prepass_f16(const uint8_t* __restrict__ W, uint32_t row_bytes, __half* __restrict__ Wh,
+                                                   uint32_t N, uint32_t K, const float* __restrict__ A, __half* __restrict__ Ah,
+                                                   size_t n4, uint32_t blocks_w) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // the GEMM may set itself up meanwhile
-    if (blockIdx.x < blocks_w) {
-        const uint32_t wpr = K / 8;                                         // words per row
-        const uint64_t total = (uint64_t)N * wpr, first = (uint64_t)blockIdx.x * (256 * kPrepItems) + threadIdx.x;
-        uint32_t dbits[kPrepItems], q[kPrepItems];
+    if (blockIdx.x >= blocks_w) return round_activations(A, Ah, n4, (size_t)(blockIdx.x - blocks_w) * (256 * kPrepItems) + threadIdx.x);
+    const uint32_t per = K / 8;
+    const uint64_t total = (uint64_t)N * per, first = (uint64_t)blockIdx.x * (256 * kPrepItems) + threadIdx.x;
+    Eight<DT> e[kPrepItems];
 #pragma unroll
-        for (int j = 0; j < kPrepItems; ++j) {
-            const uint64_t idx = first + (uint64_t)j * 256;
-            if (idx < total) {
-                const uint32_t row = (uint32_t)(idx / wpr), w = (uint32_t)(idx % wpr), blk = w >> 2, i = w & 3u;
-                const unsigned short* p = reinterpret_cast<const unsigned short*>(W + (size_t)row * row_bytes + (size_t)blk * 18u);
-                dbits[j] = __ldg(p);
-                q[j] = (uint32_t)__ldg(p + 1 + 2 * i) | ((uint32_t)__ldg(p + 2 + 2 * i) << 16);
-            }
-        }
+    for (int i = 0; i < kPrepItems; ++i) {
+        const uint64_t idx = first + (uint64_t)i * 256;
+        if (idx < total) e[i].load(W + (size_t)(uint32_t)(idx / per) * row_bytes, (uint32_t)(idx % per));
+    }
 #pragma unroll
-        for (int j = 0; j < kPrepItems; ++j) {
-            const uint64_t idx = first + (uint64_t)j * 256;
-            if (idx < total) {
-                const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits[j]));
-                const uint32_t lo = q[j] & 0x0F0F0F0Fu, hi = (q[j] >> 4) & 0x0F0F0F0Fu;
-                const uint32_t p01 = __byte_perm(lo, hi, 0x5140), p23 = __byte_perm(lo, hi, 0x7362);
-                uint4 o;
-                q4_quad(p01, d2, o.x, o.y);
-                q4_quad(p23, d2, o.z, o.w);
-                reinterpret_cast<uint4*>(Wh)[idx] = o;                      // rows are K / 8 sixteen-byte words long: word idx of the whole matrix
-            }
-        }
-    } else {
-        round_activations(A, Ah, n4, (size_t)(blockIdx.x - blocks_w) * (256 * kPrepItems) + threadIdx.x);
+    for (int i = 0; i < kPrepItems; ++i) {
+        const uint64_t idx = first + (uint64_t)i * 256;
+        if (idx < total) reinterpret_cast<uint4*>(Wh)[idx] = e[i].halves();
     }
 }
 
-// The same for Q6_K: one item per eight consecutive weights (they share the super-block scale, the sub-block scale,
-// the nibble half and the high-bit pair position), d * sc and then * (q - 32) in fp32 (both products are exact, as in
-// tmq::dequantize_row_q6_k, tensormark/quant.h:338-365), rounded once to fp16, one 16-byte store.
-__global__ void __launch_bounds__(256) prepass_q6k_f16(const uint8_t* __restrict__ W, uint32_t row_bytes, __half* __restrict__ Wh,
-                                                       uint32_t N, uint32_t K, const float* __restrict__ A, __half* __restrict__ Ah,
-                                                       size_t n4, uint32_t blocks_w) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (blockIdx.x < blocks_w) {
-        const uint32_t gpr = K / 8;                                         // groups of eight per row
-        const uint64_t total = (uint64_t)N * gpr, first = (uint64_t)blockIdx.x * (256 * kPrepItems) + threadIdx.x;
-        uint32_t qlw[kPrepItems][2], qhw[kPrepItems][2], jj[kPrepItems];
-        float ds[kPrepItems];
-#pragma unroll
-        for (int it = 0; it < kPrepItems; ++it) {
-            const uint64_t idx = first + (uint64_t)it * 256;
-            if (idx < total) {
-                const uint32_t row = (uint32_t)(idx / gpr), t = (uint32_t)(idx % gpr), k = t * 8;
-                const uint32_t e = k & 255u, h = e >> 7, j = (e >> 5) & 3u, l0 = e & 31u;
-                const uint8_t* b = W + (size_t)row * row_bytes + (size_t)(k >> 8) * 210u;
-                const unsigned short* ql = reinterpret_cast<const unsigned short*>(b + 64 * h + 32 * (j & 1u) + l0);
-                const unsigned short* qh = reinterpret_cast<const unsigned short*>(b + 128 + 32 * h + l0);
-                const uint32_t dbits = __ldg(reinterpret_cast<const unsigned short*>(b + 208));
-                const int sc = (int)(int8_t)__ldg(b + 192 + 8 * h + 2 * j + (l0 >> 4));
-                ds[it] = __fmul_rn(__half2float(__ushort_as_half((unsigned short)dbits)), __int2float_rn(sc));
-                jj[it] = j;
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    qlw[it][w] = (uint32_t)__ldg(ql + 2 * w) | ((uint32_t)__ldg(ql + 2 * w + 1) << 16);
-                    qhw[it][w] = (uint32_t)__ldg(qh + 2 * w) | ((uint32_t)__ldg(qh + 2 * w + 1) << 16);
-                }
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < kPrepItems; ++it) {
-            const uint64_t idx = first + (uint64_t)it * 256;
-            if (idx < total) {
-                const uint32_t j = jj[it];
-                uint32_t o[4];
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const uint32_t nib = ((j & 2u) ? (qlw[it][w] >> 4) : qlw[it][w]) & 0x0F0F0F0Fu;
-                    const uint32_t code = nib | (((qhw[it][w] >> (2 * j)) & 0x03030303u) << 4);          // four codes 0..63
-                    const float w0 = __fmul_rn(ds[it], __int2float_rn((int)(code & 255u) - 32));
-                    const float w1 = __fmul_rn(ds[it], __int2float_rn((int)((code >> 8) & 255u) - 32));
-                    const float w2 = __fmul_rn(ds[it], __int2float_rn((int)((code >> 16) & 255u) - 32));
-                    const float w3 = __fmul_rn(ds[it], __int2float_rn((int)(code >> 24) - 32));
-                    const __half2 a = __floats2half2_rn(w0, w1), c = __floats2half2_rn(w2, w3);
-                    o[2 * w] = *reinterpret_cast<const uint32_t*>(&a);
-                    o[2 * w + 1] = *reinterpret_cast<const uint32_t*>(&c);
-                }
-                reinterpret_cast<uint4*>(Wh)[idx] = make_uint4(o[0], o[1], o[2], o[3]);
-            }
-        }
-    } else {
-        round_activations(A, Ah, n4, (size_t)(blockIdx.x - blocks_w) * (256 * kPrepItems) + threadIdx.x);
+// Launches it; false when the type or the address is one it does not take (no error is set then).
+bool try_prepass(const uint8_t* W, uint32_t row_bytes, __half* Wh, unsigned N, unsigned K, const float* A, __half* Ah, size_t n4, unsigned dtype, cudaStream_t st) {
+    if ((uintptr_t)W % 2) return false;
+    const unsigned per = 256 * kPrepItems, blocks_w = (unsigned)(((uint64_t)N * (K / 8) + per - 1) / per), grid = blocks_w + (unsigned)((n4 + per - 1) / per);
+    switch (dtype) {
+        case DT_Q4_0: prepass_f16<DT_Q4_0><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_GGUF_Q4_0: prepass_f16<DT_GGUF_Q4_0><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_Q8_0: prepass_f16<DT_Q8_0><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_Q4_1: prepass_f16<DT_Q4_1><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_Q4_K: prepass_f16<DT_Q4_K><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_Q5_K: prepass_f16<DT_Q5_K><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        case DT_Q6_K: prepass_f16<DT_Q6_K><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
+        default: return false;
     }
+    note_launch();
+    return true;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -1075,16 +1153,7 @@ bool launch_weights_f16(const uint8_t* W, void* Wh_out, unsigned N, unsigned K, 
     if (K == 0 || K % be || K % 8) return fail("gemm: K=%u is not a multiple of %u and of 8", K, be);
     __half* Wh = (__half*)Wh_out;
     const uint32_t row_bytes = (K / be) * block_bytes(dtype);
-    const unsigned per = 256 * kPrepItems;
-    const unsigned blocks_w = (unsigned)(((uint64_t)N * (K / 8) + per - 1) / per);
-    if (dtype == DT_Q4_0 && (uintptr_t)W % 2 == 0 && row_bytes % 2 == 0) {
-        prepass_q4_f16<<<blocks_w, 256, 0, st>>>(W, row_bytes, Wh, N, K, nullptr, nullptr, 0, blocks_w);
-    } else if (dtype == DT_Q6_K && (uintptr_t)W % 2 == 0 && row_bytes % 2 == 0) {
-        prepass_q6k_f16<<<blocks_w, 256, 0, st>>>(W, row_bytes, Wh, N, K, nullptr, nullptr, 0, blocks_w);
-    } else {
-        return launch_dequant_half(W, Wh, N, K, dtype, st);
-    }
-    note_launch();
+    if (!try_prepass(W, row_bytes, Wh, N, K, nullptr, nullptr, 0, dtype, st)) return launch_dequant_half(W, Wh, N, K, dtype, st);
     return check_launch("weights_f16");
 }
 
@@ -1134,7 +1203,7 @@ size_t gemm_workspace_bytes(unsigned M, unsigned N, unsigned K) {
 }
 
 bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsigned M, unsigned N, unsigned K,
-                 unsigned dtype, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                 unsigned dtype, void* workspace, size_t workspace_bytes, cudaStream_t st, bool may_permute_k) {
     const unsigned be = block_elems(dtype);
     if (!be || dtype == DT_F16) return fail("gemm: dtype %u is not a block format", dtype);
     if (!A || !W || !C) return fail("gemm: null pointer");
@@ -1149,6 +1218,13 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
     __half* Wh = (__half*)ws;
     __half* Ah = (__half*)(ws + ((size_t)N * K * 2 + 255) / 256 * 256);
 
+    // Up to 512 tokens straight from the blocks: a weight is then converted at most twice, in the shadow of the copies. From
+    // there on converting once for all token tiles is cheaper (4096 x 4096, blocks / fp16 copy: 512 tokens Q4_0 36 / 40,
+    // Q6_K 44 / 44 us; 1000 tokens Q4_0 54 / 48, Q6_K 75 / 52 us). The knobs of the fp16 kernels keep a call on them.
+    static const bool fp16_only = std::getenv("TM_GEMM_FUSED") || std::getenv("TM_GEMM_PAIR") || std::getenv("TM_GEMM_BN");
+    if (M <= 512 && may_permute_k && !fp16_only && gemm_blocks_takes(W, M, N, K, dtype, workspace_bytes))
+        return launch_gemm_blocks(A, W, C, ldc, M, N, K, dtype, workspace, st);
+
     // Q4_0 with K a multiple of 256 and 16-byte aligned rows can be dequantized inside the GEMM (gemm_q4_tn).
     // TM_GEMM_FUSED=1 selects it; the default is the pre-pass, which is the faster of the two today
     // (2000 x 5632 x 2048: 72 us for pre-passes + TMA-fed kernel against 77 us for the producer-fed kernel,
@@ -1157,18 +1233,8 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
     const uint32_t row_bytes = (K / be) * block_bytes(dtype);
     const bool fused = allow_fused && dtype == DT_Q4_0 && K % 256 == 0 && (uintptr_t)W % 16 == 0 && row_bytes % 16 == 0;
     const size_t n4 = (size_t)M * K / 4;
-    if (!fused && dtype == DT_Q4_0 && K % 8 == 0 && (uintptr_t)W % 2 == 0 && row_bytes % 2 == 0) {
-        const unsigned per = 256 * kPrepItems;
-        const unsigned blocks_w = (unsigned)(((uint64_t)N * (K / 8) + per - 1) / per), blocks_a = (unsigned)((n4 + per - 1) / per);
-        prepass_q4_f16<<<blocks_w + blocks_a, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w);
-        note_launch();
-        if (!check_launch("prepass_q4_f16")) return false;
-    } else if (dtype == DT_Q6_K && (uintptr_t)W % 2 == 0 && row_bytes % 2 == 0) {
-        const unsigned per = 256 * kPrepItems;
-        const unsigned blocks_w = (unsigned)(((uint64_t)N * (K / 8) + per - 1) / per), blocks_a = (unsigned)((n4 + per - 1) / per);
-        prepass_q6k_f16<<<blocks_w + blocks_a, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w);
-        note_launch();
-        if (!check_launch("prepass_q6k_f16")) return false;
+    if (!fused && try_prepass(W, row_bytes, Wh, N, K, A, Ah, n4, dtype, st)) {
+        if (!check_launch("prepass_f16")) return false;
     } else {
         if (!fused && !launch_dequant_half(W, Wh, N, K, dtype, st)) return false;
         f32_to_f16_rows<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(A, Ah, n4);

@@ -11,7 +11,14 @@ namespace tmc {
 size_t gemm_workspace_bytes(unsigned M, unsigned N, unsigned K);
 // C[m * ldc + n] = sum_k A[m][k] * W[n][k]  for m < M, n < N; ldc >= N.
 bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsigned M, unsigned N, unsigned K,
-                 unsigned dtype, void* workspace, size_t workspace_bytes, cudaStream_t st);
+                 unsigned dtype, void* workspace, size_t workspace_bytes, cudaStream_t st, bool may_permute_k = true);
+// may_permute_k = false: the sums over K run in the order of launch_gemm_hh on the fp16 copy of the same weights.
+
+// The same straight from the serialized blocks (gemm_blocks.cu), for the calls that gemm_blocks_takes() accepts; Ah: that
+// many bytes of device scratch, 16-byte aligned, for the rounded tokens.
+bool gemm_blocks_takes(const uint8_t* W, unsigned M, unsigned N, unsigned K, unsigned dtype, size_t scratch_bytes);
+bool launch_gemm_blocks(const float* A, const uint8_t* W, float* C, unsigned ldc, unsigned M, unsigned N, unsigned K, unsigned dtype,
+                        void* Ah, cudaStream_t st);
 
 // For callers that keep an fp16 copy of static weights: the copy (exact fp32 value of every weight rounded once, as the
 // GEMM's own pre-pass writes it), and the GEMM against it, whose workspace only holds the rounded activations.

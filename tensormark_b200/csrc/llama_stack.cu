@@ -661,7 +661,7 @@ bool encode_layer(Stack& c, int l, int T, int pos0, cudaStream_t st) {
     const unsigned ld = QD + 2 * KVD, Tn = (unsigned)T;
     const float scale = 1.0f / std::sqrt((float)dh);
     auto gemm = [&](const float* A, const uint8_t* W, float* Cm, unsigned ldc, unsigned N, unsigned K) {
-        return launch_gemm(A, W, Cm, ldc, Tn, N, K, c.dtype, c.ws, c.ws_bytes, st);
+        return launch_gemm(A, W, Cm, ldc, Tn, N, K, c.dtype, c.ws, c.ws_bytes, st, false);      // bit for bit what resident weights give
     };
     auto gemm_h = [&](const __half* Ah, const void* Wh, float* Cm, unsigned ldc, unsigned N, unsigned K, bool accumulate) {
         return launch_gemm_hh(Ah, Wh, Cm, ldc, Tn, N, K, accumulate, st);

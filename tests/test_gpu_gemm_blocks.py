@@ -1,0 +1,51 @@
+"""The GEMM on serialized blocks, at the edges of its dispatch: row tiles of 128, groups of 256 weights, token
+tiles, tiles shared by a cluster along K, rows on and off the 16-byte grid."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tensormark_b200 import lib, synth
+from tests.gpu_util import dev_f32, ptr, stream_ptr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dt,m,n,k,shift", [
+    (synth.Q4_0, 1, 1, 32, 0), (synth.Q4_0, 2, 127, 256, 0), (synth.Q4_0, 17, 129, 288, 0), (synth.Q4_0, 16, 4096, 1024, 0),
+    (synth.Q4_0, 33, 257, 2080, 0), (synth.Q4_0, 65, 300, 4096, 0), (synth.Q4_0, 129, 1000, 512, 0), (synth.Q4_0, 256, 256, 8192, 0),
+    (synth.Q4_0, 20, 256, 2048, 2), (synth.Q4_0, 5, 9500, 2048, 0), (synth.Q4_0, 90, 19000, 512, 0),
+    (synth.GGUF_Q4_0, 12, 200, 4128, 0), (synth.GGUF_Q4_0, 70, 256, 512, 6),
+    (synth.Q4_1, 9, 130, 544, 0), (synth.Q4_1, 100, 384, 2048, 0), (synth.Q4_1, 31, 384, 2048, 4),
+    (synth.Q8_0, 3, 200, 2112, 0), (synth.Q8_0, 48, 3000, 1024, 0), (synth.Q8_0, 8, 96, 14336, 1),
+    (synth.Q6_K, 20, 5119, 256, 0), (synth.Q6_K, 77, 300, 2816, 0), (synth.Q6_K, 4, 128, 14336, 3),
+    (synth.Q5_K, 6, 250, 14336, 0), (synth.Q5_K, 128, 512, 768, 0), (synth.Q4_K, 3, 129, 256, 0), (synth.Q4_K, 200, 640, 4096, 0),
+    (synth.Q5_K, 20, 250, 512, 2), (synth.Q4_K, 20, 250, 512, 1), (synth.Q4_0, 512, 300, 1024, 0), (synth.Q6_K, 511, 257, 512, 0),
+    # past the last token count it takes: the fp16 copy, eight weights per thread
+    (synth.Q4_0, 513, 130, 544, 0), (synth.GGUF_Q4_0, 513, 130, 544, 0), (synth.Q4_1, 513, 130, 544, 0), (synth.Q8_0, 513, 130, 544, 0),
+    (synth.Q4_K, 513, 130, 768, 0), (synth.Q5_K, 513, 130, 768, 0), (synth.Q6_K, 513, 130, 768, 0), (synth.Q8_0, 513, 130, 544, 1),
+])
+def test_edges(cuda, torch_mod, orc, dt, m, n, k, shift):
+    torch = torch_mod
+    W = synth.make_weights(dt, n, k, seed=14)
+    A = synth.make_activations((m, k), seed=15)
+    flat = np.ascontiguousarray(W, dtype=np.uint8).reshape(-1)
+    Wd = torch.zeros(flat.size + 64, dtype=torch.uint8, device="cuda")
+    Wd[shift:shift + flat.size] = torch.from_numpy(flat).cuda()
+    Ad = dev_f32(torch, A)
+    Cd = torch.full((m + 1, n), float("nan"), dtype=torch.float32, device="cuda")
+    need = cuda.tm_cuda_sgemm_q_workspace(m, n, k, dt)
+    ws = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
+    base = C.c_void_p((ws.data_ptr() + 255) // 256 * 256)
+    for _ in range(2):
+        lib.check(cuda.tm_cuda_sgemm_q_dev(ptr(Ad), C.c_void_p(Wd.data_ptr() + shift), ptr(Cd), m, n, k, dt, base, need, stream_ptr(torch)),
+                  "tm_cuda_sgemm_q_dev")
+    torch.cuda.synchronize()
+    got = Cd.cpu().numpy()
+    assert np.isnan(got[m]).all()                          # nothing behind the result
+    ref = orc.gemm(dt, W, A, m, n, k, threads=4)
+    absum = np.abs(A) @ np.abs(orc.dequant(dt, W, n * k).reshape(n, k)).T
+    err = np.abs(got[:m] - ref)
+    assert np.all(err <= 1e-3 * absum), float((err / absum).max())
