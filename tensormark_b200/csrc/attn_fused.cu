@@ -10,7 +10,7 @@
 //   contiguous range of tiles of one KV head and its warps take them round-robin.
 //   * Every CTA rotates the REP query heads of its KV head into shared memory (q is tiny).
 //   * The CTA whose range holds position `pos` rotates the new k, stores k and v into the caches
-//     and, after a barrier, reads them back like any other position.
+//     and takes its own scores and values of that row from shared memory.
 //   * Scores: one LANE per POSITION. A lane reads its own K row (contiguous) and dots it with the
 //     query heads from shared memory (broadcast reads): no shuffle per position, 32 independent
 //     row reads in flight per warp.
@@ -33,17 +33,16 @@ namespace tmc {
 
 namespace {
 
-constexpr unsigned kMaxSplits = 32;      // merge scratch in shared memory: 2 * REP * kMaxSplits floats
+constexpr unsigned kMaxSplits = 32;      // a lane each in the merge
 
 __device__ __forceinline__ unsigned long long now_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// The rotation, with its contractions written out: what a token's K row is must not depend on how a compiler places them.
+__device__ __forceinline__ float rope_lo(float a, float b, float2 cs) { return fmaf(a, cs.x, -__fmul_rn(b, cs.y)); }
+__device__ __forceinline__ float rope_hi(float a, float b, float2 cs) { return fmaf(a, cs.y, __fmul_rn(b, cs.x)); }
 
 template <typename T> __device__ __forceinline__ T to_cache(float v);
 template <> __device__ __forceinline__ float to_cache<float>(float v) { return v; }
@@ -88,6 +87,106 @@ __device__ __forceinline__ void unpackv(const RawV<__half, 2>& r, float (&f)[2])
 __device__ __forceinline__ void unpackv(const RawV<float, 4>& r, float (&f)[4]) { f[0] = r.u.x; f[1] = r.u.y; f[2] = r.u.z; f[3] = r.u.w; }
 __device__ __forceinline__ void unpackv(const RawV<float, 2>& r, float (&f)[2]) { f[0] = r.u.x; f[1] = r.u.y; }
 
+// A warp's part of a split: `tile`, `tile` + 4, ... below t1, for the REP query heads. kn, vn: the new position's rows
+// (the cache's rows of it may not be visible yet when the first tile is fetched).
+template <typename T, int DPL, int REP> struct Tile {
+    static constexpr int dh = DPL * 32;
+    Raw8<T> raw[dh / 8];
+    RawV<T, DPL> vraw[32];                                     // rows past the tile's last position repeat it, their weight is 0
+    __device__ __forceinline__ void fetch(const T* kbase, const T* vbase, uint32_t t, uint32_t allow, uint32_t lane) {   // this lane's K row (lane = position) and its dims of the 32 V rows
+        const uint32_t p = t * 32 + lane, np = min(32u, allow - t * 32);
+        const T* krow = kbase + (size_t)min(p, allow - 1) * dh;
+        const T* vrow = vbase + (size_t)t * 32 * dh + lane * DPL;
+#pragma unroll
+        for (int c = 0; c < dh / 8; ++c) fetch8(krow + c * 8, raw[c]);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) fetchv(vrow + (size_t)min((uint32_t)k, np - 1) * dh, vraw[k]);
+    }
+    // what aliases the new position's row, taken from shared memory
+    __device__ __forceinline__ void patch(const T* kn, const T* vn, uint32_t kpos, uint32_t lane) {
+        if (lane >= kpos) {
+#pragma unroll
+            for (int c = 0; c < dh / 8; ++c) raw[c] = *reinterpret_cast<const Raw8<T>*>(kn + c * 8);
+        }
+        const RawV<T, DPL> v = *reinterpret_cast<const RawV<T, DPL>*>(vn + lane * DPL);
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+            if ((uint32_t)k >= kpos) vraw[k] = v;
+    }
+    __device__ __forceinline__ void attend(const T* kbase, const T* vbase, const T* kn, const T* vn, uint32_t tile, uint32_t t1, uint32_t tiles,
+                                           uint32_t allow, uint32_t lane, const float (*qs)[dh], float* sm_m, float* sm_l, float (*sm_acc)[dh]) {
+        float m[REP], l[REP], acc[REP][DPL];
+#pragma unroll
+        for (int r = 0; r < REP; ++r) {
+            m[r] = -CUDART_INF_F; l[r] = 0.f;
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) acc[r][d] = 0.f;
+        }
+        for (uint32_t t = tile; t < t1; t += 4) {
+            const uint32_t p = t * 32 + lane;
+            const bool live = p < allow;
+            float s[REP];
+#pragma unroll
+            for (int r = 0; r < REP; ++r) s[r] = 0.f;
+            // Every load of a tile is requested before anything is computed on it; the first tile's were before the wait.
+            if (t != tile) fetch(kbase, vbase, t, allow, lane);
+            if (t == tiles - 1) patch(kn, vn, allow - 1 - t * 32, lane);
+            if (live) {
+#pragma unroll
+                for (int c = 0; c < dh / 8; ++c) {
+                    float kf[8];
+                    unpack8(raw[c], kf);
+#pragma unroll
+                    for (int r = 0; r < REP; ++r) {
+                        const float4 qa = *reinterpret_cast<const float4*>(&qs[r][c * 8]);
+                        const float4 qb = *reinterpret_cast<const float4*>(&qs[r][c * 8 + 4]);
+                        float v = s[r];
+                        v = fmaf(qa.x, kf[0], v); v = fmaf(qa.y, kf[1], v); v = fmaf(qa.z, kf[2], v); v = fmaf(qa.w, kf[3], v);
+                        v = fmaf(qb.x, kf[4], v); v = fmaf(qb.y, kf[5], v); v = fmaf(qb.z, kf[6], v); v = fmaf(qb.w, kf[7], v);
+                        s[r] = v;
+                    }
+                }
+            }
+            // tile softmax statistics and this lane's weight per head
+            float pw[REP];
+#pragma unroll
+            for (int r = 0; r < REP; ++r) {
+                float tm = live ? s[r] : -CUDART_INF_F;
+#pragma unroll
+                for (int o = 16; o; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
+                const float mn = fmaxf(m[r], tm);                 // finite: every tile holds at least one live position
+                const float corr = __expf(m[r] - mn);
+                pw[r] = live ? __expf(s[r] - mn) : 0.f;
+                float ts = pw[r];
+#pragma unroll
+                for (int o = 16; o; o >>= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
+                l[r] = l[r] * corr + ts;
+#pragma unroll
+                for (int d = 0; d < DPL; ++d) acc[r][d] *= corr;
+                m[r] = mn;
+            }
+            // values: lanes own dims, the tile's positions one after another (weight 0 past the last position)
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+                float vf[DPL];
+                unpackv(vraw[k], vf);
+#pragma unroll
+                for (int r = 0; r < REP; ++r) {
+                    const float w = __shfl_sync(0xffffffffu, pw[r], k);
+#pragma unroll
+                    for (int d = 0; d < DPL; ++d) acc[r][d] = fmaf(w, vf[d], acc[r][d]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < REP; ++r) {
+            if (lane == 0) { sm_m[r] = m[r]; sm_l[r] = l[r]; }
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) sm_acc[r][lane * DPL + d] = acc[r][d];
+        }
+    }
+};
+
 template <typename T, int DPL, int REP>
 __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc, T* vc, float* part, float* stat,
                                                           unsigned* counters, float* out, uint32_t H, uint32_t KVH,
@@ -105,154 +204,80 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
     // The position was written by the previous token's last kernel and the cache rows below it by earlier tokens:
     // both are safe to read before this token's q|k|v GEMV has finished, and this CTA is resident (and idle) for
     // several microseconds before that. So the first tile's loads, with their page walks and DRAM latency, are
-    // requested now; only the row of the new position is fetched after it has been written.
+    // requested now; only the row of the new position is put in after the wait.
     const int pos_i = *(volatile const int*)st;
     const bool valid = !(pos_i < 0 || (uint32_t)pos_i >= ctx || (uint32_t)pos_i * half + half > tbl_n);   // same guard as the separate kernels
     const uint32_t pos = valid ? (uint32_t)pos_i : 0u, allow = pos + 1;
     const uint32_t tiles = (allow + 31) / 32, tps = (tiles + nsplit - 1) / nsplit;
-    const uint32_t t0 = min(tiles, split * tps), t1 = min(tiles, t0 + tps);
+    const uint32_t t0 = min(tiles, split * tps), t1 = min(tiles, t0 + tps), used = (tiles + tps - 1) / tps;    // used: splits that have a tile
     const T* kbase = kc + (size_t)kv * ctx * dh;
     const T* vbase = vc + (size_t)kv * ctx * dh;
-    Raw8<T> raw[dh / 8];
-    RawV<T, DPL> vraw[32];                                     // rows past the tile's last position repeat it, their weight is 0
-    auto fetch_tile = [&](uint32_t t) {                        // this lane's K row (lane = position) and its dims of the 32 V rows
-        const uint32_t p = t * 32 + lane, np = min(32u, allow - t * 32);
-        const T* krow = kbase + (size_t)min(p, allow - 1) * dh;
-        const T* vrow = vbase + (size_t)t * 32 * dh + lane * DPL;
-#pragma unroll
-        for (int c = 0; c < dh / 8; ++c) fetch8(krow + c * 8, raw[c]);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) fetchv(vrow + (size_t)min((uint32_t)k, np - 1) * dh, vraw[k]);
-    };
     const uint32_t t_first = t0 + warp;
-    if (valid && t_first < t1) fetch_tile(t_first);
+    Tile<T, DPL, REP> tile;
+    if (valid && t_first < t1) tile.fetch(kbase, vbase, t_first, allow, lane);
+    const float2 cs = valid ? tbl[(size_t)pos * half + threadIdx.x % half] : make_float2(0.f, 0.f);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tr) tr[1] = now_ns();
-    if (!valid) return;
+    if (!valid || t0 >= t1) return;                           // a split without positions leaves nothing to merge
 
     __shared__ __align__(16) float qs[REP][dh];
+    __shared__ __align__(16) T knew[dh];
+    __shared__ __align__(16) T vnew[dh];
     __shared__ float sm_acc[4][REP][dh];
     __shared__ float sm_m[4][REP], sm_l[4][REP];
+    __shared__ float cm[REP][kMaxSplits], inv_l[REP];
     __shared__ int sm_last;
 
-    // ---- rope(q) for this KV head's query heads, scaled, into shared memory
-    for (uint32_t i = threadIdx.x; i < REP * half; i += 128) {
-        const uint32_t r = i / half, j = i % half;
-        const float2 cs = tbl[(size_t)pos * half + j];
-        const float* q = qkv + (size_t)(kv * REP + r) * dh;
-        const float a = __ldcg(q + j), b = __ldcg(q + j + half);
-        qs[r][j] = (a * cs.x - b * cs.y) * scale;
-        qs[r][j + half] = (b * cs.x + a * cs.y) * scale;
-    }
-    // ---- the new position's k (rotated) and v go into the caches; the CTA that attends it writes them
-    if (t1 == tiles && t1 > t0) {
-        const float* kn = qkv + (size_t)(H + kv) * dh;
-        const float* vn = qkv + (size_t)(H + KVH + kv) * dh;
-        T* kdst = kc + ((size_t)kv * ctx + pos) * dh;
-        T* vdst = vc + ((size_t)kv * ctx + pos) * dh;
-        for (uint32_t j = threadIdx.x; j < (uint32_t)half; j += 128) {
-            const float2 cs = tbl[(size_t)pos * half + j];
-            const float a = __ldcg(kn + j), b = __ldcg(kn + j + half);
-            kdst[j] = to_cache<T>(a * cs.x - b * cs.y);
-            kdst[j + half] = to_cache<T>(b * cs.x + a * cs.y);
+    // ---- rope(q) for this KV head's query heads, scaled, into shared memory; the new position's k (rotated) and v into
+    // the caches and into shared memory, by the CTA that attends it. All loads are requested before the first is used.
+    {
+        constexpr int NQ = (REP * half + 127) / 128;
+        const uint32_t j = threadIdx.x % half;
+        const bool newest = t1 == tiles;
+        float a[NQ], b[NQ], ka = 0.f, kb = 0.f, va = 0.f;
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) {
+            const uint32_t r = (threadIdx.x + n * 128u) / half;
+            if (r < (uint32_t)REP) { const float* q = qkv + (size_t)(kv * REP + r) * dh; a[n] = __ldcg(q + j); b[n] = __ldcg(q + j + half); }
         }
-        for (uint32_t j = threadIdx.x; j < (uint32_t)dh; j += 128) vdst[j] = to_cache<T>(__ldcg(vn + j));
+        if (newest && threadIdx.x < half) { const float* kn = qkv + (size_t)(H + kv) * dh; ka = __ldcg(kn + j); kb = __ldcg(kn + j + half); }
+        if (newest && threadIdx.x < dh) va = __ldcg(qkv + (size_t)(H + KVH + kv) * dh + threadIdx.x);
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) {
+            const uint32_t r = (threadIdx.x + n * 128u) / half;
+            if (r < (uint32_t)REP) {
+                qs[r][j] = rope_lo(a[n], b[n], cs) * scale;
+                qs[r][j + half] = rope_hi(a[n], b[n], cs) * scale;
+            }
+        }
+        if (newest) {
+            T* kdst = kc + ((size_t)kv * ctx + pos) * dh;
+            T* vdst = vc + ((size_t)kv * ctx + pos) * dh;
+            if (threadIdx.x < half) {
+                kdst[j] = knew[j] = to_cache<T>(rope_lo(ka, kb, cs));
+                kdst[j + half] = knew[j + half] = to_cache<T>(rope_hi(ka, kb, cs));
+            }
+            if (threadIdx.x < dh) vdst[threadIdx.x] = vnew[threadIdx.x] = to_cache<T>(va);
+        }
     }
     __syncthreads();
     if (tr) tr[2] = now_ns();
 
-    // ---- this warp's tiles
-    float m[REP], l[REP], acc[REP][DPL];
-#pragma unroll
-    for (int r = 0; r < REP; ++r) {
-        m[r] = -CUDART_INF_F; l[r] = 0.f;
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) acc[r][d] = 0.f;
-    }
-    for (uint32_t t = t_first; t < t1; t += 4) {
-        const uint32_t p = t * 32 + lane;
-        const bool live = p < allow;
-        float s[REP];
-#pragma unroll
-        for (int r = 0; r < REP; ++r) s[r] = 0.f;
-        // Every load of a tile is requested before anything is computed on it. The first tile's were requested
-        // before the wait; of those, whatever aliases the new position's row is fetched again now that it is written.
-        if (t != t_first) {
-            fetch_tile(t);
-        } else if (t == tiles - 1) {
-            const uint32_t kpos = pos - t * 32;
-            if (lane >= kpos) {
-#pragma unroll
-                for (int c = 0; c < dh / 8; ++c) fetch8(kbase + (size_t)pos * dh + c * 8, raw[c]);
-            }
-#pragma unroll
-            for (int k = 0; k < 32; ++k)
-                if ((uint32_t)k >= kpos) fetchv(vbase + (size_t)pos * dh + lane * DPL, vraw[k]);
-        }
-        if (live) {
-#pragma unroll
-            for (int c = 0; c < dh / 8; ++c) {
-                float kf[8];
-                unpack8(raw[c], kf);
-#pragma unroll
-                for (int r = 0; r < REP; ++r) {
-                    const float4 qa = *reinterpret_cast<const float4*>(&qs[r][c * 8]);
-                    const float4 qb = *reinterpret_cast<const float4*>(&qs[r][c * 8 + 4]);
-                    float v = s[r];
-                    v = fmaf(qa.x, kf[0], v); v = fmaf(qa.y, kf[1], v); v = fmaf(qa.z, kf[2], v); v = fmaf(qa.w, kf[3], v);
-                    v = fmaf(qb.x, kf[4], v); v = fmaf(qb.y, kf[5], v); v = fmaf(qb.z, kf[6], v); v = fmaf(qb.w, kf[7], v);
-                    s[r] = v;
-                }
-            }
-        }
-        // tile softmax statistics and this lane's weight per head
-        float pw[REP];
-#pragma unroll
-        for (int r = 0; r < REP; ++r) {
-            float tm = live ? s[r] : -CUDART_INF_F;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
-            const float mn = fmaxf(m[r], tm);                 // finite: every tile holds at least one live position
-            const float corr = __expf(m[r] - mn);
-            pw[r] = live ? __expf(s[r] - mn) : 0.f;
-            float ts = pw[r];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
-            l[r] = l[r] * corr + ts;
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) acc[r][d] *= corr;
-            m[r] = mn;
-        }
-        // values: lanes own dims, the tile's positions one after another (weight 0 past the last position)
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            float vf[DPL];
-            unpackv(vraw[k], vf);
-#pragma unroll
-            for (int r = 0; r < REP; ++r) {
-                const float w = __shfl_sync(0xffffffffu, pw[r], k);
-#pragma unroll
-                for (int d = 0; d < DPL; ++d) acc[r][d] = fmaf(w, vf[d], acc[r][d]);
-            }
-        }
-    }
-
+    tile.attend(kbase, vbase, knew, vnew, t_first, t1, tiles, allow, lane, qs, sm_m[warp], sm_l[warp], sm_acc[warp]);
     if (tr) tr[4] = now_ns();
-    // ---- merge the four warps, leave this split's partial
-#pragma unroll
-    for (int r = 0; r < REP; ++r) {
-        if (lane == 0) { sm_m[warp][r] = m[r]; sm_l[warp][r] = l[r]; }
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) sm_acc[warp][r][lane * DPL + d] = acc[r][d];
-    }
+    // ---- merge the warps, leave this split's partial
     __syncthreads();
+#pragma unroll
     for (int r = 0; r < REP; ++r) {
         float M = -CUDART_INF_F;
 #pragma unroll
         for (int w = 0; w < 4; ++w) M = fmaxf(M, sm_m[w][r]);
         float Lsum = 0.f, f[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) { f[w] = sm_m[w][r] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][r] - M); Lsum += f[w] * sm_l[w][r]; }
+        for (int w = 0; w < 4; ++w) {
+            f[w] = sm_m[w][r] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][r] - M);
+            Lsum += f[w] * sm_l[w][r];
+        }
         const uint32_t head = kv * REP + r;
         for (int d = threadIdx.x; d < dh; d += 128) {
             float o = 0.f;
@@ -268,46 +293,55 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned prev = atomicAdd(&counters[kv], 1u);
-        sm_last = prev == nsplit - 1;
+        sm_last = prev == used - 1;
         if (sm_last) counters[kv] = 0u;                       // re-armed for the next launch
     }
     __syncthreads();
     if (tr) { tr[5] = now_ns(); tr[3] = tr[5]; }
     if (!sm_last) return;
     __threadfence();
-    // statistics of every (head, split) into shared memory with one load each, then the weights
-    float* cm = &sm_acc[0][0][0];                              // [REP][nsplit] max, reused as the split weight
-    float* cl = cm + REP * kMaxSplits;                         // [REP][nsplit] sum
-    for (uint32_t i = threadIdx.x; i < REP * nsplit; i += 128) {
-        const uint32_t r = i / nsplit, s2 = i % nsplit;
-        const float2 ml = __ldcg(reinterpret_cast<const float2*>(stat + ((size_t)s2 * H + kv * REP + r) * 2));
-        cm[r * kMaxSplits + s2] = ml.x; cl[r * kMaxSplits + s2] = ml.y;
+    // The merge is a chain of L2 latencies: BATCH splits of all the outputs of a thread are requested at a time, the first
+    // ones before the weights are known (six splits of one output at a time took 16 round trips, 10 us of the kernel).
+    constexpr int NI = (REP * dh + 127) / 128, BATCH = NI >= 8 ? 4 : 32 / NI;
+    float v[NI][BATCH], o[NI];
+    auto request = [&](uint32_t s0) {
+#pragma unroll
+        for (int n = 0; n < NI; ++n) {
+            const uint32_t i = min(threadIdx.x + n * 128u, (uint32_t)(REP * dh - 1)), head = kv * REP + i / dh, d = i % dh;
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) v[n][k] = __ldcg(part + ((size_t)min(s0 + k, used - 1) * H + head) * dh + d);
+        }
+    };
+    request(0);
+    // the splits' weights: a warp per head, a lane per split
+    for (uint32_t r = warp; r < (uint32_t)REP; r += 4) {
+        float2 ml = make_float2(-CUDART_INF_F, 0.f);
+        if (lane < used) ml = __ldcg(reinterpret_cast<const float2*>(stat + ((size_t)lane * H + kv * REP + r) * 2));
+        float M = ml.x;
+#pragma unroll
+        for (int sh = 16; sh; sh >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, sh));
+        const float wgt = ml.x == -CUDART_INF_F ? 0.f : __expf(ml.x - M);
+        float L = 0.f;
+        for (uint32_t s2 = 0; s2 < used; ++s2) L = fmaf(__shfl_sync(0xffffffffu, wgt, s2), __shfl_sync(0xffffffffu, ml.y, s2), L);
+        cm[r][lane] = wgt;
+        if (lane == 0) inv_l[r] = 1.0f / L;
     }
     __syncthreads();
-    if (threadIdx.x < REP) {
-        const uint32_t r = threadIdx.x;
-        float M = -CUDART_INF_F, L = 0.f;
-        for (uint32_t s2 = 0; s2 < nsplit; ++s2) M = fmaxf(M, cm[r * kMaxSplits + s2]);
-        for (uint32_t s2 = 0; s2 < nsplit; ++s2) {
-            const float ms = cm[r * kMaxSplits + s2];
-            const float wgt = ms == -CUDART_INF_F ? 0.f : __expf(ms - M);
-            L += wgt * cl[r * kMaxSplits + s2];
-            cm[r * kMaxSplits + s2] = wgt;
+#pragma unroll
+    for (int n = 0; n < NI; ++n) o[n] = 0.f;
+    for (uint32_t s0 = 0; s0 < used; s0 += BATCH) {
+        if (s0) request(s0);
+#pragma unroll
+        for (int n = 0; n < NI; ++n) {
+            const uint32_t r = min(threadIdx.x + n * 128u, (uint32_t)(REP * dh - 1)) / dh;
+#pragma unroll
+            for (int k = 0; k < BATCH; ++k) if (s0 + k < used) o[n] = __fadd_rn(o[n], __fmul_rn(cm[r][s0 + k], v[n][k]));
         }
-        sm_l[0][r] = 1.0f / L;
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < REP * (uint32_t)dh; i += 128) {
-        const uint32_t r = i / dh, d = i % dh, head = kv * REP + r;
-        float o = 0.f;
-        for (uint32_t s0 = 0; s0 < nsplit; s0 += 6) {
-            float v[6];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) v[k] = __ldcg(part + ((size_t)min(s0 + k, nsplit - 1) * H + head) * dh + d);
-#pragma unroll
-            for (int k = 0; k < 6; ++k) o += s0 + k < nsplit ? cm[r * kMaxSplits + s0 + k] * v[k] : 0.f;
-        }
-        out[(size_t)head * dh + d] = o * sm_l[0][r];
+    for (int n = 0; n < NI; ++n) {
+        const uint32_t i = threadIdx.x + n * 128u;
+        if (i < (uint32_t)(REP * dh)) out[(size_t)(kv * REP) * dh + i] = o[n] * inv_l[i / dh];
     }
 }
 
@@ -352,6 +386,7 @@ bool launch_rep(unsigned REP, dim3 grid, cudaStream_t st, const float* qkv, void
 unsigned attn_fused_splits(unsigned H, unsigned KVH, unsigned dh, unsigned ctx, size_t scratch_bytes) {
     unsigned nsplit = ((unsigned)device_sm_count() + KVH - 1) / KVH;
     const unsigned tiles = (ctx + 31) / 32;
+    static_assert(kMaxSplits <= 32, "the merge gives every split a lane");
     if (nsplit > tiles) nsplit = tiles;
     if (nsplit > kMaxSplits) nsplit = kMaxSplits;
     const size_t per_split = (size_t)H * (dh + 2) * sizeof(float);

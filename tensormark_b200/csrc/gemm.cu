@@ -983,7 +983,10 @@ __global__ void __launch_bounds__(256) prepass_f16(const uint8_t* __restrict__ W
 #pragma unroll
     for (int i = 0; i < kPrepItems; ++i) {
         const uint64_t idx = first + (uint64_t)i * 256;
-        if (idx < total) e[i].load(W + (size_t)(uint32_t)(idx / per) * row_bytes, (uint32_t)(idx % per));
+        if (idx < total) {
+            const uint32_t row = total >> 32 ? (uint32_t)(idx / per) : (uint32_t)idx / per;      // a 64-bit division costs more than the rest of an item
+            e[i].load(W + (size_t)row * row_bytes, (uint32_t)(idx - (uint64_t)row * per));
+        }
     }
 #pragma unroll
     for (int i = 0; i < kPrepItems; ++i) {
