@@ -224,6 +224,7 @@ gemm_f16_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     bool dead = false;
     // Launched with programmatic stream serialization: everything above (barriers, TMEM) overlaps the pre-pass that
     // writes the fp16 operands; nothing below may start before that kernel has finished.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp == 0 || warp >= 6) {
@@ -475,6 +476,7 @@ gemm_f16_tn_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool dead = false;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");           // the pre-pass has written the fp16 operands
 
     if (warp == 0 || warp >= 6) {

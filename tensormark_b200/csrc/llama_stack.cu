@@ -41,6 +41,21 @@ __device__ __forceinline__ float wsum(float v) {
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
+// Kernels of a layer follow each other closely: each may be set up while the one before it drains, and waits for it here.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
 __device__ __forceinline__ float wmax(float v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -55,6 +70,7 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restri
                                                            OT* __restrict__ out, uint32_t D, float eps) {
     __shared__ float part[8];
     __shared__ float inv_s;
+    pdl_enter();
     const float* xr = x + (size_t)blockIdx.x * D;
     OT* o = out + (size_t)blockIdx.x * D;
     // rows of up to 8192 values stay in registers between the two passes (16-byte loads, all requested at once)
@@ -117,34 +133,49 @@ __global__ void bias_rows_kernel(float* __restrict__ y, const float* __restrict_
 // For every token t of the batch (position pos0 + t): rotate q in place, rotate k into the K cache row, copy v into the
 // V cache row (ll_rope + ll_kv_append, metal_llama.h:61-87; pairs (j, j + dh/2), angles from the shared table).
 // kh / vh (both or neither): fp16 copies of the same cache rows, the operands of prefill_attn_h_kernel.
+// grid (tokens, items), an item = four dims of a head's lower half with the four of its upper half, or four of v: bound by
+// its reads and writes, 16 bytes at a time (one value per thread and two 64-bit divisions each took 24 us for 1499 tokens
+// of 40 heads of 128, now 12).
 __global__ void rope_append_kernel(float* __restrict__ qkv, uint32_t ld, float* __restrict__ kc, float* __restrict__ vc,
                                    __half* __restrict__ kh, __half* __restrict__ vh,
                                    uint32_t H, uint32_t KVH, uint32_t dh, uint32_t ctx, uint32_t pos0, uint32_t T,
                                    const float2* __restrict__ tbl, uint32_t tbl_n) {
-    const uint32_t half = dh / 2, per_tok = (H + KVH) * half + KVH * dh;
-    const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (size_t)T * per_tok) return;
-    const uint32_t t = (uint32_t)(gid / per_tok), e = (uint32_t)(gid % per_tok), pos = pos0 + t;
+    pdl_enter();
+    const uint32_t quarter = dh / 8, rot = (H + KVH) * quarter, t = blockIdx.x, pos = pos0 + t;
+    uint32_t e = blockIdx.y * blockDim.x + threadIdx.x;
     float* row = qkv + (size_t)t * ld;
-    if (e < (H + KVH) * half) {
-        const uint32_t h = e / half, j = e % half;
-        if ((size_t)pos * half + j >= tbl_n) return;
-        const float2 cs = tbl[(size_t)pos * half + j];
-        float* r = row + (size_t)h * dh;                       // q heads, then k heads, are contiguous in the row
-        const float a = r[j], b = r[j + half];
-        const float ra = a * cs.x - b * cs.y, rb = b * cs.x + a * cs.y;
-        if (h < H) { r[j] = ra; r[j + half] = rb; }
-        else {
-            const size_t at = ((size_t)(h - H) * ctx + pos) * dh;
-            kc[at + j] = ra; kc[at + j + half] = rb;
-            if (kh) { kh[at + j] = __float2half_rn(ra); kh[at + j + half] = __float2half_rn(rb); }
+    auto halves = [](float4 v) {
+        const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+        return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    };
+    if (e < rot) {
+        const uint32_t h = e / quarter, j = 4 * (e % quarter), half = dh / 2;
+        if ((size_t)pos * half + j + 3 >= tbl_n) return;
+        const float4* cs = reinterpret_cast<const float4*>(tbl + (size_t)pos * half + j);
+        const float4 c01 = cs[0], c23 = cs[1];
+        float* r = row + (size_t)h * dh + j;                   // q heads, then k heads, are contiguous in the row
+        const float4 a = *reinterpret_cast<const float4*>(r), b = *reinterpret_cast<const float4*>(r + half);
+        // contractions written out: the rows do not depend on how a compiler places them
+        auto lo = [](float x, float y, float c, float sn) { return fmaf(x, c, -__fmul_rn(y, sn)); };
+        auto hi = [](float x, float y, float c, float sn) { return fmaf(x, sn, __fmul_rn(y, c)); };
+        const float4 ra = make_float4(lo(a.x, b.x, c01.x, c01.y), lo(a.y, b.y, c01.z, c01.w), lo(a.z, b.z, c23.x, c23.y), lo(a.w, b.w, c23.z, c23.w));
+        const float4 rb = make_float4(hi(a.x, b.x, c01.x, c01.y), hi(a.y, b.y, c01.z, c01.w), hi(a.z, b.z, c23.x, c23.y), hi(a.w, b.w, c23.z, c23.w));
+        if (h < H) {
+            *reinterpret_cast<float4*>(r) = ra; *reinterpret_cast<float4*>(r + half) = rb;
+        } else {
+            const size_t at = ((size_t)(h - H) * ctx + pos) * dh + j;
+            *reinterpret_cast<float4*>(kc + at) = ra; *reinterpret_cast<float4*>(kc + at + half) = rb;
+            if (kh) { *reinterpret_cast<uint2*>(kh + at) = halves(ra); *reinterpret_cast<uint2*>(kh + at + half) = halves(rb); }
         }
-    } else {
-        const uint32_t i = e - (H + KVH) * half, kv = i / dh, l = i % dh;
-        const float v = row[(size_t)(H + KVH) * dh + i];
-        vc[((size_t)kv * ctx + pos) * dh + l] = v;
-        if (vh) vh[((size_t)kv * ctx + pos) * dh + l] = __float2half_rn(v);
+        return;
     }
+    e -= rot;
+    if (e >= KVH * dh / 4) return;
+    const uint32_t i = 4 * e, kv = i / dh, l = i % dh;
+    const float4 v = *reinterpret_cast<const float4*>(row + (size_t)(H + KVH) * dh + i);
+    const size_t at = ((size_t)kv * ctx + pos) * dh + l;
+    *reinterpret_cast<float4*>(vc + at) = v;
+    if (vh) *reinterpret_cast<uint2*>(vh + at) = halves(v);
 }
 
 __device__ __forceinline__ uint32_t to_tf32(float v) {
@@ -159,7 +190,7 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Causal GQA attention of a token batch against the fp32 caches. grid (token blocks, KVH), 128 threads = 4 warps.
+// Causal GQA attention of a token batch against the fp32 caches. grid: token blocks from the last one on x KVH, 128 threads = 4 warps.
 // Row r of a CTA = token t0 + r / REP, query head g * REP + r % REP; BT = 64 / REP tokens per CTA, keys in tiles of 32.
 // Both products run on the tensor cores as m16n8k8 tf32 MMAs with fp32 accumulation: q (pre-scaled), k, v and the
 // probabilities are rounded once to tf32 (10 mantissa bits, the precision the projections' fp16 operands have, with
@@ -187,7 +218,8 @@ __global__ void __launch_bounds__(128, 3) prefill_attn_kernel(const float* __res
     constexpr int NT = DH / 8;                                  // output n-tiles (a warp holds all DH dims of its rows)
     constexpr int PER = 32 * D4 / 128;                          // 16-byte pieces per thread, tile and tensor
     extern __shared__ __align__(16) float sm[];                 // ring: [buf][K 32 x RS | V 32 x RS]
-    const uint32_t BT = 64u / REP, nrows = BT * REP, g = blockIdx.y, t0 = blockIdx.x * BT;
+    const uint32_t BT = 64u / REP, nrows = BT * REP, nblk = (T + BT - 1) / BT, kvh = gridDim.x / nblk;
+    const uint32_t g = blockIdx.x % kvh, t0 = (nblk - 1 - blockIdx.x / kvh) * BT;     // the longest rows of every head first
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int fg = lane >> 2, ft = lane & 3;
     const uint32_t t_end = min(T, t0 + BT);
@@ -361,6 +393,8 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // q (pre-scaled), k, v and the probabilities carry fp16's 10 mantissa bits, as tf32 does; what fp16 lacks is range, and
 // a cache value beyond 65504 becomes inf here as it does in the decode lane's fp16 K/V slots. Scores, softmax
 // statistics and the output stay fp32. Three 32-key tiles of K and V ride a cp.async ring: one barrier per tile.
+// A CTA's work grows with its token block, so the blocks of the last tokens start first (1499 tokens, 32 heads of 128: 139 us
+// in ascending order, where the longest CTAs of the last head were the tail, now 100; the MMAs alone take 66).
 template <int DH, typename OT>
 __global__ void __launch_bounds__(128, 3) prefill_attn_h_kernel(const float* __restrict__ qkv, uint32_t ld, const __half* __restrict__ kh,
                                                                 const __half* __restrict__ vh, OT* __restrict__ out, uint32_t QD,
@@ -372,8 +406,10 @@ __global__ void __launch_bounds__(128, 3) prefill_attn_h_kernel(const float* __r
     constexpr int C8 = DH / 8;                                  // 16-byte pieces per row
     constexpr int PER = 32 * C8 / 128;                          // pieces per thread, tile and tensor
     extern __shared__ __align__(16) unsigned char sm_raw[];     // ring: [NS][K 32 x RSH | V 32 x RSH] halves
+    pdl_enter();
     __half* smh = reinterpret_cast<__half*>(sm_raw);
-    const uint32_t BT = 64u / REP, nrows = BT * REP, g = blockIdx.y, t0 = blockIdx.x * BT;
+    const uint32_t BT = 64u / REP, nrows = BT * REP, nblk = (T + BT - 1) / BT, kvh = gridDim.x / nblk;
+    const uint32_t g = blockIdx.x % kvh, t0 = (nblk - 1 - blockIdx.x / kvh) * BT;     // the longest rows of every head first
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int fg = lane >> 2, ft = lane & 3;
     const uint32_t t_end = min(T, t0 + BT);
@@ -667,7 +703,7 @@ bool encode_layer(Stack& c, int l, int T, int pos0, cudaStream_t st) {
         return launch_gemm_hh(Ah, Wh, Cm, ldc, Tn, N, K, accumulate, st);
     };
     // 1. norm, q / k / v into one [T][QD + 2 KVD] buffer
-    if (c.resident) rmsnorm_rows_kernel<__half><<<Tn, 256, 0, st>>>(c.x, L.rms1, c.hh, D, c.eps);
+    if (c.resident) launch_pdl(rmsnorm_rows_kernel<__half>, dim3(Tn), dim3(256), 0, st, c.x, L.rms1, c.hh, D, c.eps);
     else rmsnorm_rows_kernel<float><<<Tn, 256, 0, st>>>(c.x, L.rms1, c.h, D, c.eps);
     note_launch();
     if (c.resident) {
@@ -685,9 +721,9 @@ bool encode_layer(Stack& c, int l, int T, int pos0, cudaStream_t st) {
     unsigned tbl_n = 0;
     const float* tbl = lane_rope_table(dh, (unsigned)(pos0 + T), c.theta, &tbl_n);
     if (!tbl) return false;
-    const size_t per_tok = (size_t)(c.H + c.KVH) * (dh / 2) + (size_t)c.KVH * dh;
-    rope_append_kernel<<<(unsigned)(((size_t)T * per_tok + 255) / 256), 256, 0, st>>>(c.qkv, ld, L.kc, L.vc, L.kh, L.vh, (unsigned)c.H, (unsigned)c.KVH, dh,
-                                                                                     (unsigned)c.ctx, (unsigned)pos0, Tn, (const float2*)tbl, tbl_n);
+    const unsigned per_tok = (unsigned)(c.H + c.KVH) * (dh / 8) + (unsigned)c.KVH * dh / 4;
+    launch_pdl(rope_append_kernel, dim3(Tn, (per_tok + 255) / 256), dim3(256), 0, st, c.qkv, ld, L.kc, L.vc, L.kh, L.vh, (unsigned)c.H, (unsigned)c.KVH, dh,
+               (unsigned)c.ctx, (unsigned)pos0, Tn, (const float2*)tbl, tbl_n);
     note_launch();
     cudaEventRecord(L.kv_ready, st);
     cudaStreamWaitEvent(c.copy, L.kv_ready, 0);
@@ -699,13 +735,13 @@ bool encode_layer(Stack& c, int l, int T, int pos0, cudaStream_t st) {
     cudaEventRecord(L.kv_done, c.copy);
     // 3. causal attention of the batch over [0, pos]
     const unsigned BT = 64u / (unsigned)c.REP;
-    const dim3 grid((Tn + BT - 1) / BT, (unsigned)c.KVH);
+    const dim3 grid((unsigned)c.KVH * ((Tn + BT - 1) / BT));
     auto attend = [&](auto dhc, auto* dst) -> bool {
         constexpr int DHC = decltype(dhc)::value;
         using OT = std::remove_pointer_t<decltype(dst)>;
         if (L.kh) {
             if (!attn_h_ready<DHC, OT>()) return false;
-            prefill_attn_h_kernel<DHC, OT><<<grid, 128, attn_h_smem<DHC>(), st>>>(c.qkv, ld, L.kh, L.vh, dst, QD, Tn, (unsigned)pos0, (unsigned)c.ctx, (unsigned)c.REP, scale);
+            launch_pdl(prefill_attn_h_kernel<DHC, OT>, grid, dim3(128), attn_h_smem<DHC>(), st, c.qkv, ld, L.kh, L.vh, dst, QD, Tn, (unsigned)pos0, (unsigned)c.ctx, (unsigned)c.REP, scale);
             return true;
         }
         if (!attn_ready<DHC, OT>()) return false;
@@ -720,7 +756,7 @@ bool encode_layer(Stack& c, int l, int T, int pos0, cudaStream_t st) {
         // activations travel as fp16 between the kernels that make them and the GEMMs that read them (one rounding, the
         // one the GEMM's pre-pass would apply), and the residual adds are the GEMMs' own epilogues
         if (!gemm_h(c.aoh, L.wo, c.x, D, D, QD, true)) return false;
-        rmsnorm_rows_kernel<__half><<<Tn, 256, 0, st>>>(c.x, L.rms2, c.hh, D, c.eps); note_launch();
+        launch_pdl(rmsnorm_rows_kernel<__half>, dim3(Tn), dim3(256), 0, st, c.x, L.rms2, c.hh, D, c.eps); note_launch();
         // gate and up rows are interleaved in wgu: one GEMM whose epilogue writes silu(gate) * up as the fp16 operand
         if (!launch_gemm_hh_silu_mul(c.hh, L.wgu, c.acth, Tn, F, D, st)) return false;
         if (!gemm_h(c.acth, L.wdown, c.x, D, D, F, true)) return false;
