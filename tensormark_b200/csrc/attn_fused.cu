@@ -44,6 +44,10 @@ __device__ __forceinline__ unsigned long long now_ns() {
 __device__ __forceinline__ float rope_lo(float a, float b, float2 cs) { return fmaf(a, cs.x, -__fmul_rn(b, cs.y)); }
 __device__ __forceinline__ float rope_hi(float a, float b, float2 cs) { return fmaf(a, cs.y, __fmul_rn(b, cs.x)); }
 
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 template <typename T> __device__ __forceinline__ T to_cache(float v);
 template <> __device__ __forceinline__ float to_cache<float>(float v) { return v; }
 template <> __device__ __forceinline__ __half to_cache<__half>(float v) { return __float2half_rn(v); }
@@ -187,6 +191,64 @@ template <typename T, int DPL, int REP> struct Tile {
     }
 };
 
+// The same for one tile that lies in shared memory and NH of the query heads: what a warp's first tile comes to in attend(),
+// operation for operation. kt: rows of KST halves, vt: rows of dh.
+template <int DPL, int NH, int KST>
+__device__ __forceinline__ void attend_shared(const __half* kt, const __half* vt, bool live, uint32_t lane, const float (*qs)[DPL * 32], float* sm_m, float* sm_l,
+                                              float (*sm_acc)[DPL * 32]) {
+    constexpr int dh = DPL * 32;
+    float s[NH], pw[NH], acc[NH][DPL];
+#pragma unroll
+    for (int r = 0; r < NH; ++r) {
+        s[r] = 0.f;
+#pragma unroll
+        for (int d = 0; d < DPL; ++d) acc[r][d] = 0.f;
+    }
+#pragma unroll 4
+    for (int c = 0; c < dh / 8; ++c) {
+        Raw8<__half> raw;
+        raw.u = *reinterpret_cast<const uint4*>(kt + lane * KST + c * 8);
+        float kf[8];
+        unpack8(raw, kf);
+#pragma unroll
+        for (int r = 0; r < NH; ++r) {
+            const float4 qa = *reinterpret_cast<const float4*>(&qs[r][c * 8]);
+            const float4 qb = *reinterpret_cast<const float4*>(&qs[r][c * 8 + 4]);
+            float v = s[r];
+            v = fmaf(qa.x, kf[0], v); v = fmaf(qa.y, kf[1], v); v = fmaf(qa.z, kf[2], v); v = fmaf(qa.w, kf[3], v);
+            v = fmaf(qb.x, kf[4], v); v = fmaf(qb.y, kf[5], v); v = fmaf(qb.z, kf[6], v); v = fmaf(qb.w, kf[7], v);
+            s[r] = v;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < NH; ++r) {
+        float tm = live ? s[r] : -CUDART_INF_F;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
+        pw[r] = live ? __expf(s[r] - tm) : 0.f;
+        float ts = pw[r];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) ts += __shfl_xor_sync(0xffffffffu, ts, o);
+        if (lane == 0) { sm_m[r] = tm; sm_l[r] = ts; }
+    }
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+        const RawV<__half, DPL> raw = *reinterpret_cast<const RawV<__half, DPL>*>(vt + k * dh + lane * DPL);
+        float vf[DPL];
+        unpackv(raw, vf);
+#pragma unroll
+        for (int r = 0; r < NH; ++r) {
+            const float w = __shfl_sync(0xffffffffu, pw[r], k);
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) acc[r][d] = fmaf(w, vf[d], acc[r][d]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < NH; ++r)
+#pragma unroll
+        for (int d = 0; d < DPL; ++d) sm_acc[r][lane * DPL + d] = acc[r][d];
+}
+
 template <typename T, int DPL, int REP>
 __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc, T* vc, float* part, float* stat,
                                                           unsigned* counters, float* out, uint32_t H, uint32_t KVH,
@@ -212,9 +274,32 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
     const uint32_t t0 = min(tiles, split * tps), t1 = min(tiles, t0 + tps), used = (tiles + tps - 1) / tps;    // used: splits that have a tile
     const T* kbase = kc + (size_t)kv * ctx * dh;
     const T* vbase = vc + (size_t)kv * ctx * dh;
+    // Splits of one or two tiles (an 8-head fp16 cache: up to 1216 positions) take their tiles through shared memory, and the
+    // warps share the query heads out between them: with a tile per warp three of the four had nothing to do and the fourth
+    // was a chain of REP * 64 dependent steps. Longer splits have a tile for every warp.
+    constexpr int MAXT = sizeof(T) != 2 ? 0 : REP == 8 && DPL == 4 ? 1 : 2, KST = dh + 8;
+    constexpr int NH = REP < 4 ? 1 : REP / 4, GROUPS = REP / NH;
+    __shared__ __align__(16) T kt[MAXT ? MAXT : 1][MAXT ? 32 : 1][KST];
+    __shared__ __align__(16) T vt[MAXT ? MAXT : 1][MAXT ? 32 : 1][dh];
+    const bool shared = tps <= (uint32_t)MAXT;
     const uint32_t t_first = t0 + warp;
     Tile<T, DPL, REP> tile;
-    if (valid && t_first < t1) tile.fetch(kbase, vbase, t_first, allow, lane);
+    if (valid && shared) {
+        constexpr uint32_t C = dh / 8;                         // 16-byte pieces of a row
+        for (uint32_t i = threadIdx.x; i < (t1 - t0) * 32u * C; i += 128) {
+            const uint32_t t = i / (32u * C), r = i / C % 32u, c = i % C, p = (t0 + t) * 32u + r;
+            T *kd = &kt[MAXT ? t : 0][MAXT ? r : 0][8 * c], *vd = &vt[MAXT ? t : 0][MAXT ? r : 0][8 * c];
+            if (p < pos) {
+                cp_async16(kd, kbase + (size_t)p * dh + 8 * c);
+                cp_async16(vd, vbase + (size_t)p * dh + 8 * c);
+            } else if (p > pos) {
+                *reinterpret_cast<uint4*>(kd) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(vd) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+    } else if (valid && t_first < t1) {
+        tile.fetch(kbase, vbase, t_first, allow, lane);
+    }
     const float2 cs = valid ? tbl[(size_t)pos * half + threadIdx.x % half] : make_float2(0.f, 0.f);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tr) tr[1] = now_ns();
@@ -223,7 +308,7 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
     __shared__ __align__(16) float qs[REP][dh];
     __shared__ __align__(16) T knew[dh];
     __shared__ __align__(16) T vnew[dh];
-    __shared__ float sm_acc[4][REP][dh];
+    __shared__ __align__(16) float sm_acc[4][REP][dh];
     __shared__ float sm_m[4][REP], sm_l[4][REP];
     __shared__ float cm[REP][kMaxSplits], inv_l[REP];
     __shared__ int sm_last;
@@ -258,58 +343,77 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
                 kdst[j + half] = knew[j + half] = to_cache<T>(rope_hi(ka, kb, cs));
             }
             if (threadIdx.x < dh) vdst[threadIdx.x] = vnew[threadIdx.x] = to_cache<T>(va);
+            if (shared) {                                      // its row of the tile
+                const uint32_t t = MAXT ? tiles - 1 - t0 : 0u, r = MAXT ? pos % 32u : 0u;
+                if (threadIdx.x < half) { kt[t][r][j] = knew[j]; kt[t][r][j + half] = knew[j + half]; }
+                if (threadIdx.x < dh) vt[t][r][threadIdx.x] = vnew[threadIdx.x];
+            }
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (tr) tr[2] = now_ns();
 
-    tile.attend(kbase, vbase, knew, vnew, t_first, t1, tiles, allow, lane, qs, sm_m[warp], sm_l[warp], sm_acc[warp]);
+    const uint32_t vwarps = shared ? t1 - t0 : 4u;             // partials of the split
+    if constexpr (MAXT != 0) {
+        if (shared) {
+            for (uint32_t i = warp; i < vwarps * GROUPS; i += 4) {
+                const uint32_t t = i / GROUPS, r0 = i % GROUPS * NH;
+                attend_shared<DPL, NH, KST>(&kt[t][0][0], &vt[t][0][0], (t0 + t) * 32u + lane < allow, lane, qs + r0, sm_m[t] + r0, sm_l[t] + r0, sm_acc[t] + r0);
+            }
+        }
+    }
+    if (!shared) tile.attend(kbase, vbase, knew, vnew, t_first, t1, tiles, allow, lane, qs, sm_m[warp], sm_l[warp], sm_acc[warp]);
     if (tr) tr[4] = now_ns();
-    // ---- merge the warps, leave this split's partial
+    // ---- merge the warps, leave this split's partial. A thread takes four dims of one head, here and below: this part of the
+    // kernel runs once, by a few warps, so its time is the latency of its steps and of fetching its code. (Four outputs apart
+    // per thread, unrolled over heads and splits, with a fence by every thread: 2.8 us to the counter and 4.5 behind it.)
     __syncthreads();
+    constexpr int QUADS = REP * dh / 4, NV = (QUADS + 127) / 128;
 #pragma unroll
-    for (int r = 0; r < REP; ++r) {
-        float M = -CUDART_INF_F;
+    for (int n = 0; n < NV; ++n) {
+        const uint32_t q = threadIdx.x + n * 128u, r = q / (dh / 4), d = q % (dh / 4) * 4;
+        if (q < (uint32_t)QUADS) {
+            float M = -CUDART_INF_F;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) M = fmaxf(M, sm_m[w][r]);
-        float Lsum = 0.f, f[4];
+            for (int w = 0; w < 4; ++w) if (w < (int)vwarps) M = fmaxf(M, sm_m[w][r]);
+            float L = 0.f;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            f[w] = sm_m[w][r] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][r] - M);
-            Lsum += f[w] * sm_l[w][r];
+            for (int w = 0; w < 4; ++w)
+                if (w < (int)vwarps) {
+                    const float f = sm_m[w][r] == -CUDART_INF_F ? 0.f : __expf(sm_m[w][r] - M);
+                    const float4 a = *reinterpret_cast<const float4*>(&sm_acc[w][r][d]);
+                    L = fmaf(f, sm_l[w][r], L);
+                    o.x = fmaf(f, a.x, o.x); o.y = fmaf(f, a.y, o.y); o.z = fmaf(f, a.z, o.z); o.w = fmaf(f, a.w, o.w);
+                }
+            const size_t head = (size_t)split * H + kv * REP + r;
+            *reinterpret_cast<float4*>(part + head * dh + d) = o;
+            if (d == 0) *reinterpret_cast<float2*>(stat + head * 2) = make_float2(M, L);
         }
-        const uint32_t head = kv * REP + r;
-        for (int d = threadIdx.x; d < dh; d += 128) {
-            float o = 0.f;
-#pragma unroll
-            for (int w = 0; w < 4; ++w) o += f[w] * sm_acc[w][r][d];
-            part[((size_t)split * H + head) * dh + d] = o;
-        }
-        if (threadIdx.x == 0) { stat[((size_t)split * H + head) * 2] = M; stat[((size_t)split * H + head) * 2 + 1] = Lsum; }
     }
 
     // ---- the CTA that arrives last at this KV head merges the splits
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned prev = atomicAdd(&counters[kv], 1u);
+        unsigned prev;                                        // releases the CTA's partial (the barrier orders it), acquires the others'
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(&counters[kv]) : "memory");
         sm_last = prev == used - 1;
         if (sm_last) counters[kv] = 0u;                       // re-armed for the next launch
     }
     __syncthreads();
     if (tr) { tr[5] = now_ns(); tr[3] = tr[5]; }
     if (!sm_last) return;
-    __threadfence();
-    // The merge is a chain of L2 latencies: BATCH splits of all the outputs of a thread are requested at a time, the first
-    // ones before the weights are known (six splits of one output at a time took 16 round trips, 10 us of the kernel).
-    constexpr int NI = (REP * dh + 127) / 128, BATCH = NI >= 8 ? 4 : 32 / NI;
-    float v[NI][BATCH], o[NI];
+    // BATCH splits are requested at a time, the first ones before the weights are known.
+    constexpr int BATCH = NV > 1 ? 5 : 10;
+    float4 v[NV][BATCH], o[NV];
     auto request = [&](uint32_t s0) {
 #pragma unroll
-        for (int n = 0; n < NI; ++n) {
-            const uint32_t i = min(threadIdx.x + n * 128u, (uint32_t)(REP * dh - 1)), head = kv * REP + i / dh, d = i % dh;
+        for (int n = 0; n < NV; ++n) {
+            const float* from = part + ((size_t)s0 * H + kv * REP) * dh + 4 * (threadIdx.x + n * 128u);
 #pragma unroll
-            for (int k = 0; k < BATCH; ++k) v[n][k] = __ldcg(part + ((size_t)min(s0 + k, used - 1) * H + head) * dh + d);
+            for (int k = 0; k < BATCH; ++k)
+                if (s0 + k < used && threadIdx.x + n * 128u < (uint32_t)QUADS) v[n][k] = __ldcg(reinterpret_cast<const float4*>(from + (size_t)k * H * dh));
         }
     };
     request(0);
@@ -328,20 +432,29 @@ __global__ void __launch_bounds__(128) attn_fused_kernel(const float* qkv, T* kc
     }
     __syncthreads();
 #pragma unroll
-    for (int n = 0; n < NI; ++n) o[n] = 0.f;
+    for (int n = 0; n < NV; ++n) o[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
     for (uint32_t s0 = 0; s0 < used; s0 += BATCH) {
         if (s0) request(s0);
 #pragma unroll
-        for (int n = 0; n < NI; ++n) {
-            const uint32_t r = min(threadIdx.x + n * 128u, (uint32_t)(REP * dh - 1)) / dh;
+        for (int n = 0; n < NV; ++n) {
+            const uint32_t r = min((threadIdx.x + n * 128u) / (dh / 4), (uint32_t)(REP - 1));
 #pragma unroll
-            for (int k = 0; k < BATCH; ++k) if (s0 + k < used) o[n] = __fadd_rn(o[n], __fmul_rn(cm[r][s0 + k], v[n][k]));
+            for (int k = 0; k < BATCH; ++k)
+                if (s0 + k < used) {
+                    const float w = cm[r][s0 + k];
+                    o[n].x = __fadd_rn(o[n].x, __fmul_rn(w, v[n][k].x)); o[n].y = __fadd_rn(o[n].y, __fmul_rn(w, v[n][k].y));
+                    o[n].z = __fadd_rn(o[n].z, __fmul_rn(w, v[n][k].z)); o[n].w = __fadd_rn(o[n].w, __fmul_rn(w, v[n][k].w));
+                }
         }
     }
 #pragma unroll
-    for (int n = 0; n < NI; ++n) {
-        const uint32_t i = threadIdx.x + n * 128u;
-        if (i < (uint32_t)(REP * dh)) out[(size_t)(kv * REP) * dh + i] = o[n] * inv_l[i / dh];
+    for (int n = 0; n < NV; ++n) {
+        const uint32_t q = threadIdx.x + n * 128u;
+        if (q < (uint32_t)QUADS) {
+            const float w = inv_l[q / (dh / 4)];
+            *reinterpret_cast<float4*>(out + (size_t)(kv * REP) * dh + 4 * q) = make_float4(o[n].x * w, o[n].y * w, o[n].z * w, o[n].w * w);
+        }
     }
 }
 
