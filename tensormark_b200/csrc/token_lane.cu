@@ -667,14 +667,15 @@ static void gemv_fused_impl(const char* who, int xslot, size_t xoff, int x_op, i
         if (!u) return;
         f.x2 = (const float*)(u + x2off);
     } else if (x_op != 0) { latch("%s: unknown x transform %d", who, x_op); return; }
-    // Heavy staging (SiLU * up, or a long K) is done once per launch by a small kernel ahead of the GEMV instead of by
-    // every CTA; a GEMV that follows on the same x (k and v after q) reuses the image. Light staging stays in the CTAs:
-    // there the extra dependent kernel costs what it saves.
+    // Long vectors are staged once per launch by a small kernel ahead of the GEMV instead of by every CTA; a GEMV that
+    // follows on the same x (k and v after q) reuses the image. Shorter ones are staged in the CTAs: there the extra
+    // dependent kernel costs more than it saves (SiLU * up of 5632: 1.3 us a layer more, of 14336: 1.0 us less; having the
+    // CTAs of the gate | up GEMV stage the groups they complete cost its tail 2 us, as much as the launch it saved).
     const float* xp = (const float*)(x + xoff);
     float* yp = (float*)(y + yoff);
     State::XImage* used = nullptr;
     const size_t img = xq_bytes(K, dtype);
-    if ((f.x_op == 2 || K >= 8192) && img && img <= kXImageBytes && x_images_ready()) {
+    if (K >= 8192 && img && img <= kXImageBytes && x_images_ready()) {
         if (!(wait_site < 0 && image_holds(s.x_prep, xp, f.x_op, f.x2, eps, K, dtype))) {
             Exchange xw = xc;
             xw.npush = 0;                                    // the staging kernel only waits for the gather, it pushes nothing
