@@ -47,6 +47,9 @@ struct GemvParams {
     // instead of staging x itself. Layout: 16 header words ([0] = the RMSNorm
     // factor as a float, 1.0 when none), then the groups.
     const uint32_t* xq;
+    uint32_t* share;            // the same image, made by this launch's CTAs together (GemvFuse::share)
+    unsigned* share_ctr;
+    uint32_t share_want;        // the counter's value when it is complete
 };
 
 __device__ __forceinline__ const uint8_t* row_ptr(const GemvParams& p, uint32_t row) {
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
         // DRAM latency would sit between the dependency wait and the first row. They do not depend on the preceding
         // kernel: ask for them now. x itself may still be written by the preceding kernel, but L2 is where its writes
         // land: asking for the lines now costs nothing when they are there and saves the DRAM round trip when not.
-        if (!p.xq) {
+        if (!p.xq && !p.share) {
             for (uint32_t i = threadIdx.x * 32u; i < p.K; i += kConsumers * 1024u) {
                 if (p.x_op == 1u) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x2 + i) : "memory");
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + i) : "memory");
@@ -211,6 +214,21 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
                 red[0] = __uint_as_float(__ldcg(p.xq));
                 ok = mbar_wait(xb, 0, &gone);
             }
+        } else if (AL && p.share) {
+            // A part per CTA, read once; the lowest CTAs have them and wait for nobody first, so the others' wait ends as
+            // soon as those have run. (A staging launch ahead of the GEMV cost a second launch and its hand-over: a host
+            // call of 256 x 2048 20.7 us, now 19.6.)
+            (void)stage_groups<DT>(p.share + kXqHeaderWords, nullptr, p.x, nullptr, 0u, p.K, blockIdx.x + (uint32_t)warp * gridDim.x, ge.ngroups,
+                                   (uint32_t)kConsumers * gridDim.x, lane);
+            consumer_sync();
+            if (threadIdx.x == 0) {
+                if (blockIdx.x < ge.ngroups) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.share_ctr) : "memory");
+                ok = wait_counter(p.share_ctr, p.share_want, kWaitLimitNs, nullptr);
+            }
+            consumer_sync();
+            const uint4* from = reinterpret_cast<const uint4*>(p.share + kXqHeaderWords);
+            for (uint32_t i = threadIdx.x; i < ge.ngroups * (uint32_t)kXGroupWords / 4u; i += kConsumers * 32)
+                reinterpret_cast<uint4*>(img)[i] = __ldcg(from + i);
         } else {
             float ss = stage_groups<DT, !AL>(img, img + x_image_bytes(ge.ngroups) / 4u, p.x, p.x2, p.x_op, p.K, (uint32_t)warp, ge.ngroups, (uint32_t)kConsumers, lane);
             if (p.x_op == 1u) {
@@ -435,7 +453,7 @@ template <int DT> bool launch_generic_only(GemvParams p, cudaStream_t st);
 
 // aligned: every row starts on a 16-byte boundary; even: on an even address.
 template <int DT>
-bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st) {
+bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st, unsigned* share_total) {
     p.ge = tile_geom(DT, p.K, aligned);
     const uint32_t fixed = x_smem(p.ge, aligned) + kRingBarBytes;
     if (!aligned) p.xq = nullptr;                           // such an image has two planes
@@ -451,6 +469,10 @@ bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st) {
         if (S > (unsigned)kRingSlots) S = kRingSlots;
         if (S > items) S = items;
         p.slots = S;
+        if (p.share && aligned) {
+            const unsigned parts = p.ge.ngroups < grid ? p.ge.ngroups : grid;
+            p.share_want = *share_total += parts;
+        }
         const size_t smem = fixed + (size_t)S * p.ge.slot_bytes;
         return aligned ? launch_stream<DT, true>(p, grid, smem, st) : launch_stream<DT, false>(p, grid, smem, st);
     }
@@ -475,15 +497,15 @@ bool launch_generic_only(GemvParams p, cudaStream_t st) {
     return check_launch("gemv_generic");
 }
 
-bool launch_any(const GemvParams& p, unsigned dtype, bool aligned, bool even, cudaStream_t st) {
+bool launch_any(const GemvParams& p, unsigned dtype, bool aligned, bool even, cudaStream_t st, unsigned* share_total) {
     switch (dtype) {
-        case DT_Q8_0: return launch_dt<0>(p, aligned, even, st);
-        case DT_Q4_0: return launch_dt<1>(p, aligned, even, st);
-        case DT_Q4_1: return launch_dt<4>(p, aligned, even, st);
-        case DT_Q5_K: return launch_dt<5>(p, aligned, even, st);
-        case DT_Q4_K: return launch_dt<8>(p, aligned, even, st);
-        case DT_GGUF_Q4_0: return launch_dt<9>(p, aligned, even, st);
-        default: return launch_dt<6>(p, aligned, even, st);
+        case DT_Q8_0: return launch_dt<0>(p, aligned, even, st, share_total);
+        case DT_Q4_0: return launch_dt<1>(p, aligned, even, st, share_total);
+        case DT_Q4_1: return launch_dt<4>(p, aligned, even, st, share_total);
+        case DT_Q5_K: return launch_dt<5>(p, aligned, even, st, share_total);
+        case DT_Q4_K: return launch_dt<8>(p, aligned, even, st, share_total);
+        case DT_GGUF_Q4_0: return launch_dt<9>(p, aligned, even, st, share_total);
+        default: return launch_dt<6>(p, aligned, even, st, share_total);
     }
 }
 }  // namespace
@@ -506,7 +528,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
     p.seg = seg; p.status = device_status_word(); p.trace = device_trace();
     p.x2 = nullptr; p.eps = 0.f; p.x_op = 0; p.accumulate = 0;
     p.xc = Exchange{};
-    p.xq = nullptr;
+    p.xq = nullptr; p.share = nullptr; p.share_ctr = nullptr; p.share_want = 0;
     if (fuse && fuse->xchg) p.xc = *fuse->xchg;
     if (p.xc.npush > (unsigned)kMaxPeers || (p.xc.nwait && (!p.xc.wait_ctrs || !p.xc.wait_ctas || !p.xc.epoch)))
         return fail("gemv: incomplete peer exchange description");
@@ -517,6 +539,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
             if ((uintptr_t)fuse->xq % 16) return fail("gemv: the staged x image must be 16-byte aligned");
             p.xq = fuse->xq;
         }
+        if (fuse->share && fuse->x_op == 0) { p.share = fuse->share; p.share_ctr = fuse->share_ctr; }
     }
     bool aligned = ((uintptr_t)W % 16 == 0) && (p.row_bytes % 16 == 0), even = (uintptr_t)W % 2 == 0;
     for (unsigned s = 0; s < seg.nseg; ++s) { aligned = aligned && (seg.woff[s] % 16 == 0); even = even && (seg.woff[s] % 2 == 0); }
@@ -524,7 +547,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
         p.xq = nullptr;
         return launch_generic_only<7>(p, st);
     }
-    return launch_any(p, dtype, aligned, even, st);
+    return launch_any(p, dtype, aligned, even, st, fuse ? fuse->share_total : nullptr);
 }
 
 size_t xq_bytes(unsigned K, unsigned dtype) {

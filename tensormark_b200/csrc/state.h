@@ -62,6 +62,8 @@ struct State {
     // per-tensor host-pointer entries
     std::map<std::pair<const void*, size_t>, uint8_t*> wcache;
     Scratch io_x, io_y, io_big, io_a, io_xq, gemm_ws;
+    unsigned* io_count = nullptr;                               // parts of x staged into io_xq since the counter was zeroed, and
+    unsigned io_total = 0;                                      // what the launches so far add up to
 
     // token lane
     std::vector<Slot> slots;
