@@ -855,9 +855,10 @@ template <int BIAS> __device__ __forceinline__ void half_quad(uint32_t q, uint32
 }
 template <int DT> struct Eight;
 template <> struct Eight<DT_Q4_0> {
+    static constexpr uint32_t N = 8;
     uint32_t d, q;
     __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) { const uint8_t* b = row + (size_t)(t >> 2) * 18u; d = ld16(b); q = ld32(b + 2 + 4 * (t & 3u)); }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ uint4 halves(int) const {
         const uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;                            // byte j: weights 2j and 2j + 1
         uint4 o;
         half_quad<8>(__byte_perm(lo, hi, 0x5140), d, o.x, o.y);
@@ -866,12 +867,13 @@ template <> struct Eight<DT_Q4_0> {
     }
 };
 template <> struct Eight<DT_GGUF_Q4_0> {
+    static constexpr uint32_t N = 8;
     uint32_t d, q0, q1, up;
     __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
         const uint8_t* b = row + (size_t)(t >> 2) * 18u;
         d = ld16(b); q0 = ld32(b + 2 + 8 * (t & 1u)); q1 = ld32(b + 6 + 8 * (t & 1u)); up = 2u * (t & 2u);
     }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ uint4 halves(int) const {
         uint4 o;
         half_quad<8>((q0 >> up) & 0x0F0F0F0Fu, d, o.x, o.y);
         half_quad<8>((q1 >> up) & 0x0F0F0F0Fu, d, o.z, o.w);
@@ -879,12 +881,13 @@ template <> struct Eight<DT_GGUF_Q4_0> {
     }
 };
 template <> struct Eight<DT_Q8_0> {
+    static constexpr uint32_t N = 8;
     uint32_t d, q0, q1;
     __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
         const uint8_t* b = row + (size_t)(t >> 2) * 34u;
         d = ld16(b); q0 = ld32(b + 2 + 8 * (t & 3u)); q1 = ld32(b + 6 + 8 * (t & 3u));
     }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ uint4 halves(int) const {
         uint4 o;
         half_quad<128>(q0 ^ 0x80808080u, d, o.x, o.y);
         half_quad<128>(q1 ^ 0x80808080u, d, o.z, o.w);
@@ -892,13 +895,23 @@ template <> struct Eight<DT_Q8_0> {
     }
 };
 __device__ __forceinline__ float byte_float(uint32_t q, int i) { return __uint2float_rn((q >> (8 * i)) & 255u); }
+// Codes below 64 in the bytes of u, bit 7 of each set: a byte permutation makes 1 + code / 128 of one, an fma a * that + b.
+// With a = 128 s and b = -(128 + offset) s every s * (code - offset) comes out exactly, without a conversion per code.
+__device__ __forceinline__ float code_float(uint32_t u, int i, float a, float b) {
+    return __fmaf_rn(__uint_as_float(__byte_perm(u, 0x3f000000u, 0x7044 | (i << 8))), a, b);
+}
+__device__ __forceinline__ void code_floats(uint32_t u, float a, float b, uint32_t& o01, uint32_t& o23) {
+    o01 = half_pair(code_float(u, 0, a, b), code_float(u, 1, a, b));
+    o23 = half_pair(code_float(u, 2, a, b), code_float(u, 3, a, b));
+}
 template <> struct Eight<DT_Q4_1> {
+    static constexpr uint32_t N = 8;
     uint32_t dm, q0, q1, up;
     __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
         const uint8_t* b = row + (size_t)(t >> 2) * 20u;
         dm = ld32(b); q0 = ld32(b + 4 + 8 * (t & 1u)); q1 = ld32(b + 8 + 8 * (t & 1u)); up = 2u * (t & 2u);
     }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ uint4 halves(int) const {
         const float d = half_bits(dm & 0xffffu), m = half_bits(dm >> 16);
         uint32_t o[4];
 #pragma unroll
@@ -910,6 +923,7 @@ template <> struct Eight<DT_Q4_1> {
     }
 };
 template <bool FIVE> struct EightK {                                     // Q4_K and Q5_K: 32 items per super-block, four per sub-block
+    static constexpr uint32_t N = 8;
     uint32_t dm, s, m, q0, q1, h0, h1, j;
     __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
         const uint8_t* b = row + (size_t)(t >> 5) * (FIVE ? 176u : 144u);
@@ -930,40 +944,47 @@ template <bool FIVE> struct EightK {                                     // Q4_K
         q0 = ld32(q); q1 = ld32(q + 4);
         if (FIVE) { h0 = ld32(b + 16 + l); h1 = ld32(b + 20 + l); }
     }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ uint4 halves(int) const {
         const float d1 = __fmul_rn(half_bits(dm & 0xffffu), __uint2float_rn(s)), m1 = __fmul_rn(half_bits(dm >> 16), __uint2float_rn(m));
         uint32_t o[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            uint32_t c = ((i < 2 ? q0 : q1) >> (4u * (j & 1u))) & 0x0F0F0F0Fu;
+            uint32_t c = (((i < 2 ? q0 : q1) >> (4u * (j & 1u))) & 0x0F0F0F0Fu) | 0x80808080u;
             if (FIVE) c |= (((i < 2 ? h0 : h1) >> j) & 0x01010101u) << 4;
-            o[i] = half_pair(__fsub_rn(__fmul_rn(d1, byte_float(c, 2 * (i & 1))), m1), __fsub_rn(__fmul_rn(d1, byte_float(c, 2 * (i & 1) + 1)), m1));
+            const float a = 128.0f * d1;
+            o[i] = half_pair(__fsub_rn(code_float(c, 2 * (i & 1), a, -a), m1), __fsub_rn(code_float(c, 2 * (i & 1) + 1, a, -a), m1));
         }
         return make_uint4(o[0], o[1], o[2], o[3]);
     }
 };
 template <> struct Eight<DT_Q4_K> : EightK<false> {};
 template <> struct Eight<DT_Q5_K> : EightK<true> {};
-template <> struct Eight<DT_Q6_K> {                                      // eight weights share both scales, the nibble half and the high bits' place
-    uint32_t q0, q1, h0, h1, j;
+template <> struct Eight<DT_Q6_K> {                                      // sixteen: they share both scales, the nibble half and the high bits' place
+    static constexpr uint32_t N = 16;
+    uint32_t q[4], h[4], j;
     float ds;
-    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
-        const uint32_t e = 8u * (t & 31u), h = e >> 7, l = e & 31u;
-        const uint8_t* b = row + (size_t)(t >> 5) * 210u;
-        j = (e >> 5) & 3u;
-        const uint8_t *ql = b + 64 * h + 32 * (j & 1u) + l, *qh = b + 128 + 32 * h + l;
-        q0 = ld32(ql); q1 = ld32(ql + 4); h0 = ld32(qh); h1 = ld32(qh + 4);
-        ds = __fmul_rn(half_bits(ld16(b + 208)), __int2float_rn((int)(int8_t)__ldg(b + 192 + 8 * h + 2 * j + (l >> 4))));
+    __device__ __forceinline__ static void four(const uint8_t* p, uint32_t (&o)[4]) {       // 16 bytes from an even address
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(p - ((uintptr_t)p & 2u));
+        uint32_t v[5];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) v[i] = __ldg(w + i);                 // the fifth word still lies in the block
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = __funnelshift_r(v[i], v[i + 1], 8u * (uint32_t)((uintptr_t)p & 2u));
     }
-    __device__ __forceinline__ uint4 halves() const {
+    __device__ __forceinline__ void load(const uint8_t* row, uint32_t t) {
+        const uint32_t e = 16u * (t & 15u), hf = e >> 7, l = e & 31u;
+        const uint8_t* b = row + (size_t)(t >> 4) * 210u;
+        j = (e >> 5) & 3u;
+        four(b + 64 * hf + 32 * (j & 1u) + l, q);
+        four(b + 128 + 32 * hf + l, h);
+        ds = __fmul_rn(half_bits(ld16(b + 208)), __int2float_rn((int)(int8_t)__ldg(b + 192 + (e >> 4))));
+    }
+    __device__ __forceinline__ uint4 halves(int part) const {
         uint32_t o[4];
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
-            const uint32_t nib = ((w ? q1 : q0) >> (2u * (j & 2u))) & 0x0F0F0F0Fu, code = nib | ((((w ? h1 : h0) >> (2 * j)) & 0x03030303u) << 4);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                o[2 * w + i] = half_pair(__fmul_rn(ds, __int2float_rn((int)((code >> (16 * i)) & 255u) - 32)),
-                                         __fmul_rn(ds, __int2float_rn((int)((code >> (16 * i + 8)) & 255u) - 32)));
+            const uint32_t nib = ((q[2 * part + w] >> (2u * (j & 2u))) & 0x0F0F0F0Fu) | 0x80808080u;
+            code_floats(nib | (((h[2 * part + w] >> (2 * j)) & 0x03030303u) << 4), 128.0f * ds, -160.0f * ds, o[2 * w], o[2 * w + 1]);
         }
         return make_uint4(o[0], o[1], o[2], o[3]);
     }
@@ -972,14 +993,16 @@ template <> struct Eight<DT_Q6_K> {                                      // eigh
 // Both operand conversions of the pre-pass form in one launch: blocks [0, blocks_w) turn weights into fp16, consecutive
 // threads consecutive sixteen-byte words; the remaining blocks round the activations. (The K-quants, Q8_0 and Q4_1 went
 // through the byte-wise fp32 dequantizer and a launch for the activations before: 2000 tokens x 4096 x 4096 Q5_K 120 us,
-// now 77; Q8_0 91, now 72.)
+// now 77; Q8_0 91, now 72. Q6_K takes sixteen weights per thread: its cost is instructions, 32000 x 2048 54 us with eight,
+// 46 with sixteen and without a conversion instruction per code.)
 template <int DT>
 __global__ void __launch_bounds__(256) prepass_f16(const uint8_t* __restrict__ W, uint32_t row_bytes, __half* __restrict__ Wh,
                                                    uint32_t N, uint32_t K, const float* __restrict__ A, __half* __restrict__ Ah,
                                                    size_t n4, uint32_t blocks_w) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // the GEMM may set itself up meanwhile
     if (blockIdx.x >= blocks_w) return round_activations(A, Ah, n4, (size_t)(blockIdx.x - blocks_w) * (256 * kPrepItems) + threadIdx.x);
-    const uint32_t per = K / 8;
+    constexpr uint32_t EN = Eight<DT>::N;                                  // weights per item
+    const uint32_t per = K / EN;
     const uint64_t total = (uint64_t)N * per, first = (uint64_t)blockIdx.x * (256 * kPrepItems) + threadIdx.x;
     Eight<DT> e[kPrepItems];
 #pragma unroll
@@ -993,14 +1016,17 @@ __global__ void __launch_bounds__(256) prepass_f16(const uint8_t* __restrict__ W
 #pragma unroll
     for (int i = 0; i < kPrepItems; ++i) {
         const uint64_t idx = first + (uint64_t)i * 256;
-        if (idx < total) reinterpret_cast<uint4*>(Wh)[idx] = e[i].halves();
+        if (idx < total) {
+#pragma unroll
+            for (uint32_t h = 0; h < EN / 8; ++h) reinterpret_cast<uint4*>(Wh)[idx * (EN / 8) + h] = e[i].halves((int)h);
+        }
     }
 }
 
 // Launches it; false when the type or the address is one it does not take (no error is set then).
 bool try_prepass(const uint8_t* W, uint32_t row_bytes, __half* Wh, unsigned N, unsigned K, const float* A, __half* Ah, size_t n4, unsigned dtype, cudaStream_t st) {
     if ((uintptr_t)W % 2) return false;
-    const unsigned per = 256 * kPrepItems, blocks_w = (unsigned)(((uint64_t)N * (K / 8) + per - 1) / per), grid = blocks_w + (unsigned)((n4 + per - 1) / per);
+    const unsigned per = 256 * kPrepItems, blocks_w = (unsigned)(((uint64_t)N * (K / (dtype == DT_Q6_K ? Eight<DT_Q6_K>::N : 8u)) + per - 1) / per), grid = blocks_w + (unsigned)((n4 + per - 1) / per);
     switch (dtype) {
         case DT_Q4_0: prepass_f16<DT_Q4_0><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
         case DT_GGUF_Q4_0: prepass_f16<DT_GGUF_Q4_0><<<grid, 256, 0, st>>>(W, row_bytes, Wh, N, K, A, Ah, n4, blocks_w); break;
