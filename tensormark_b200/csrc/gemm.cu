@@ -146,29 +146,38 @@ __device__ __forceinline__ uint64_t umma_desc_at(uint32_t lo, uint32_t k) {     
     return ((uint64_t)hi << 32) | (uint64_t)(lo + 2u * k);                        // 32 bytes = 2 units of 16
 }
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (1u << 16); }
+// lead: the lane that issues. The whole warp runs the issuing loop and only the instructions themselves are predicated, so
+// that their operands stay in uniform registers; inside an `if (lane == 0)` every one of them is moved there first.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
 __device__ __forceinline__ bool umma_kblock(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc_first,
-                                            uint64_t* next_bar, uint32_t next_parity) {
+                                            uint64_t* next_bar, uint32_t next_parity, uint32_t lead) {
     const uint32_t la = umma_desc_lo(a), lb = umma_desc_lo(b);
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t"
+        "{\n\t.reg .pred p, q, t, l;\n\t"
         "setp.ne.b32 q, %12, 0;\n\t"
         "setp.eq.b32 t, 0, 0;\n\t"
+        "setp.ne.b32 l, %15, 0;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p, [%13], %14;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %10, q;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %4, %5, %10, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %6, %7, %10, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%1], %8, %9, %10, t;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %10, q;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f16 [%1], %4, %5, %10, t;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f16 [%1], %6, %7, %10, t;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f16 [%1], %8, %9, %10, t;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(tmem_d), "l"(umma_desc_at(la, 0)), "l"(umma_desc_at(lb, 0)), "l"(umma_desc_at(la, 1)), "l"(umma_desc_at(lb, 1)),
           "l"(umma_desc_at(la, 2)), "l"(umma_desc_at(lb, 2)), "l"(umma_desc_at(la, 3)), "l"(umma_desc_at(lb, 3)),
-          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(next_bar)), "r"(next_parity)
+          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(next_bar)), "r"(next_parity), "r"(lead)
         : "memory");
-    return ok != 0;
+    return __all_sync(0xffffffffu, ok != 0);
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t lead) {
+    asm volatile("{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %1, 0;\n\t"
+                 "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lead) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -201,7 +210,7 @@ gemm_f16_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     uint64_t* tempty = tfull + 2;
     uint32_t* tmem_slot = (uint32_t*)(tempty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t num_kb = (K + BK - 1) / BK;
     const uint32_t tiles_n = (n_rows + BM - 1) / BM, tiles_m = (m_tok + bn - 1) / bn, tiles = tiles_n * tiles_m;
     const uint32_t idesc = (1u << 4) | ((bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);      // kIdesc with N = bn
@@ -248,27 +257,26 @@ gemm_f16_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 tma_load_2d(lane == 0 ? a : a + A_BYTES, lane == 0 ? &tmA : &tmB, (int)(kb * BK), lane == 0 ? n0 : m0, &full[s]);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t s = 0, ph = 0, tcount = 0;
-            bool ready = false;                                  // what the probe issued with the previous k-block said
-            for (uint32_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x, ++tcount) {
-                const uint32_t buf = tcount & 1u;
-                if (!mbar_wait(&tempty[buf], ((tcount >> 1) & 1u) ^ 1u)) { dead = true; break; }
+        const uint32_t lead = elect_one();
+        uint32_t s = 0, ph = 0, tcount = 0;
+        bool ready = false;                                  // what the probe issued with the previous k-block said
+        for (uint32_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x, ++tcount) {
+            const uint32_t buf = tcount & 1u;
+            if (!mbar_wait(&tempty[buf], ((tcount >> 1) & 1u) ^ 1u)) { dead = true; break; }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + buf * BN;
+            for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                if (!ready && !mbar_wait(&full[s], ph)) { dead = true; break; }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ready && !mbar_wait(&full[s], ph)) { dead = true; break; }
-                    tc_fence_after();
-                    const uint32_t a = smem_u32(smem) + s * stage_bytes;
-                    uint32_t s1 = s + 1, ph1 = ph;
-                    if (s1 == stages) { s1 = 0; ph1 ^= 1u; }
-                    ready = umma_kblock(d_tmem, a, a + A_BYTES, idesc, kb ? 1u : 0u, &full[s1], ph1);
-                    umma_commit(&empty[s]);            // the stage is free once these MMAs have read it
-                    s = s1; ph = ph1;
-                }
-                if (dead) break;
-                umma_commit(&tfull[buf]);              // accumulator complete
+                const uint32_t a = smem_u32(smem) + s * stage_bytes;
+                uint32_t s1 = s + 1, ph1 = ph;
+                if (s1 == stages) { s1 = 0; ph1 ^= 1u; }
+                ready = umma_kblock(d_tmem, a, a + A_BYTES, idesc, kb ? 1u : 0u, &full[s1], ph1, lead);
+                umma_commit(&empty[s], lead);            // the stage is free once these MMAs have read it
+                s = s1; ph = ph1;
             }
+            if (dead) break;
+            umma_commit(&tfull[buf], lead);              // accumulator complete
         }
     } else {
         const uint32_t q = (uint32_t)warp & 3u;        // TMEM lane quarter this warp may read
@@ -380,23 +388,24 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
 // The MMAs of TWO consecutive stages (eight MMAs) behind probes of the two stages after them: per 64 columns of K the
 // issuing thread spends half a probe and four MMA issues. Bit 0 of the result: bar0's phase is complete, bit 1: bar1's.
 __device__ __forceinline__ uint32_t umma_kblock2_pair(uint32_t tmem_d, uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1, uint32_t idesc,
-                                                      uint32_t acc_first, uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1) {
+                                                      uint32_t acc_first, uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, uint32_t lead) {
     const uint32_t la = umma_desc_lo(a0), lb = umma_desc_lo(b0), la1 = umma_desc_lo(a1), lb1 = umma_desc_lo(b1);
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p0, p1, q, t;\n\t.reg .u32 r0, r1;\n\t"
+        "{\n\t.reg .pred p0, p1, q, t, l;\n\t.reg .u32 r0, r1;\n\t"
         "setp.ne.b32 q, %20, 0;\n\t"
+        "setp.ne.b32 l, %25, 0;\n\t"
         "setp.eq.b32 t, 0, 0;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p0, [%21], %22;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p1, [%23], %24;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, q;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %4, %5, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %6, %7, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %8, %9, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %10, %11, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %12, %13, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %14, %15, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %16, %17, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, q;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %4, %5, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %6, %7, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %8, %9, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %10, %11, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %12, %13, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %14, %15, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %16, %17, %18, {%19, %19, %19, %19, %19, %19, %19, %19}, t;\n\t"
         "selp.u32 r0, 1, 0, p0;\n\t"
         "selp.u32 r1, 2, 0, p1;\n\t"
         "or.b32 %0, r0, r1;\n\t}"
@@ -405,36 +414,38 @@ __device__ __forceinline__ uint32_t umma_kblock2_pair(uint32_t tmem_d, uint32_t 
           "l"(umma_desc_at(la, 2)), "l"(umma_desc_at(lb, 2)), "l"(umma_desc_at(la, 3)), "l"(umma_desc_at(lb, 3)),
           "l"(umma_desc_at(la1, 0)), "l"(umma_desc_at(lb1, 0)), "l"(umma_desc_at(la1, 1)), "l"(umma_desc_at(lb1, 1)),
           "l"(umma_desc_at(la1, 2)), "l"(umma_desc_at(lb1, 2)), "l"(umma_desc_at(la1, 3)), "l"(umma_desc_at(lb1, 3)),
-          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(bar0)), "r"(parity0), "r"(smem_u32(bar1)), "r"(parity1)
+          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(bar0)), "r"(parity0), "r"(smem_u32(bar1)), "r"(parity1), "r"(lead)
         : "memory");
-    return ok;
+    return __reduce_and_sync(0xffffffffu, ok);
 }
 // One stage (a tile's odd last k-block), one probe.
 __device__ __forceinline__ uint32_t umma_kblock_pair(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc_first,
-                                                     uint64_t* next_bar, uint32_t next_parity) {
+                                                     uint64_t* next_bar, uint32_t next_parity, uint32_t lead) {
     const uint32_t la = umma_desc_lo(a), lb = umma_desc_lo(b);
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p, q, t;\n\t"
+        "{\n\t.reg .pred p, q, t, l;\n\t"
+        "setp.ne.b32 l, %15, 0;\n\t"
         "setp.ne.b32 q, %12, 0;\n\t"
         "setp.eq.b32 t, 0, 0;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p, [%13], %14;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, q;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %4, %5, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %6, %7, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%1], %8, %9, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %2, %3, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, q;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %4, %5, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %6, %7, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%1], %8, %9, %10, {%11, %11, %11, %11, %11, %11, %11, %11}, t;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(tmem_d), "l"(umma_desc_at(la, 0)), "l"(umma_desc_at(lb, 0)), "l"(umma_desc_at(la, 1)), "l"(umma_desc_at(lb, 1)),
           "l"(umma_desc_at(la, 2)), "l"(umma_desc_at(lb, 2)), "l"(umma_desc_at(la, 3)), "l"(umma_desc_at(lb, 3)),
-          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(next_bar)), "r"(next_parity)
+          "r"(idesc), "r"(0), "r"(acc_first), "r"(smem_u32(next_bar)), "r"(next_parity), "r"(lead)
         : "memory");
-    return ok;
+    return __reduce_and_sync(0xffffffffu, ok);
 }
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {        // arrives on `bar` at this offset in both CTAs
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t lead) {        // arrives on `bar` at this offset in both CTAs
     const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(both) : "memory");
+    asm volatile("{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %2, 0;\n\t"
+                 "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+                 ::"r"(smem_u32(bar)), "h"(both), "r"(lead) : "memory");
 }
 
 // tmA: box 64 x 128 of the fp16 weights. tmB: box 64 x bn/2 of the fp16 activations. bn: tokens per pair tile, a
@@ -452,7 +463,7 @@ gemm_f16_tn_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint64_t* tempty = tfull + 2;
     uint32_t* tmem_slot = (uint32_t*)(tempty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                     // 0: issues the MMAs and owns full[] and tempty[]
     const uint32_t pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const uint32_t half = bn >> 1;
@@ -497,7 +508,8 @@ gemm_f16_tn_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 tma_load_2d_pair(lane == 0 ? a : a + A_BYTES, lane == 0 ? &tmA : &tmB, (int)(kb * BK), lane == 0 ? n0 : m0, bar);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const uint32_t lead = elect_one();
             uint32_t s = 0, ph = 0, tcount = 0, ready = 0;      // ready: bit 0 / 1 = stage s / the one after it was complete when last probed
             auto next = [&](uint32_t& st, uint32_t& p) { if (++st == stages) { st = 0; p ^= 1u; } };
             for (uint32_t tile = pair; tile < tiles && !dead; tile += npairs, ++tcount) {
@@ -518,18 +530,18 @@ gemm_f16_tn_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         next(s2, ph2);
                         uint32_t s3 = s2, ph3 = ph2;
                         next(s3, ph3);
-                        ready = umma_kblock2_pair(d_tmem, a0, a0 + A_BYTES, a1, a1 + A_BYTES, idesc, kb ? 1u : 0u, &full[s2], ph2, &full[s3], ph3);
-                        umma_commit_pair(&empty[s]);
-                        umma_commit_pair(&empty[s1]);
+                        ready = umma_kblock2_pair(d_tmem, a0, a0 + A_BYTES, a1, a1 + A_BYTES, idesc, kb ? 1u : 0u, &full[s2], ph2, &full[s3], ph3, lead);
+                        umma_commit_pair(&empty[s], lead);
+                        umma_commit_pair(&empty[s1], lead);
                         s = s2; ph = ph2;
                     } else {
-                        ready = umma_kblock_pair(d_tmem, a0, a0 + A_BYTES, idesc, kb ? 1u : 0u, &full[s1], ph1);
-                        umma_commit_pair(&empty[s]);
+                        ready = umma_kblock_pair(d_tmem, a0, a0 + A_BYTES, idesc, kb ? 1u : 0u, &full[s1], ph1, lead);
+                        umma_commit_pair(&empty[s], lead);
                         s = s1; ph = ph1;
                     }
                 }
                 if (dead) break;
-                umma_commit_pair(&tfull[buf]);
+                umma_commit_pair(&tfull[buf], lead);
             }
         }
     } else {
@@ -698,11 +710,11 @@ gemm_q4_tn(const uint8_t* __restrict__ W, uint32_t row_bytes, const __grid_const
                     for (int k = 0; k < BK / UMMA_K; ++k)
                         umma_f16(d_tmem, umma_desc(a + k * UMMA_K * 2), umma_desc(b + k * UMMA_K * 2), kIdesc,
                                  (kb | (uint32_t)k) ? 1u : 0u);
-                    umma_commit(&aempty[sa]);          // both stages are free once these MMAs have read them
-                    umma_commit(&bempty[sb]);
+                    umma_commit(&aempty[sa], 1u);          // both stages are free once these MMAs have read them
+                    umma_commit(&bempty[sb], 1u);
                 }
                 if (dead) break;
-                umma_commit(&tfull[buf]);
+                umma_commit(&tfull[buf], 1u);
             }
         }
     } else if (warp < 6) {
