@@ -6,13 +6,15 @@
 // embed_h_row (2396-2407, tok_embed_h 3260-3271); bf16 has no GPU kernel in the reference (its loader keeps such
 // tensors on the CPU, tensormark/llama.h:4599-4606) and is served by the same kernel here.
 //
-// Bound: HBM, 2 bytes per weight. x is copied into shared memory once per CTA as fp32; a warp owns a row at a time and
-// its lanes read the row as 16-byte pieces (eight weights), four independent loads in flight per lane, fp32 FMA, one
-// shuffle reduction per row. Rows must be 16-byte aligned for that form (K a multiple of 8 and an aligned base);
-// anything else takes a scalar-load kernel with the same arithmetic.
+// Bound: HBM, 2 bytes per weight. x is copied into shared memory once per CTA as fp32; LPR lanes (8, or 1 to 8 warps) share a
+// row and read it as 16-byte pieces (eight weights), eight independent loads in flight per lane, fp32 FMA, one shuffle
+// reduction per warp and row. A CTA's first loads do not depend on x: they are requested before it is waited for. Few rows take more
+// warps each, so that the machine is not left with one row per SM and a chain of loads (105 x 3584: 6.8 us a launch with one, now 3.4; 43913 x 4896: 82.7 us, now 78.6). Rows must be
+// 16-byte aligned for that form (K a multiple of 8 and an aligned base); anything else takes a scalar-load kernel.
 #include "common.cuh"
 
 #include <cuda_fp16.h>
+#include <type_traits>
 
 namespace tmc {
 namespace {
@@ -39,26 +41,54 @@ template <bool BF16> __device__ __forceinline__ float dot8(const uint4 w, const 
     return s;
 }
 
-template <bool BF16>
-__global__ void __launch_bounds__(256) gemv_half_rows(const float* __restrict__ x, const uint16_t* __restrict__ W, float* __restrict__ y,
+template <bool BF16, int LPR>
+__global__ void __launch_bounds__(256, 3) gemv_half_rows(const float* __restrict__ x, const uint16_t* __restrict__ W, float* __restrict__ y,
                                                       uint32_t N, uint32_t K) {
+    constexpr uint32_t ROWS = 256 / LPR, STEP = LPR, U = 8, WPR = LPR / 32;    // WPR 0: several rows per warp
     extern __shared__ __align__(16) float xs[];
+    __shared__ float sums[2][8];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k8 = K / 8, first = threadIdx.x % LPR;
+    uint4 w[U];
+    auto request = [&](uint32_t row, uint32_t i0) {
+        const uint4* wr = reinterpret_cast<const uint4*>(W + (size_t)row * K);
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u)
+            if (i0 + u * STEP < k8) w[u] = __ldg(wr + i0 + u * STEP);
+    };
+    const uint32_t row0 = blockIdx.x * ROWS + threadIdx.x / LPR;
+    if (row0 < N) request(row0, first);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");          // x may come from the preceding kernel of the stream
     for (uint32_t i = threadIdx.x; i < K / 4; i += blockDim.x) reinterpret_cast<float4*>(xs)[i] = __ldcg(reinterpret_cast<const float4*>(x) + i);
     __syncthreads();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k8 = K / 8;
-    for (uint32_t row = blockIdx.x * 8 + warp; row < N; row += gridDim.x * 8) {
-        const uint4* wr = reinterpret_cast<const uint4*>(W + (size_t)row * K);
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t i = lane;
-        for (; i + 96 < k8; i += 128) {                         // four 16-byte loads in flight per lane
-            const uint4 w0 = __ldg(wr + i), w1 = __ldg(wr + i + 32), w2 = __ldg(wr + i + 64), w3 = __ldg(wr + i + 96);
-            acc[0] += dot8<BF16>(w0, xs + 8 * i); acc[1] += dot8<BF16>(w1, xs + 8 * (i + 32));
-            acc[2] += dot8<BF16>(w2, xs + 8 * (i + 64)); acc[3] += dot8<BF16>(w3, xs + 8 * (i + 96));
+    uint32_t turn = 0;
+    for (uint32_t base = blockIdx.x * ROWS; base < N; base += gridDim.x * ROWS, turn ^= 1u) {
+        const uint32_t row = base + threadIdx.x / LPR, next = row + gridDim.x * ROWS;
+        float acc[2] = {0.f, 0.f};
+        if (row < N) {
+            for (uint32_t i = first; i < k8; i += U * STEP) {
+                uint4 v[U];
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u) v[u] = w[u];
+                if (i + U * STEP < k8) request(row, i + U * STEP);
+                else if (next < N) request(next, first);
+#pragma unroll
+                for (uint32_t u = 0; u < U; ++u)
+                    if (i + u * STEP < k8) acc[u & 1] += dot8<BF16>(v[u], xs + 8 * (i + u * STEP));
+            }
+            if (first >= k8 && next < N) request(next, first);
         }
-        for (; i < k8; i += 32) acc[0] += dot8<BF16>(__ldg(wr + i), xs + 8 * i);
-        const float v = warp_total((acc[0] + acc[1]) + (acc[2] + acc[3]));
-        if (lane == 0) y[row] = v;
+        float v = acc[0] + acc[1];
+#pragma unroll
+        for (int o = (LPR < 32 ? LPR : 32) / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if constexpr (WPR > 1) {
+            if (lane == 0) sums[turn][warp] = v;
+            __syncthreads();                                    // the other half of `sums` is free: everybody has passed this barrier once since
+            v = 0.f;
+#pragma unroll
+            for (uint32_t p = 0; p < WPR; ++p) v += sums[turn][warp / WPR * WPR + p];
+        }
+        if (first == 0 && row < N) y[row] = v;
     }
 }
 
@@ -113,18 +143,33 @@ bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsig
     const uint16_t* w = (const uint16_t*)W;
     const size_t smem = (size_t)K * 4;
     if (K % 8 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)x % 16 == 0 && smem <= 200 * 1024) {
-        unsigned grid = (N + 7) / 8;
-        const unsigned cap = (unsigned)device_sm_count() * 4;
-        if (grid > cap) grid = cap;
-        static bool attr[2] = {false, false};
-        if (smem > 48 * 1024 && !attr[bf16]) {
-            const cudaError_t e = bf16 ? cudaFuncSetAttribute(gemv_half_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)
-                                       : cudaFuncSetAttribute(gemv_half_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            if (e != cudaSuccess) return fail("gemv_h: cannot raise the dynamic shared memory limit");
-            attr[bf16] = true;
-        }
-        if (bf16) gemv_half_rows<true><<<grid, 256, smem, st>>>(x, w, y, N, K);
-        else gemv_half_rows<false><<<grid, 256, smem, st>>>(x, w, y, N, K);
+        const unsigned sms = (unsigned)device_sm_count();
+        // One wave: three CTAs per SM by registers, fewer where x is long. A row takes as many warps as leave all CTAs in it, with
+        // four pieces of the row for every lane (one CTA per SM where x is so long that staging it costs as much as the rows);
+        // rows of up to 1024 take eight lanes, so that a lane has as many as it can request, where that fills the machine.
+        const unsigned fit = (unsigned)((224 * 1024) / (smem + 2048)), wave = sms * (fit < 1 ? 1 : fit < 3 ? fit : 3);
+        unsigned lpr = K <= 1024 && N > 32 * sms ? 8 : 32;
+        while (lpr >= 32 && lpr < 256 && (uint64_t)N * lpr * 2 <= 256ull * (smem > 52 * 1024 ? sms : wave) && K / 8 >= 8 * lpr) lpr *= 2;
+        auto launch = [&](auto b, auto parts) {
+            constexpr auto kernel = gemv_half_rows<decltype(b)::value, decltype(parts)::value>;
+            static const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            if (attr != cudaSuccess) return fail("gemv_h: cannot raise the dynamic shared memory limit");
+            const unsigned rows = 256 / lpr, want = (N + rows - 1) / rows;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(want < wave ? want : wave); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at; cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, kernel, x, w, y, (uint32_t)N, (uint32_t)K);
+            return true;
+        };
+        auto pick = [&](auto b) {
+            return lpr == 8 ? launch(b, std::integral_constant<int, 8>{}) : lpr == 32 ? launch(b, std::integral_constant<int, 32>{})
+                 : lpr == 64 ? launch(b, std::integral_constant<int, 64>{}) : lpr == 128 ? launch(b, std::integral_constant<int, 128>{})
+                 : launch(b, std::integral_constant<int, 256>{});
+        };
+        if (!(bf16 ? pick(std::true_type{}) : pick(std::false_type{}))) return false;
     } else {
         if (bf16) gemv_half_generic<true><<<(N + 7) / 8, 256, 0, st>>>(x, w, y, N, K);
         else gemv_half_generic<false><<<(N + 7) / 8, 256, 0, st>>>(x, w, y, N, K);
