@@ -114,7 +114,7 @@ __host__ __device__ inline uint32_t x_smem(const TileGeom& g, bool aligned) { re
 static_assert(kRingBarBytes % 128 == 0, "the ring starts on a 128-byte boundary");
 
 template <int DT, bool AL>
-__global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams p) {
+__global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[kConsumers];
     __shared__ int gone;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
     const uint32_t cta_lo = min(p.N, blockIdx.x * p.rows_per_cta), rows = min(p.N, cta_lo + p.rows_per_cta) - cta_lo;
 
     if (threadIdx.x == 0) {
-        rg.init();
+        rg.init(reducers(DT));
         mbar_init(smem_u32(&xbar), 1);
         gone = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_stream(const GemvParams 
         const uint32_t e0 = p.seg.yoff[0] + cta_lo, x_op = p.x_op, npush = p.xc.npush;
         const bool plain = p.seg.nseg == 1u, add = p.accumulate != 0u;
         RingPos pos{0, 0};
-        reduce(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane,
+        reduce<reducers(DT)>(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane,
                [&] {                                         // the sums of squares are in place since before the first item
                    if (p.xq) {
                        norm_inv = red[0];                    // written with the image by whoever staged it
@@ -438,7 +438,7 @@ bool launch_stream(const GemvParams& p, unsigned grid, size_t smem, cudaStream_t
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kGemvThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(gemv_threads(DT)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;

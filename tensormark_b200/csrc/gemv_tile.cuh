@@ -23,8 +23,11 @@ namespace tmc {
 
 constexpr int kConsumers = 16;                              // warps that multiply
 constexpr int kProducers = 3;                               // warps that issue the row copies
-constexpr int kReducers = 2;                                // warps that add a tile's partial sums and store its rows
-constexpr int kGemvThreads = 32 * (kConsumers + kProducers + kReducers);
+// Warps that add a tile's partial sums and store its rows. Formats that are cheap to multiply go through more tiles per
+// microsecond and want four (Q8_0 32000 x 2048 13.0 -> 12.8 us, Q4_0 28672 x 4096 13.4 -> 13.1, a token of 8B shapes 1 %); the K-quants
+// lose more issue slots to the two extra warps than they gain (Q6_K 128256 x 4096 74.4 -> 76.7).
+__host__ __device__ constexpr int reducers(int dt) { return dt == 5 || dt == 6 || dt == 8 ? 2 : 4; }
+constexpr int gemv_threads(int dt) { return 32 * (kConsumers + kProducers + reducers(dt)); }
 constexpr int kTileRows = 16;
 constexpr int kRingSlots = 16;                              // most slots of a ring (its barriers have fixed places)
 
@@ -188,8 +191,8 @@ struct Ring {
     __device__ __forceinline__ uint32_t full(uint32_t s) const { return bars + 8u * s; }
     __device__ __forceinline__ uint32_t done(uint32_t s) const { return bars + 8u * (kRingSlots + s); }
     __device__ __forceinline__ uint32_t spare(uint32_t s) const { return bars + 8u * (2u * kRingSlots + s); }
-    __device__ __forceinline__ void init() const {          // one thread, before anybody waits
-        for (uint32_t s = 0; s < slots; ++s) { mbar_init(full(s), 1); mbar_init(done(s), kConsumers); mbar_init(spare(s), kReducers); }
+    __device__ __forceinline__ void init(uint32_t reds) const {      // one thread, before anybody waits
+        for (uint32_t s = 0; s < slots; ++s) { mbar_init(full(s), 1); mbar_init(done(s), kConsumers); mbar_init(spare(s), reds); }
     }
 };
 constexpr uint32_t kRingBarBytes = 3 * kRingSlots * 8;
@@ -209,7 +212,7 @@ template <typename F> __device__ __forceinline__ void for_items(const TileGeom& 
 // Producer `mine`: the row copies of every ge.producers-th item. pos starts at parity 1 (the first pass over the ring finds
 // every slot free). rows: how many there are; src(row): its address. The ring has as many slots as producers at least, so
 // a producer that waits for item i's slot has seen item i - slots - producers freed, and with it everything before (a
-// reducer frees in order and both arrive for every item): the phase it waits for is the next one.
+// reducer frees in order and all arrive for every item): the phase it waits for is the next one.
 template <bool AL, typename Src>
 __device__ __forceinline__ bool produce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t row_bytes,
                                         uint32_t mine, int lane, Src src_of) {
@@ -309,12 +312,12 @@ __device__ __forceinline__ bool consume(const Ring& rg, RingPos& pos, const Tile
                             : consume_items<DT, AL, false>(rg, pos, ge, rows, K, img, warp, lane, mis);
 }
 
-// Reducer `mine` of kReducers: tiles mine, mine + kReducers, ... What a reducer does per tile is a chain of latencies (wait,
+// Reducer `mine` of R: tiles mine, mine + R, ... (R >= 2, the tiles that a long row's chunks alternate between.) What a reducer does per tile is a chain of latencies (wait,
 // loads, sums, shuffles, store), and it was the slowest role when both took half of every tile (750 clocks per item;
 // Q4_0 28672 x 4096 13.9 -> 13.1 us, 4096 x 4096 4.6 -> 4.3).
 // store(row, sum) is called by one lane per finished row. ready() is called once, after the first item is through the
 // consumers.
-template <typename Ready, typename Store>
+template <uint32_t R, typename Ready, typename Store>
 __device__ __forceinline__ void reduce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t mine, int lane, Ready ready, Store store) {
     const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, prow = 4u * ge.prow, part0 = rg.at + kTileRows * ge.stride + prow * g + 4u * t;
     const uint32_t kw = ge.kw, ngroups = ge.ngroups, last = ge.nchunks - 1u;
@@ -323,7 +326,7 @@ __device__ __forceinline__ void reduce(const Ring& rg, RingPos& pos, const TileG
     for_items(ge, (rows + kTileRows - 1) / kTileRows, [&](uint32_t tile, uint32_t c, uint32_t) {
         (void)mbar_wait(rg.done(pos.slot), pos.par, rg.gone);      // a consumer that gave up says so itself
         if (first) { first = false; ready(); }
-        if (tile % kReducers == mine) {
+        if (tile % R == mine) {
             const uint32_t part = part0 + pos.slot * rg.slot_bytes, n = min(kw, ngroups - c * kw);
             row_sum(part, part + 8u * prow, n, v0, v1, c == 0u);
             __syncwarp();
