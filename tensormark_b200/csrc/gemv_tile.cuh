@@ -22,7 +22,7 @@
 namespace tmc {
 
 constexpr int kConsumers = 16;                              // warps that multiply
-constexpr int kProducers = 3;                               // warps that issue the row copies
+constexpr int kProducers = 4;                               // warps that issue the row copies (two to four of them do)
 // Warps that add a tile's partial sums and store its rows. Formats that are cheap to multiply go through more tiles per
 // microsecond and want four (Q8_0 32000 x 2048 13.0 -> 12.8 us, Q4_0 28672 x 4096 13.4 -> 13.1, a token of 8B shapes 1 %); the K-quants
 // lose more issue slots to the two extra warps than they gain (Q6_K 128256 x 4096 74.4 -> 76.7).
@@ -69,8 +69,9 @@ inline __host__ __device__ TileGeom tile_geom(unsigned dt, uint32_t K, bool alig
     g.prow = ((g.kw + 7u) & ~7u) * 4u + 4u;                 // four quarters per group of whole steps; the pad spreads the rows over the banks
     // A warp's sixteen row copies take it 0.6-0.7 us: two warps keep up with the HBM rate from 2 KB copies on, shorter ones
     // want a third (Q6_K 128256 x 4096, 1680-byte copies: 81.9 -> 75.0 us; Q4_1 32000 x 2048, 1280: 10.8 -> 9.7), which
-    // only gets in the way of long ones (Q4_0 28672 x 4096, 2304: 13.1 -> 14.1).
-    g.producers = g.chunk_bytes < 2048u ? 3u : 2u;
+    // only gets in the way of long ones (Q4_0 28672 x 4096, 2304: 13.1 -> 14.1). Copies around a kilobyte and below want a
+    // fourth (102687 x 1024 Q4_0, 576 bytes: 22.0 -> 19.5; 81669 x 1792, 1008: 21.0 -> 20.0; Q8_0 54564 x 256, 272: 12.3 -> 10.8).
+    g.producers = g.chunk_bytes < 1200u ? 4u : g.chunk_bytes < 2048u ? 3u : 2u;
     g.slot_bytes = (kTileRows * (g.stride + 4u * g.prow) + 127u) & ~127u;
     return g;
 }
