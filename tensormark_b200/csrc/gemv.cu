@@ -5,7 +5,7 @@
 // 915-1078) and adds the Q8_0 kernel the reference GPU lane lacks.
 //
 // Bound: HBM; every weight byte is read exactly once, at its serialized width. One CTA per SM takes a contiguous range
-// of rows. Two or three producer warps stream it through a ring in shared memory with bulk asynchronous copies (cp.async.bulk
+// of rows. Two to four producer warps stream it through a ring in shared memory with bulk asynchronous copies (cp.async.bulk
 // global -> shared, completion on an mbarrier), so the bytes in flight are set by the ring and no thread ever holds a
 // weight load in a register; sixteen consumer warps multiply on the integer tensor cores (gemv_tile.cuh has the
 // geometry, gemv_lanes.cuh the arithmetic).
