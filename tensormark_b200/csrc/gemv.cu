@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
     rg.at = rg.bars + kRingBarBytes;
     rg.slots = p.slots; rg.slot_bytes = ge.slot_bytes; rg.gone = &gone;
     const uint32_t cta_lo = min(p.N, blockIdx.x * p.rows_per_cta), rows = min(p.N, cta_lo + p.rows_per_cta) - cta_lo;
+    // What the consumers may spend on x before the first row: the peers' limits, one after another, and their own wait for it.
+    const unsigned long long x_ns = 2ull * kWaitLimitNs + p.xc.nwait * p.xc.limit_ns;
 
     if (threadIdx.x == 0) {
         rg.init(reducers(DT));
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
         const uint32_t e0 = p.seg.yoff[0] + cta_lo, x_op = p.x_op, npush = p.xc.npush;
         const bool plain = p.seg.nseg == 1u, add = p.accumulate != 0u;
         RingPos pos{0, 0};
-        reduce<reducers(DT)>(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane,
+        const bool ok = reduce<reducers(DT)>(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane, x_ns,
                [&] {                                         // the sums of squares are in place since before the first item
                    if (p.xq) {
                        norm_inv = red[0];                    // written with the image by whoever staged it
@@ -171,13 +173,14 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
                    y[e] = v;
                    for (uint32_t q = 0; q < npush; ++q) p.xc.peer_y[q][e] = v;      // a sharded model's peers
                });
+        if (!ok && lane == 0) *(volatile int*)p.status = 1;
     } else if (warp >= kConsumers) {
         // The producers touch only weights and run ahead of everything the consumers wait for.
         RingPos pos{0, 1};
         const bool plain = p.seg.nseg == 1u;
         const uint32_t row_bytes = p.row_bytes;
         const uint8_t* const first = p.W + p.seg.woff[0] + (size_t)cta_lo * row_bytes;
-        if (!produce<AL>(rg, pos, ge, rows, row_bytes, (uint32_t)(warp - kConsumers), lane,
+        if (!produce<AL>(rg, pos, ge, rows, row_bytes, (uint32_t)(warp - kConsumers), lane, x_ns,
                          [&](uint32_t row) { return plain ? first + (size_t)row * row_bytes : row_ptr(p, cta_lo + row); }) && lane == 0) {
             *(volatile int*)p.status = 1;
             drain(rg);

@@ -214,14 +214,22 @@ template <typename F> __device__ __forceinline__ void for_items(const TileGeom& 
 // every slot free). rows: how many there are; src(row): its address. The ring has as many slots as producers at least, so
 // a producer that waits for item i's slot has seen item i - slots - producers freed, and with it everything before (a
 // reducer frees in order and all arrive for every item): the phase it waits for is the next one.
+// x_ns: how long the consumers may take for x once the preceding kernel is through; the first slot to come back takes
+// that long. However long the preceding kernel runs, its time is not counted: griddepcontrol.wait comes first.
 template <bool AL, typename Src>
 __device__ __forceinline__ bool produce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t row_bytes,
-                                        uint32_t mine, int lane, Src src_of) {
-    bool ok = true;
+                                        uint32_t mine, int lane, unsigned long long x_ns, Src src_of) {
+    bool ok = true, reused = false;
     uint32_t turn = 0;
     for_items(ge, (rows + kTileRows - 1) / kTileRows, [&](uint32_t tile, uint32_t c, uint32_t) {
         if (turn == mine && ok) {
-            if (!__all_sync(0xffffffffu, mbar_wait(rg.spare(pos.slot), pos.par, rg.gone))) {
+            unsigned long long limit = kWaitLimitNs;
+            if (pos.par == 0u && !reused) {                  // this warp's first item of the ring's second round
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                limit = x_ns;
+                reused = true;
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(rg.spare(pos.slot), pos.par, rg.gone, limit))) {
                 ok = false;
             } else {
                 const uint32_t row = tile * kTileRows + (uint32_t)lane, off = c * ge.chunk_bytes, len = min(ge.chunk_bytes, row_bytes - off);
@@ -317,15 +325,16 @@ __device__ __forceinline__ bool consume(const Ring& rg, RingPos& pos, const Tile
 // loads, sums, shuffles, store), and it was the slowest role when both took half of every tile (750 clocks per item;
 // Q4_0 28672 x 4096 13.9 -> 13.1 us, 4096 x 4096 4.6 -> 4.3).
 // store(row, sum) is called by one lane per finished row. ready() is called once, after the first item is through the
-// consumers.
+// consumers, which takes as long as x (x_ns, see produce). After a wait that ran out nothing is stored any more.
 template <uint32_t R, typename Ready, typename Store>
-__device__ __forceinline__ void reduce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t mine, int lane, Ready ready, Store store) {
+__device__ __forceinline__ bool reduce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t mine, int lane, unsigned long long x_ns,
+                                       Ready ready, Store store) {
     const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, prow = 4u * ge.prow, part0 = rg.at + kTileRows * ge.stride + prow * g + 4u * t;
     const uint32_t kw = ge.kw, ngroups = ge.ngroups, last = ge.nchunks - 1u;
     float v0 = 0.f, v1 = 0.f;                               // rows g and g + 8 of the tile in hand
-    bool first = true;
+    bool first = true, ok = true;
     for_items(ge, (rows + kTileRows - 1) / kTileRows, [&](uint32_t tile, uint32_t c, uint32_t) {
-        (void)mbar_wait(rg.done(pos.slot), pos.par, rg.gone);      // a consumer that gave up says so itself
+        ok = __all_sync(0xffffffffu, mbar_wait(rg.done(pos.slot), pos.par, rg.gone, first ? x_ns : kWaitLimitNs)) && ok;
         if (first) { first = false; ready(); }
         if (tile % R == mine) {
             const uint32_t part = part0 + pos.slot * rg.slot_bytes, n = min(kw, ngroups - c * kw);
@@ -333,12 +342,13 @@ __device__ __forceinline__ void reduce(const Ring& rg, RingPos& pos, const TileG
             __syncwarp();
             mbar_arrive_if(rg.spare(pos.slot), lane == 0);
             const uint32_t row = tile * kTileRows + g + (t << 3);      // lanes 0 and 1 of a row's four have rows g and g + 8
-            if (c == last && t < 2u && row < rows) store(row, t ? v1 : v0);
+            if (ok && c == last && t < 2u && row < rows) store(row, t ? v1 : v0);
         } else {
             mbar_arrive_if(rg.spare(pos.slot), lane == 0);  // in order and for every item, so that a freed slot means that all before it are free
         }
         pos.next(rg.slots);
     });
+    return ok;
 }
 
 }  // namespace tmc
