@@ -80,6 +80,7 @@ constexpr int kXqHeaderWords = 16;
 size_t xq_bytes(unsigned K, unsigned dtype);            // size of such an image; 0 for an unknown format
 
 // ---- kernel launchers (one per .cu) -----------------------------------------
+struct ShareCount;                          // share_count.h
 struct GemvFuse {                           // optional fusions of the decode chain
     unsigned x_op;                          // 0 none, 1 rmsnorm (x2 = weights, eps), 2 silu(x) * x2
     const float* x2;
@@ -89,8 +90,7 @@ struct GemvFuse {                           // optional fusions of the decode ch
     const uint32_t* xq;                     // x (after x_op) already in unit form for this dtype and K; the fp32 x is
                                             // still passed: rows that are not 16-byte aligned take the plain kernel
     uint32_t* share;                        // device scratch of xq_bytes(): x is far away (host memory), so the CTAs stage a part
-    unsigned* share_ctr;                    // of it each and share the image; a device counter of theirs, and the caller's
-    unsigned* share_total;                  // running total of what all launches added to it
+    ShareCount* share_count;                // of it each and share the image, which this counts
 };
 // x (after x_op) in unit form for a GEMV of `dtype`; xchg: wait for a peer gather first.
 bool launch_xprep(uint32_t* out, const float* x, const float* x2, unsigned x_op, float eps, unsigned K, unsigned dtype,

@@ -244,17 +244,19 @@ bool tm_cuda_gemv_q(const float* x, const void* W, float* y, unsigned N, unsigne
         const size_t img = wb / N % 16 == 0 ? xq_bytes(K, dtype) : 0;      // rows off the 16-byte grid are multiplied by a finer image, made in the CTAs
         if (img && cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost && ax.devicePointer &&
             (uintptr_t)ax.devicePointer % 16 == 0) {
-            if (!s.io_count) {
-                if (cudaMalloc(&s.io_count, 256) != cudaSuccess) { cudaGetLastError(); s.io_count = nullptr; return fail("gemv: out of device memory"); }
-                cudaMemsetAsync(s.io_count, 0, 256, s.stream);
-            }
-            const float* xm = (const float*)ax.devicePointer;
+            ShareCount& sc = s.io_share;
             GemvFuse f{};
-            f.share = (uint32_t*)s.io_xq.get(img); f.share_ctr = s.io_count; f.share_total = &s.io_total;
+            f.share = (uint32_t*)s.io_xq.get(img); f.share_count = &sc;
             if (!f.share) return fail("gemv: out of device memory");
-            if (!launch_gemv(xm, dW, dy, N, K, dtype, one_segment(N), s.stream, &f)) return false;
+            if (!sc.level) {
+                if (!sc.parts && cudaMalloc(&sc.parts, 256) != cudaSuccess) { cudaGetLastError(); sc.parts = nullptr; return fail("gemv: out of device memory"); }
+                if (cudaMemsetAsync(sc.parts, 0, 256, s.stream) != cudaSuccess) return check_launch("gemv: clearing a counter");
+                sc.total = 0;
+            }
+            sc.level = false;                                // until the kernel is known to have run
+            if (!launch_gemv((const float*)ax.devicePointer, dW, dy, N, K, dtype, one_segment(N), s.stream, &f)) return false;
             if (!direct && cudaMemcpyAsync(y, dy, (size_t)N * 4, cudaMemcpyDeviceToHost, s.stream) != cudaSuccess) return check_launch("gemv: y download");
-            return sync_stream(s.stream, "gemv");
+            return sc.level = sync_stream(s.stream, "gemv");
         }
         cudaGetLastError();
     }

@@ -20,6 +20,7 @@
 //     kernel with the same per-row arithmetic contract (tolerance-level, not bitwise, agreement).
 #include "common.cuh"
 #include "gemv_tile.cuh"
+#include "share_count.h"
 
 #include <cstdlib>
 
@@ -456,7 +457,7 @@ template <int DT> bool launch_generic_only(GemvParams p, cudaStream_t st);
 
 // aligned: every row starts on a 16-byte boundary; even: on an even address.
 template <int DT>
-bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st, unsigned* share_total) {
+bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st, ShareCount* share) {
     p.ge = tile_geom(DT, p.K, aligned);
     const uint32_t fixed = x_smem(p.ge, aligned) + kRingBarBytes;
     if (!aligned) p.xq = nullptr;                           // such an image has two planes
@@ -472,11 +473,12 @@ bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st, unsigned*
         if (S > (unsigned)kRingSlots) S = kRingSlots;
         if (S > items) S = items;
         p.slots = S;
-        if (p.share && aligned) {
-            const unsigned parts = p.ge.ngroups < grid ? p.ge.ngroups : grid;
-            p.share_want = *share_total += parts;
-        }
         const size_t smem = fixed + (size_t)S * p.ge.slot_bytes;
+        if (p.share && aligned)                             // CTA b makes groups b, b + grid, ...: a part each, while there are groups
+            return share->launch(p.ge.ngroups < grid ? p.ge.ngroups : grid, [&](unsigned want) {
+                p.share_want = want;
+                return launch_stream<DT, true>(p, grid, smem, st);
+            });
         return aligned ? launch_stream<DT, true>(p, grid, smem, st) : launch_stream<DT, false>(p, grid, smem, st);
     }
     return launch_generic_only<DT>(p, st);
@@ -500,15 +502,15 @@ bool launch_generic_only(GemvParams p, cudaStream_t st) {
     return check_launch("gemv_generic");
 }
 
-bool launch_any(const GemvParams& p, unsigned dtype, bool aligned, bool even, cudaStream_t st, unsigned* share_total) {
+bool launch_any(const GemvParams& p, unsigned dtype, bool aligned, bool even, cudaStream_t st, ShareCount* share) {
     switch (dtype) {
-        case DT_Q8_0: return launch_dt<0>(p, aligned, even, st, share_total);
-        case DT_Q4_0: return launch_dt<1>(p, aligned, even, st, share_total);
-        case DT_Q4_1: return launch_dt<4>(p, aligned, even, st, share_total);
-        case DT_Q5_K: return launch_dt<5>(p, aligned, even, st, share_total);
-        case DT_Q4_K: return launch_dt<8>(p, aligned, even, st, share_total);
-        case DT_GGUF_Q4_0: return launch_dt<9>(p, aligned, even, st, share_total);
-        default: return launch_dt<6>(p, aligned, even, st, share_total);
+        case DT_Q8_0: return launch_dt<0>(p, aligned, even, st, share);
+        case DT_Q4_0: return launch_dt<1>(p, aligned, even, st, share);
+        case DT_Q4_1: return launch_dt<4>(p, aligned, even, st, share);
+        case DT_Q5_K: return launch_dt<5>(p, aligned, even, st, share);
+        case DT_Q4_K: return launch_dt<8>(p, aligned, even, st, share);
+        case DT_GGUF_Q4_0: return launch_dt<9>(p, aligned, even, st, share);
+        default: return launch_dt<6>(p, aligned, even, st, share);
     }
 }
 }  // namespace
@@ -542,7 +544,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
             if ((uintptr_t)fuse->xq % 16) return fail("gemv: the staged x image must be 16-byte aligned");
             p.xq = fuse->xq;
         }
-        if (fuse->share && fuse->x_op == 0) { p.share = fuse->share; p.share_ctr = fuse->share_ctr; }
+        if (fuse->share && fuse->x_op == 0) { p.share = fuse->share; p.share_ctr = fuse->share_count->parts; }
     }
     bool aligned = ((uintptr_t)W % 16 == 0) && (p.row_bytes % 16 == 0), even = (uintptr_t)W % 2 == 0;
     for (unsigned s = 0; s < seg.nseg; ++s) { aligned = aligned && (seg.woff[s] % 16 == 0); even = even && (seg.woff[s] % 2 == 0); }
@@ -550,7 +552,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
         p.xq = nullptr;
         return launch_generic_only<7>(p, st);
     }
-    return launch_any(p, dtype, aligned, even, st, fuse ? fuse->share_total : nullptr);
+    return launch_any(p, dtype, aligned, even, st, fuse ? fuse->share_count : nullptr);
 }
 
 size_t xq_bytes(unsigned K, unsigned dtype) {

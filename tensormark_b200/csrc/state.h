@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "share_count.h"
 
 namespace tmc {
 
@@ -62,8 +63,7 @@ struct State {
     // per-tensor host-pointer entries
     std::map<std::pair<const void*, size_t>, uint8_t*> wcache;
     Scratch io_x, io_y, io_big, io_a, io_xq, gemm_ws;
-    unsigned* io_count = nullptr;                               // parts of x staged into io_xq since the counter was zeroed, and
-    unsigned io_total = 0;                                      // what the launches so far add up to
+    ShareCount io_share;                                        // parts of x staged into io_xq
 
     // token lane
     std::vector<Slot> slots;

@@ -112,3 +112,25 @@ __attribute__((visibility("default"))) int hc_pool_gemv(unsigned dtype, const vo
     } catch (...) { return -2; }
 }
 }
+
+// A launch that fails between two that succeed: the total stays what the device counter of a fake device says. 0: it does.
+#include "../../tensormark_b200/csrc/share_count.h"
+extern "C" __attribute__((visibility("default"))) int hc_share_count_selftest() {
+    tmc::ShareCount c;
+    unsigned device = 0;
+    bool fails = false;
+    auto launch = [&](unsigned n) {
+        return c.launch(n, [&](unsigned want) {
+            if (fails) return false;
+            device += n;
+            return want == device;
+        });
+    };
+    if (!launch(8)) return 1;
+    fails = true;
+    if (launch(56)) return 2;
+    fails = false;
+    if (!launch(3) || c.total != device) return 3;
+    c.total = device = ~0u - 1u;                     // and past the counter's end
+    return launch(8) && c.total == 6u ? 0 : 4;
+}

@@ -73,6 +73,10 @@ def test_projection_strategy_contract(hc):
     assert hc.hc_strategy_selftest() == 0
 
 
+def test_failed_launch_is_not_counted(hc):
+    assert hc.hc_share_count_selftest() == 0
+
+
 @pytest.mark.parametrize("dt", [synth.Q4_0, synth.Q5_K])
 def test_gemv_pool_rows(hc, orc, dt):
     n, k = 200, 512                         # 200 rows: three full 64-row chunks and a ragged one
