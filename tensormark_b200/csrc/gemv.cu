@@ -51,6 +51,7 @@ struct GemvParams {
     uint32_t* share;            // the same image, made by this launch's CTAs together (GemvFuse::share)
     unsigned* share_ctr;
     uint32_t share_want;        // the counter's value when it is complete
+    unsigned long long x_ns;            // how long x may take once the preceding kernel is through, and a row after that
 };
 
 __device__ __forceinline__ const uint8_t* row_ptr(const GemvParams& p, uint32_t row) {
@@ -118,7 +119,7 @@ template <int DT, bool AL>
 __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[kConsumers];
-    __shared__ int gone;
+    __shared__ Patience patience;
     __shared__ __align__(8) uint64_t xbar;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned long long* tr = nullptr;                       // this launch's timeline record (CTA 0, thread 0 only)
@@ -136,15 +137,13 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
     Ring rg;
     rg.bars = smem_base(smem) + x_smem(ge, AL);
     rg.at = rg.bars + kRingBarBytes;
-    rg.slots = p.slots; rg.slot_bytes = ge.slot_bytes; rg.gone = &gone;
+    rg.slots = p.slots; rg.slot_bytes = ge.slot_bytes; rg.patience = &patience;
     const uint32_t cta_lo = min(p.N, blockIdx.x * p.rows_per_cta), rows = min(p.N, cta_lo + p.rows_per_cta) - cta_lo;
-    // What the consumers may spend on x before the first row: the peers' limits, one after another, and their own wait for it.
-    const unsigned long long x_ns = 2ull * kWaitLimitNs + p.xc.nwait * p.xc.limit_ns;
 
     if (threadIdx.x == 0) {
         rg.init(reducers(DT));
         mbar_init(smem_u32(&xbar), 1);
-        gone = 0;
+        patience = {0, p.status, p.x_ns};
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
         const uint32_t e0 = p.seg.yoff[0] + cta_lo, x_op = p.x_op, npush = p.xc.npush;
         const bool plain = p.seg.nseg == 1u, add = p.accumulate != 0u;
         RingPos pos{0, 0};
-        const bool ok = reduce<reducers(DT)>(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane, x_ns,
+        reduce<reducers(DT)>(rg, pos, ge, rows, (uint32_t)(warp - kConsumers - kProducers), lane,
                [&] {                                         // the sums of squares are in place since before the first item
                    if (p.xq) {
                        norm_inv = red[0];                    // written with the image by whoever staged it
@@ -174,18 +173,14 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
                    y[e] = v;
                    for (uint32_t q = 0; q < npush; ++q) p.xc.peer_y[q][e] = v;      // a sharded model's peers
                });
-        if (!ok && lane == 0) *(volatile int*)p.status = 1;
     } else if (warp >= kConsumers) {
         // The producers touch only weights and run ahead of everything the consumers wait for.
         RingPos pos{0, 1};
         const bool plain = p.seg.nseg == 1u;
         const uint32_t row_bytes = p.row_bytes;
         const uint8_t* const first = p.W + p.seg.woff[0] + (size_t)cta_lo * row_bytes;
-        if (!produce<AL>(rg, pos, ge, rows, row_bytes, (uint32_t)(warp - kConsumers), lane, x_ns,
-                         [&](uint32_t row) { return plain ? first + (size_t)row * row_bytes : row_ptr(p, cta_lo + row); }) && lane == 0) {
-            *(volatile int*)p.status = 1;
-            drain(rg);
-        }
+        if (!produce<AL>(rg, pos, ge, rows, row_bytes, (uint32_t)(warp - kConsumers), lane,
+                         [&](uint32_t row) { return plain ? first + (size_t)row * row_bytes : row_ptr(p, cta_lo + row); }) && lane == 0) drain(rg);
     } else {
         // RMSNorm weights are read once per token, 4 GB of streamed blocks apart: by then they have left L2, and their
         // DRAM latency would sit between the dependency wait and the first row. They do not depend on the preceding
@@ -209,14 +204,13 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
         if (tr) tr[1] = global_ns();
 
         // x image into shared memory: one bulk copy when it was written once for the whole launch, else staged here
-        bool ok = true;
         if (p.xq) {
             if (threadIdx.x == 0) {
                 const uint32_t xbytes = ge.ngroups * (uint32_t)kXGroupWords * 4u, xb = smem_u32(&xbar);
                 mbar_expect_tx(xb, xbytes);
                 bulk_g2s(smem_u32(img), p.xq + kXqHeaderWords, xbytes, xb);
                 red[0] = __uint_as_float(__ldcg(p.xq));
-                ok = mbar_wait(xb, 0, &gone);
+                if (!mbar_wait(xb, 0, &patience.gone)) *(volatile int*)p.status = 1;
             }
         } else if (AL && p.share) {
             // A part per CTA, read once; the lowest CTAs have them and wait for nobody first, so the others' wait ends as
@@ -227,7 +221,7 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
             consumer_sync();
             if (threadIdx.x == 0) {
                 if (blockIdx.x < ge.ngroups) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.share_ctr) : "memory");
-                ok = wait_counter(p.share_ctr, p.share_want, kWaitLimitNs, nullptr);
+                if (!wait_counter(p.share_ctr, p.share_want, kWaitLimitNs, nullptr)) *(volatile int*)p.status = 1;
             }
             consumer_sync();
             const uint4* from = reinterpret_cast<const uint4*>(p.share + kXqHeaderWords);
@@ -244,9 +238,7 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
         consumer_sync();                                     // the image and the warps' partial sums of squares are in place
         if (tr) tr[2] = global_ns();
         RingPos pos{0, 0};
-        ok = consume<DT, AL>(rg, pos, ge, rows, p.K, smem_base(img), warp, lane,
-                             [&](uint32_t row) { return (uint32_t)(uintptr_t)row_ptr(p, cta_lo + row) & 15u; }) && ok;
-        if (!ok && lane == 0) *(volatile int*)p.status = 1;
+        consume<DT, AL>(rg, pos, ge, rows, p.K, smem_base(img), warp, lane, [&](uint32_t row) { return (uint32_t)(uintptr_t)row_ptr(p, cta_lo + row) & 15u; });
     }
     exchange_signal(p.xc);                                   // sharded models: this CTA's rows are on every peer
     if (tr) tr[3] = global_ns();
@@ -537,6 +529,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
     if (fuse && fuse->xchg) p.xc = *fuse->xchg;
     if (p.xc.npush > (unsigned)kMaxPeers || (p.xc.nwait && (!p.xc.wait_ctrs || !p.xc.wait_ctas || !p.xc.epoch)))
         return fail("gemv: incomplete peer exchange description");
+    p.x_ns = 2ull * kWaitLimitNs + p.xc.nwait * p.xc.limit_ns;      // the peers' limits, one after another, and what the kernel waits for itself
     if (fuse) {
         if (fuse->x_op > 2 || (fuse->x_op != 0 && (!fuse->x2 || (uintptr_t)fuse->x2 % 16))) return fail("gemv: bad fused x transform");
         p.x2 = fuse->x2; p.eps = fuse->eps; p.x_op = fuse->x_op; p.accumulate = fuse->accumulate ? 1u : 0u;

@@ -184,11 +184,41 @@ __device__ __forceinline__ float stage_groups(uint32_t* units, uint32_t* fine, c
 }
 
 // ---- the ring and its three roles ------------------------------------------------------------------------------------
+// What the waits of a CTA's ring share (in shared memory). Producers and reducers may have to wait for as long as the consumers
+// wait for x: for the preceding kernel, whose time does not count, and for the peers of a sharded model. So a wait whose
+// usual limit has passed first lets the preceding kernel end and then gives the rest `ns`. (Looked at only then: most waits
+// come here for a moment, and anything done on the way in is paid for by every slot.) One that runs out says so in the
+// status word.
+struct Patience {
+    int gone;                                               // a wait ran out: nobody waits as long again
+    int* status;
+    unsigned long long ns;
+};
+static __device__ __noinline__ bool ring_wait_slow(uint32_t bar, uint32_t parity, volatile Patience* pt) {
+    if (mbar_try_wait(bar, parity)) return true;
+    unsigned long long t0 = global_ns(), limit = kWaitLimitNs;
+    for (bool last = false;;) {
+        for (int i = 0; i < 64; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (pt->gone) break;
+        if (global_ns() - t0 <= limit) continue;
+        if (last) break;
+        last = true;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        t0 = global_ns();
+        limit = pt->ns;
+    }
+    pt->gone = 1;
+    *(volatile int*)pt->status = 1;
+    return false;
+}
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, Patience* pt) { return mbar_test(bar, parity) || ring_wait_slow(bar, parity, pt); }
+
 struct Ring {
     uint32_t at;                                            // shared-memory address of slot 0
     uint32_t bars;                                          // full[kRingSlots], done[kRingSlots], spare[kRingSlots]
     uint32_t slots, slot_bytes;
-    volatile int* gone;
+    Patience* patience;
     __device__ __forceinline__ uint32_t full(uint32_t s) const { return bars + 8u * s; }
     __device__ __forceinline__ uint32_t done(uint32_t s) const { return bars + 8u * (kRingSlots + s); }
     __device__ __forceinline__ uint32_t spare(uint32_t s) const { return bars + 8u * (2u * kRingSlots + s); }
@@ -214,22 +244,14 @@ template <typename F> __device__ __forceinline__ void for_items(const TileGeom& 
 // every slot free). rows: how many there are; src(row): its address. The ring has as many slots as producers at least, so
 // a producer that waits for item i's slot has seen item i - slots - producers freed, and with it everything before (a
 // reducer frees in order and all arrive for every item): the phase it waits for is the next one.
-// x_ns: how long the consumers may take for x once the preceding kernel is through; the first slot to come back takes
-// that long. However long the preceding kernel runs, its time is not counted: griddepcontrol.wait comes first.
 template <bool AL, typename Src>
 __device__ __forceinline__ bool produce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t row_bytes,
-                                        uint32_t mine, int lane, unsigned long long x_ns, Src src_of) {
-    bool ok = true, reused = false;
+                                        uint32_t mine, int lane, Src src_of) {
+    bool ok = true;
     uint32_t turn = 0;
     for_items(ge, (rows + kTileRows - 1) / kTileRows, [&](uint32_t tile, uint32_t c, uint32_t) {
         if (turn == mine && ok) {
-            unsigned long long limit = kWaitLimitNs;
-            if (pos.par == 0u && !reused) {                  // this warp's first item of the ring's second round
-                asm volatile("griddepcontrol.wait;" ::: "memory");
-                limit = x_ns;
-                reused = true;
-            }
-            if (!__all_sync(0xffffffffu, mbar_wait(rg.spare(pos.slot), pos.par, rg.gone, limit))) {
+            if (!__all_sync(0xffffffffu, ring_wait(rg.spare(pos.slot), pos.par, rg.patience))) {
                 ok = false;
             } else {
                 const uint32_t row = tile * kTileRows + (uint32_t)lane, off = c * ge.chunk_bytes, len = min(ge.chunk_bytes, row_bytes - off);
@@ -256,8 +278,9 @@ __device__ __forceinline__ bool produce(const Ring& rg, RingPos& pos, const Tile
 }
 // After a wait that ran out: copies may still be in flight into this CTA's shared memory; a last bounded chance to land.
 __device__ __forceinline__ void drain(const Ring& rg) {
-    *rg.gone = 0;
-    for (uint32_t s = 0; s < rg.slots; ++s) (void)mbar_wait(rg.full(s), 0, rg.gone, 50000000ull), (void)mbar_wait(rg.full(s), 1, rg.gone, 50000000ull);
+    volatile int* gone = &rg.patience->gone;
+    *gone = 0;
+    for (uint32_t s = 0; s < rg.slots; ++s) (void)mbar_wait(rg.full(s), 0, gone, 50000000ull), (void)mbar_wait(rg.full(s), 1, gone, 50000000ull);
 }
 
 // Consumer warp: multiplies its groups by x (image at shared address img). AL = false: rows on any even address; mis(row)
@@ -265,7 +288,7 @@ __device__ __forceinline__ void drain(const Ring& rg) {
 // rate), so what it needs is in registers and its control is warp-uniform: a wait, the group, an arrival.
 // ONE: a row is one chunk, so a warp multiplies by the same group throughout and keeps it in registers.
 template <int DT, bool AL, bool ONE, typename Mis>
-__device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t K, uint32_t img, int warp, int lane, Mis mis) {
+__device__ __forceinline__ void consume_items(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t K, uint32_t img, int warp, int lane, Mis mis) {
     using L = Lane<DT>;
     const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, kw = ge.kw, team = (uint32_t)warp / kw, wk = (uint32_t)warp % kw;
     const uint32_t ngroups = ge.ngroups, nchunks = ONE ? 1u : ge.nchunks, rw = ge.rw, stride8 = 8u * ge.stride, prow8 = 32u * ge.prow;
@@ -277,13 +300,12 @@ __device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, cons
     const uint32_t src0 = rg.at + g * ge.stride + wk * (uint32_t)L::GB + quarter_off<DT>(t);
     const uint32_t dst0 = rg.at + kTileRows * ge.stride + 4u * (g * ge.prow + 4u * wk + t);
     const uint32_t tiles = (rows + kTileRows - 1) / kTileRows;
-    bool ok = true;
     XRegs x;
     if (ONE) load_x<DT, !AL>(x, xb0, xf0);
     uint32_t tg = 0, c = 0, r = 0, gi = wk, rr = min(rw, tiles);
 #pragma unroll 1
     for (uint32_t left = tiles * nchunks; left; --left) {
-        if (!mbar_wait(rg.full(pos.slot), pos.par, rg.gone)) ok = false;      // the caller reports it; what is multiplied then does not matter
+        (void)ring_wait(rg.full(pos.slot), pos.par, rg.patience);     // when it ran out, what is multiplied does not matter
         if (r == team && (ONE || gi < ngroups)) {
             const uint32_t at = pos.slot * rg.slot_bytes;
             uint32_t r0 = src0 + at, r1 = r0 + stride8;
@@ -313,28 +335,26 @@ __device__ __forceinline__ bool consume_items(const Ring& rg, RingPos& pos, cons
             }
         }
     }
-    return ok;
 }
 template <int DT, bool AL, typename Mis>
-__device__ __forceinline__ bool consume(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t K, uint32_t img, int warp, int lane, Mis mis) {
-    return ge.nchunks == 1u ? consume_items<DT, AL, true>(rg, pos, ge, rows, K, img, warp, lane, mis)
-                            : consume_items<DT, AL, false>(rg, pos, ge, rows, K, img, warp, lane, mis);
+__device__ __forceinline__ void consume(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t K, uint32_t img, int warp, int lane, Mis mis) {
+    if (ge.nchunks == 1u) consume_items<DT, AL, true>(rg, pos, ge, rows, K, img, warp, lane, mis);
+    else consume_items<DT, AL, false>(rg, pos, ge, rows, K, img, warp, lane, mis);
 }
 
 // Reducer `mine` of R: tiles mine, mine + R, ... (R >= 2, the tiles that a long row's chunks alternate between.) What a reducer does per tile is a chain of latencies (wait,
 // loads, sums, shuffles, store), and it was the slowest role when both took half of every tile (750 clocks per item;
 // Q4_0 28672 x 4096 13.9 -> 13.1 us, 4096 x 4096 4.6 -> 4.3).
 // store(row, sum) is called by one lane per finished row. ready() is called once, after the first item is through the
-// consumers, which takes as long as x (x_ns, see produce). After a wait that ran out nothing is stored any more.
+// consumers.
 template <uint32_t R, typename Ready, typename Store>
-__device__ __forceinline__ bool reduce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t mine, int lane, unsigned long long x_ns,
-                                       Ready ready, Store store) {
+__device__ __forceinline__ void reduce(const Ring& rg, RingPos& pos, const TileGeom& ge, uint32_t rows, uint32_t mine, int lane, Ready ready, Store store) {
     const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u, prow = 4u * ge.prow, part0 = rg.at + kTileRows * ge.stride + prow * g + 4u * t;
     const uint32_t kw = ge.kw, ngroups = ge.ngroups, last = ge.nchunks - 1u;
     float v0 = 0.f, v1 = 0.f;                               // rows g and g + 8 of the tile in hand
-    bool first = true, ok = true;
+    bool first = true;
     for_items(ge, (rows + kTileRows - 1) / kTileRows, [&](uint32_t tile, uint32_t c, uint32_t) {
-        ok = __all_sync(0xffffffffu, mbar_wait(rg.done(pos.slot), pos.par, rg.gone, first ? x_ns : kWaitLimitNs)) && ok;
+        (void)ring_wait(rg.done(pos.slot), pos.par, rg.patience);
         if (first) { first = false; ready(); }
         if (tile % R == mine) {
             const uint32_t part = part0 + pos.slot * rg.slot_bytes, n = min(kw, ngroups - c * kw);
@@ -342,13 +362,12 @@ __device__ __forceinline__ bool reduce(const Ring& rg, RingPos& pos, const TileG
             __syncwarp();
             mbar_arrive_if(rg.spare(pos.slot), lane == 0);
             const uint32_t row = tile * kTileRows + g + (t << 3);      // lanes 0 and 1 of a row's four have rows g and g + 8
-            if (ok && c == last && t < 2u && row < rows) store(row, t ? v1 : v0);
+            if (c == last && t < 2u && row < rows) store(row, t ? v1 : v0);
         } else {
             mbar_arrive_if(rg.spare(pos.slot), lane == 0);  // in order and for every item, so that a freed slot means that all before it are free
         }
         pos.next(rg.slots);
     });
-    return ok;
 }
 
 }  // namespace tmc
