@@ -52,6 +52,7 @@ struct GemvParams {
     unsigned* share_ctr;
     uint32_t share_want;        // the counter's value when it is complete
     unsigned long long x_ns;            // how long x may take once the preceding kernel is through, and a row after that
+    unsigned long long share_ns;        // how long a CTA waits for the others' parts
 };
 
 __device__ __forceinline__ const uint8_t* row_ptr(const GemvParams& p, uint32_t row) {
@@ -213,20 +214,26 @@ __global__ void __launch_bounds__(gemv_threads(DT), 1) gemv_stream(const GemvPar
                 if (!mbar_wait(xb, 0, &patience.gone)) *(volatile int*)p.status = 1;
             }
         } else if (AL && p.share) {
-            // A part per CTA, read once; the lowest CTAs have them and wait for nobody first, so the others' wait ends as
-            // soon as those have run. (A staging launch ahead of the GEMV cost a second launch and its hand-over: a host
-            // call of 256 x 2048 20.7 us, now 19.6.)
+            // A part per CTA, read once. The lowest CTAs have them and wait for nobody before they make theirs; the image is
+            // complete a few microseconds after the last of those has started. When that is depends on what else the GPU
+            // runs (another stream's kernel may hold its SM), so a CTA whose patience (share_ns) ends stages all of x for
+            // itself: 4 K more bytes over PCIe, the same bits. (A staging launch ahead of the GEMV cost a second launch and
+            // its hand-over: a host call of 256 x 2048 20.7 us, now 19.6.)
             (void)stage_groups<DT>(p.share + kXqHeaderWords, nullptr, p.x, nullptr, 0u, p.K, blockIdx.x + (uint32_t)warp * gridDim.x, ge.ngroups,
                                    (uint32_t)kConsumers * gridDim.x, lane);
             consumer_sync();
             if (threadIdx.x == 0) {
                 if (blockIdx.x < ge.ngroups) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.share_ctr) : "memory");
-                if (!wait_counter(p.share_ctr, p.share_want, kWaitLimitNs, nullptr)) *(volatile int*)p.status = 1;
+                red[0] = p.share_ns && wait_counter(p.share_ctr, p.share_want, p.share_ns, nullptr) ? 1.f : 0.f;
             }
             consumer_sync();
-            const uint4* from = reinterpret_cast<const uint4*>(p.share + kXqHeaderWords);
-            for (uint32_t i = threadIdx.x; i < ge.ngroups * (uint32_t)kXGroupWords / 4u; i += kConsumers * 32)
-                reinterpret_cast<uint4*>(img)[i] = __ldcg(from + i);
+            if (red[0] != 0.f) {
+                const uint4* from = reinterpret_cast<const uint4*>(p.share + kXqHeaderWords);
+                for (uint32_t i = threadIdx.x; i < ge.ngroups * (uint32_t)kXGroupWords / 4u; i += kConsumers * 32)
+                    reinterpret_cast<uint4*>(img)[i] = __ldcg(from + i);
+            } else {
+                (void)stage_groups<DT>(img, nullptr, p.x, nullptr, 0u, p.K, (uint32_t)warp, ge.ngroups, (uint32_t)kConsumers, lane);
+            }
         } else {
             float ss = stage_groups<DT, !AL>(img, img + x_image_bytes(ge.ngroups) / 4u, p.x, p.x2, p.x_op, p.K, (uint32_t)warp, ge.ngroups, (uint32_t)kConsumers, lane);
             if (p.x_op == 1u) {
@@ -525,7 +532,7 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
     p.seg = seg; p.status = device_status_word(); p.trace = device_trace();
     p.x2 = nullptr; p.eps = 0.f; p.x_op = 0; p.accumulate = 0;
     p.xc = Exchange{};
-    p.xq = nullptr; p.share = nullptr; p.share_ctr = nullptr; p.share_want = 0;
+    p.xq = nullptr; p.share = nullptr; p.share_ctr = nullptr; p.share_want = 0; p.share_ns = 0;
     if (fuse && fuse->xchg) p.xc = *fuse->xchg;
     if (p.xc.npush > (unsigned)kMaxPeers || (p.xc.nwait && (!p.xc.wait_ctrs || !p.xc.wait_ctas || !p.xc.epoch)))
         return fail("gemv: incomplete peer exchange description");
@@ -537,7 +544,9 @@ bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigne
             if ((uintptr_t)fuse->xq % 16) return fail("gemv: the staged x image must be 16-byte aligned");
             p.xq = fuse->xq;
         }
-        if (fuse->share && fuse->x_op == 0) { p.share = fuse->share; p.share_ctr = fuse->share_count->parts; }
+        // TM_GEMV_SHARE_WAIT_US: 0 has every CTA stage x for itself
+        static const unsigned long long share_ns = [] { const char* e = std::getenv("TM_GEMV_SHARE_WAIT_US"); return e && *e ? 1000ull * std::strtoul(e, nullptr, 10) : 200000ull; }();
+        if (fuse->share && fuse->x_op == 0) { p.share_ns = share_ns; p.share = fuse->share; p.share_ctr = fuse->share_count->parts; }
     }
     bool aligned = ((uintptr_t)W % 16 == 0) && (p.row_bytes % 16 == 0), even = (uintptr_t)W % 2 == 0;
     for (unsigned s = 0; s < seg.nseg; ++s) { aligned = aligned && (seg.woff[s] % 16 == 0); even = even && (seg.woff[s] % 2 == 0); }

@@ -3,6 +3,9 @@ that outlives the call."""
 from __future__ import annotations
 
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -15,6 +18,35 @@ pytestmark = pytest.mark.gpu
 
 def pinned(torch, a: np.ndarray):
     return torch.from_numpy(a).pin_memory()
+
+
+def check_call(cuda, torch, orc, dt, n, k, seed):
+    W, x = synth.make_weights(dt, n, k, seed=seed), synth.make_activations(k, seed=seed + 1)
+    xp, yp = pinned(torch, x), torch.full((n,), float("nan")).pin_memory()
+    lib.check(cuda.tm_cuda_gemv_q(ptr(xp), W.ctypes.data, ptr(yp), n, k, dt), "tm_cuda_gemv_q")
+    cuda.tm_cuda_release_weights()
+    y64, yabs = orc.gemv_f64(dt, W, x, n, k)
+    assert np.all(np.abs(yp.numpy() - y64) <= 1e-4 * yabs), (dt, n, k)
+    return yp.numpy().copy()
+
+
+def test_cta_that_does_not_wait_for_the_others(cuda, torch_mod, orc):
+    """A CTA that has waited long enough stages x for itself, with the same bits: here one whose patience is nil, in a child."""
+    shapes = [(synth.Q4_0, 256, 2048), (synth.Q8_0, 40, 14336), (synth.Q6_K, 3000, 2048)]
+    want = [check_call(cuda, torch_mod, orc, dt, n, k, seed=30) for dt, n, k in shapes]
+    code = ("import numpy as np, torch\n"
+            "from oracle import binding\n"
+            "from tensormark_b200 import lib\n"
+            "from tests.test_gpu_host_gemv import check_call\n"
+            "L = lib.load()\n"
+            "lib.check(L.tm_cuda_init(-1), 'tm_cuda_init')\n"
+            f"for dt, n, k in {shapes}:\n"
+            "    print(check_call(L, torch, binding.oracle(), dt, n, k, seed=30).tobytes().hex())\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, TM_GEMV_SHARE_WAIT_US="0"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    for line, w in zip(r.stdout.split(), want, strict=True):
+        assert np.array_equal(np.frombuffer(bytes.fromhex(line), np.float32), w)
 
 
 def test_call_that_never_ran(cuda, torch_mod, orc):
