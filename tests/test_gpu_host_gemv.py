@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from tensormark_b200 import lib, synth
-from tests.gpu_util import ptr
+from tests.gpu_util import dev_bytes, dev_f32, gemv_dev, ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +66,31 @@ def test_call_that_never_ran(cuda, torch_mod, orc):
     assert np.array_equal(yp.numpy(), want)
     y64, yabs = orc.gemv_f64(dt, W, x, n, k)
     assert np.all(np.abs(want - y64) <= 1e-4 * yabs)
+
+
+def test_calls_in_a_row(cuda, torch_mod, orc):
+    """One process, page-locked x and y: formats, fewer and more groups of x than CTAs, a K that is no multiple of 256, a
+    scratch buffer that grows and is then larger than needed, x changed between two calls, pageable calls in between. Bits are
+    those of the entry with device pointers."""
+    torch = torch_mod
+    shapes = [(synth.Q4_0, 256, 2048), (synth.Q8_0, 1, 14336), (synth.Q4_1, 40, 14336), (synth.Q4_1, 5632, 2176), (synth.Q6_K, 300, 2048),
+              (synth.Q4_0, 17, 256), (synth.GGUF_Q4_0, 9000, 4096), (synth.Q5_K, 7, 14336), (synth.Q4_0, 130, 352), (synth.Q4_K, 148, 512), (synth.Q8_0, 20, 28672)]
+    keep = []                                    # copies on the device go by host address
+    for i, (dt, n, k) in enumerate(shapes):
+        W = synth.make_weights(dt, n, k, seed=40 + i)
+        keep.append(W)
+        Wd = dev_bytes(torch, W)
+        xp, yp = pinned(torch, np.empty(k, np.float32)), torch.empty(n).pin_memory()
+        for again in range(3):
+            x = synth.make_activations(k, seed=60 + 10 * i + again)
+            want = gemv_dev(cuda, torch, dt, Wd, dev_f32(torch, x), n, k)
+            xp.copy_(torch.from_numpy(x))
+            yp.fill_(float("nan"))
+            lib.check(cuda.tm_cuda_gemv_q(ptr(xp), W.ctypes.data, ptr(yp), n, k, dt), "tm_cuda_gemv_q")
+            assert np.array_equal(yp.numpy(), want), (dt, n, k)
+            if again == 1:
+                y = np.empty(n, np.float32)
+                lib.check(cuda.tm_cuda_gemv_q(x.ctypes.data, W.ctypes.data, y.ctypes.data, n, k, dt), "tm_cuda_gemv_q")
+                assert np.array_equal(y, want)
+        y64, yabs = orc.gemv_f64(dt, W, x, n, k)
+        assert np.all(np.abs(want - y64) <= 1e-4 * yabs), (dt, n, k)
