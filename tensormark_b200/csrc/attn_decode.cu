@@ -111,8 +111,10 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
     __shared__ __align__(16) float pbuf[NW][PW][REP];                        // a warp's weights of its positions
     __shared__ __align__(16) float cbuf[NW][REP];                            // its correction factors
     __shared__ float sm_m[NW][REP], sm_l[NW][REP];
+    __shared__ __align__(16) uint4 nothing;                                  // what a lane without a row multiplies its weight 0 by
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
+        nothing = make_uint4(0u, 0u, 0u, 0u);
         for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&bars[s]), 1); mbar_init(smem_u32(&bars[kStages + s]), NW); }
         gone = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -172,7 +174,7 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
             const uint32_t np = min((uint32_t)TP, p1 - p0 - t * TP);         // positions of this stage
             if (!mbar_wait(full + 8u * s, par, &gone)) ok = false;
             const uint32_t at = ring + s * 2u * HALF;
-            uint32_t off[kLoads];                                            // rows past the end: the last row again, with weight 0
+            uint32_t off[kLoads];                                            // rows past the end: the last row's K again, whose score is dropped
 #pragma unroll
             for (int i = 0; i < kLoads; ++i) {
                 const uint32_t pos = (uint32_t)(warp * kLoads + i) * RW + rg;
@@ -259,8 +261,8 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
             }
 #pragma unroll
             for (int i = 0; i < kLoads; ++i) {
-                uint64_t v2[NP];
-                Elems<T>::pairs(lds16(at + HALF + off[i]), v2);
+                uint64_t v2[NP];                                             // past the end zeros: the last row's V may be infinite
+                Elems<T>::pairs(lds16((uint32_t)(warp * kLoads + i) * RW + rg < np ? at + HALF + off[i] : smem_u32(&nothing)), v2);
                 float pw[REP];
                 if constexpr (REP % 4 == 0) {
 #pragma unroll

@@ -13,11 +13,13 @@ from tests.gpu_util import dev_f32, ptr, stream_ptr
 pytestmark = pytest.mark.gpu
 
 
-def run(cuda, torch, orc, KVH, rep, dh, ctx, allow, half, off=0):
+def run(cuda, torch, orc, KVH, rep, dh, ctx, allow, half, off=0, last_v=None):
     rng = np.random.default_rng(allow + rep)
     H, scale = KVH * rep, 1.0 / np.sqrt(dh)
     q = rng.standard_normal((H, dh)).astype(np.float32) * 2
     kv = rng.standard_normal((2, KVH, ctx, dh)).astype(np.float16 if half else np.float32)
+    if last_v is not None:
+        kv[1, :, allow - 1, ::3] = last_v
     qd = dev_f32(torch, q)
     flat = [torch.zeros(kv[0].size + 8, dtype=torch.float16 if half else torch.float32, device="cuda") for _ in range(2)]
     for t, a in zip(flat, kv):
@@ -55,3 +57,12 @@ def test_ranges_around_a_stage(cuda, torch_mod, orc, KVH, rep, allow):
 def test_caches_off_the_grid(cuda, torch_mod, orc, half):
     run(cuda, torch_mod, orc, 2, 4, 128, 300, 257, half, off=1)
     run(cuda, torch_mod, orc, 3, 8, 64, 300, 300, half, off=3)
+
+
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("rep,dh", [(1, 128), (4, 64), (8, 128)])
+def test_infinite_values(cuda, torch_mod, orc, rep, dh, half):
+    """A value that overflowed its cache: the dims that it is in are infinite, not the product of nothing and infinity."""
+    for allow in (1, 33, 1000):
+        run(cuda, torch_mod, orc, 2, rep, dh, 1024, allow, half, last_v=np.inf)
+        run(cuda, torch_mod, orc, 2, rep, dh, 1024, allow, half, last_v=-np.inf)
