@@ -1264,8 +1264,9 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
     // Up to 512 tokens straight from the blocks: a weight is then converted at most twice, in the shadow of the copies. From
     // there on converting once for all token tiles is cheaper (4096 x 4096, blocks / fp16 copy: 512 tokens Q4_0 36 / 40,
     // Q6_K 44 / 44 us; 1000 tokens Q4_0 54 / 48, Q6_K 75 / 52 us). The knobs of the fp16 kernels keep a call on them.
+    // The kernels sum in different orders, so sizes choose and not what the caller's scratch has room for beyond its need.
     static const bool fp16_only = std::getenv("TM_GEMM_FUSED") || std::getenv("TM_GEMM_PAIR") || std::getenv("TM_GEMM_BN");
-    if (M <= 512 && may_permute_k && !fp16_only && gemm_blocks_takes(W, M, N, K, dtype, workspace_bytes))
+    if (M <= 512 && may_permute_k && !fp16_only && gemm_blocks_takes(W, M, N, K, dtype, gemm_workspace_bytes(M, N, K)))
         return launch_gemm_blocks(A, W, C, ldc, M, N, K, dtype, workspace, st);
 
     // Q4_0 with K a multiple of 256 and 16-byte aligned rows can be dequantized inside the GEMM (gemm_q4_tn).

@@ -49,3 +49,25 @@ def test_edges(cuda, torch_mod, orc, dt, m, n, k, shift):
     absum = np.abs(A) @ np.abs(orc.dequant(dt, W, n * k).reshape(n, k)).T
     err = np.abs(got[:m] - ref)
     assert np.all(err <= 1e-3 * absum), float((err / absum).max())
+
+
+@pytest.mark.parametrize("dt,m,n,k", [(synth.Q4_0, 512, 32, 288), (synth.Q8_0, 400, 16, 96), (synth.Q4_0, 512, 300, 1024), (synth.Q4_0, 300, 130, 64)])
+def test_scratch_size_does_not_choose_the_kernel(cuda, torch_mod, orc, dt, m, n, k):
+    """A call's bits come from its operands: also where the fp16 tokens, K rounded up to 64, need more than the scratch that
+    the call asks for."""
+    torch = torch_mod
+    W, A = synth.make_weights(dt, n, k, seed=24), synth.make_activations((m, k), seed=25)
+    Wd = torch.from_numpy(np.ascontiguousarray(np.concatenate([W.reshape(-1), np.zeros(32, np.uint8)]))).cuda()
+    Ad = dev_f32(torch, A)
+    need = cuda.tm_cuda_sgemm_q_workspace(m, n, k, dt)
+    ws = torch.empty(2 * need + (1 << 20), dtype=torch.uint8, device="cuda")
+    base = C.c_void_p((ws.data_ptr() + 255) // 256 * 256)
+    got = []
+    for size in (need, 2 * need + (1 << 19)):
+        Cd = torch.empty((m, n), dtype=torch.float32, device="cuda")
+        lib.check(cuda.tm_cuda_sgemm_q_dev(ptr(Ad), ptr(Wd), ptr(Cd), m, n, k, dt, base, size, stream_ptr(torch)), "tm_cuda_sgemm_q_dev")
+        torch.cuda.synchronize()
+        got.append(Cd.cpu().numpy())
+    assert np.array_equal(got[0], got[1])
+    absum = np.abs(A) @ np.abs(orc.dequant(dt, W, n * k).reshape(n, k)).T
+    assert np.all(np.abs(got[0] - orc.gemm(dt, W, A, m, n, k, threads=4)) <= 1e-3 * absum)
