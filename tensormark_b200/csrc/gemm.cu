@@ -1265,7 +1265,9 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
     // there on converting once for all token tiles is cheaper (4096 x 4096, blocks / fp16 copy: 512 tokens Q4_0 36 / 40,
     // Q6_K 44 / 44 us; 1000 tokens Q4_0 54 / 48, Q6_K 75 / 52 us). The knobs of the fp16 kernels keep a call on them.
     // The kernels sum in different orders, so sizes choose and not what the caller's scratch has room for beyond its need.
-    static const bool fp16_only = std::getenv("TM_GEMM_FUSED") || std::getenv("TM_GEMM_PAIR") || std::getenv("TM_GEMM_BN");
+    auto knob = [](const char* name, int unset) { const char* e = std::getenv(name); return e && *e ? std::atoi(e) : unset; };
+    static const bool allow_fused = knob("TM_GEMM_FUSED", 0) == 1;
+    static const bool fp16_only = allow_fused || knob("TM_GEMM_PAIR", -1) >= 0 || knob("TM_GEMM_BN", 0) > 0;
     if (M <= 512 && may_permute_k && !fp16_only && gemm_blocks_takes(W, M, N, K, dtype, gemm_workspace_bytes(M, N, K)))
         return launch_gemm_blocks(A, W, C, ldc, M, N, K, dtype, workspace, st);
 
@@ -1273,7 +1275,6 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
     // TM_GEMM_FUSED=1 selects it; the default is the pre-pass, which is the faster of the two today
     // (2000 x 5632 x 2048: 72 us for pre-passes + TMA-fed kernel against 77 us for the producer-fed kernel,
     // whose tensor pipe is 30 % busy with the producers stalled on their barriers).
-    static const bool allow_fused = [] { const char* e = std::getenv("TM_GEMM_FUSED"); return e && *e == '1'; }();
     const uint32_t row_bytes = (K / be) * block_bytes(dtype);
     const bool fused = allow_fused && dtype == DT_Q4_0 && K % 256 == 0 && (uintptr_t)W % 16 == 0 && row_bytes % 16 == 0;
     const size_t n4 = (size_t)M * K / 4;

@@ -3,6 +3,9 @@ tiles, tiles shared by a cluster along K, rows on and off the 16-byte grid."""
 from __future__ import annotations
 
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -71,3 +74,21 @@ def test_scratch_size_does_not_choose_the_kernel(cuda, torch_mod, orc, dt, m, n,
     assert np.array_equal(got[0], got[1])
     absum = np.abs(A) @ np.abs(orc.dequant(dt, W, n * k).reshape(n, k)).T
     assert np.all(np.abs(got[0] - orc.gemm(dt, W, A, m, n, k, threads=4)) <= 1e-3 * absum)
+
+
+@pytest.mark.parametrize("env,launches", [({}, 1), ({"TM_GEMM_FUSED": "0", "TM_GEMM_BN": ""}, 1), ({"TM_GEMM_FUSED": "1"}, 2), ({"TM_GEMM_PAIR": "0"}, 2)])
+def test_knobs(env, launches):
+    """A few tokens are one launch, and a knob that is off leaves it at that."""
+    code = ("import numpy as np, torch\n"
+            "from tensormark_b200 import lib, synth\n"
+            "L = lib.load()\n"
+            "lib.check(L.tm_cuda_init(-1), 'tm_cuda_init')\n"
+            "W, A, C = synth.make_weights(synth.Q4_0, 256, 512, seed=1), synth.make_activations((17, 512), seed=2), np.empty((17, 256), np.float32)\n"
+            "before = L.tm_cuda_launch_count()\n"
+            "lib.check(L.tm_cuda_sgemm_q4(A.ctypes.data, W.ctypes.data, C.ctypes.data, 17, 256, 512), 'tm_cuda_sgemm_q4')\n"
+            "print(L.tm_cuda_launch_count() - before)\n")
+    clean = {k: v for k, v in os.environ.items() if not k.startswith("TM_GEMM")}
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env={**clean, **env}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert int(r.stdout) == launches
