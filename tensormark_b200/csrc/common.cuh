@@ -77,6 +77,7 @@ unsigned last_gemv_grid();                  // CTAs of the most recent GEMV laun
 // more dependent L2 round trips at the end of the producer): measured on the 8B decode chain, 2.24 / 2.03 / 1.94 ms
 // per token with tails + staging kernels / staging kernels everywhere / neither.
 constexpr int kXqHeaderWords = 16;
+constexpr unsigned kMaxPlaneK = 32768;                  // longest x that is multiplied in that form; a longer one stays fp32
 size_t xq_bytes(unsigned K, unsigned dtype);            // size of such an image; 0 for an unknown format
 
 // ---- kernel launchers (one per .cu) -----------------------------------------

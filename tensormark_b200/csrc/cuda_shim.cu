@@ -241,7 +241,8 @@ bool tm_cuda_gemv_q(const float* x, const void* W, float* y, unsigned N, unsigne
     // consume for all the others. Pageable x takes the copy.
     {
         cudaPointerAttributes ax;
-        const size_t img = wb / N % 16 == 0 ? xq_bytes(K, dtype) : 0;      // rows off the 16-byte grid are multiplied by a finer image, made in the CTAs
+        // rows off the 16-byte grid are multiplied by a finer image, made in the CTAs, and a very long x by x itself
+        const size_t img = wb / N % 16 == 0 && K <= kMaxPlaneK ? xq_bytes(K, dtype) : 0;
         if (img && cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost && ax.devicePointer &&
             (uintptr_t)ax.devicePointer % 16 == 0) {
             ShareCount& sc = s.io_share;

@@ -460,9 +460,11 @@ bool launch_dt(GemvParams p, bool aligned, bool even, cudaStream_t st, ShareCoun
     p.ge = tile_geom(DT, p.K, aligned);
     const uint32_t fixed = x_smem(p.ge, aligned) + kRingBarBytes;
     if (!aligned) p.xq = nullptr;                           // such an image has two planes
-    // a slot per producer at least: a longer x than that (some 40000 activations, half as many where x has four planes)
-    // leaves no room for the ring
-    if (even && fixed + p.ge.producers * p.ge.slot_bytes <= kSmemLimit) {
+    // A slot per producer at least: where x has four planes, some 29000 activations leave no room for the ring. Two would fit
+    // twice as many, but above kMaxPlaneK x has always been multiplied in fp32, and two planes hold less: a small activation
+    // beside a large one of its 32 keeps what is left of 15 bits.
+    const bool held = !aligned || p.K <= kMaxPlaneK;
+    if (even && held && fixed + p.ge.producers * p.ge.slot_bytes <= kSmemLimit) {
         const unsigned sms = (unsigned)device_sm_count();
         // as many CTAs as SMs, rows spread evenly: with one CTA per SM the longest range is the launch's time
         p.rows_per_cta = (p.N + sms - 1) / sms;

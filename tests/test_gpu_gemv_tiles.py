@@ -28,3 +28,17 @@ def test_tile_edges(cuda, torch_mod, orc, dt, n, k):
     assert np.all(err <= activation_rounding_bound(orc, dt, W, x, n, k) + 2e-6 * yabs), float((err / yabs).max())
     if W.shape[1] % 16:                        # there x is held as closely as fp32 does
         assert np.all(err <= 2e-6 * yabs), float((err / yabs).max())
+
+
+@pytest.mark.parametrize("n,k", [(33, 33024), (5, 49152)])
+def test_longer_than_the_planes_serve(cuda, torch_mod, orc, n, k):
+    """Beyond 32768 activations x is multiplied in fp32: a large one under a weight of zero costs its neighbours nothing."""
+    W = synth.make_weights(synth.Q4_0, n, k, seed=82)
+    first = W.reshape(n, k // 32, 18)[:, :, 2]
+    first[:] = (first & 0xF0) | 8              # the block's first weight is zero
+    x = synth.make_activations(k, seed=83)
+    x[::32] = 1000.0
+    y = gemv_dev(cuda, torch_mod, synth.Q4_0, dev_bytes(torch_mod, W), dev_f32(torch_mod, x), n, k)
+    y64, yabs = orc.gemv_f64(synth.Q4_0, W, x, n, k)
+    err = np.abs(y - y64)
+    assert np.all(err <= 2e-6 * yabs), float((err / yabs).max())

@@ -74,7 +74,8 @@ def test_calls_in_a_row(cuda, torch_mod, orc):
     those of the entry with device pointers."""
     torch = torch_mod
     shapes = [(synth.Q4_0, 256, 2048), (synth.Q8_0, 1, 14336), (synth.Q4_1, 40, 14336), (synth.Q4_1, 5632, 2176), (synth.Q6_K, 300, 2048),
-              (synth.Q4_0, 17, 256), (synth.GGUF_Q4_0, 9000, 4096), (synth.Q5_K, 7, 14336), (synth.Q4_0, 130, 352), (synth.Q4_K, 148, 512), (synth.Q8_0, 20, 28672)]
+              (synth.Q4_0, 17, 256), (synth.GGUF_Q4_0, 9000, 4096), (synth.Q5_K, 7, 14336), (synth.Q4_0, 130, 352), (synth.Q4_K, 148, 512), (synth.Q8_0, 20, 28672),
+              (synth.Q4_0, 9, 33024)]
     keep = []                                    # copies on the device go by host address
     for i, (dt, n, k) in enumerate(shapes):
         W = synth.make_weights(dt, n, k, seed=40 + i)
