@@ -108,7 +108,9 @@ void tm_cuda_release_weights(void);
 /* Bytes of an N x K tensor of `dtype`; 0 when K is not whole blocks (tmq.h:124-133). */
 size_t tm_cuda_weight_bytes(unsigned dtype, size_t N, size_t K);
 /* y = W x. W must be 16-byte aligned. (metal.h:3457-3480 tok_gemv, 3647-3669 tok_gemv_kq; dtype 3 / 10: plain fp16 /
- * bf16 rows, metal.h:575-613 f16_gemv_coop and 3693-3721 tok_gemv_h) */
+ * bf16 rows, metal.h:575-613 f16_gemv_coop and 3693-3721 tok_gemv_h). x, and W of plain rows, may be what the kernel before
+ * in the stream writes. W of a block format is read before that kernel has ended when it lets its successor start early
+ * (programmatic dependent launch, as this library's kernels do): blocks are complete before such a kernel is launched. */
 bool tm_cuda_gemv_q_dev(const float* x, const void* W, float* y, unsigned N, unsigned K, unsigned dtype, void* stream);
 /* nblocks Q4_0 blocks in GGUF's split nibble order, rewritten in place in the container's interleaved order (what the
  * reference's converter does on the host, convert_gguf.cpp:124-135): same scale, same codes, bit-identical weights. */

@@ -99,7 +99,8 @@ bool launch_xprep(uint32_t* out, const float* x, const float* x2, unsigned x_op,
 bool launch_gemv(const float* x, const uint8_t* W, float* y, unsigned N, unsigned K, unsigned dtype,
                  const SegTable& seg, cudaStream_t st, const GemvFuse* fuse = nullptr);
 // gemv_f16.cu: plain 16-bit rows (fp16 or bf16), and the GGUF -> container Q4_0 nibble reorder
-bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsigned K, bool bf16, cudaStream_t st);
+// fixed: no kernel of the stream writes W; it is then read before the preceding kernel has ended.
+bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsigned K, bool bf16, bool fixed, cudaStream_t st);
 bool launch_embed_half(const unsigned* tok, unsigned idx, const void* W, float* x, unsigned D, bool bf16, cudaStream_t st);
 bool launch_q4_split_to_interleaved(uint8_t* blocks, size_t nblocks, cudaStream_t st);
 bool launch_dequant(const uint8_t* W, float* out, unsigned N, unsigned K, unsigned dtype, cudaStream_t st);

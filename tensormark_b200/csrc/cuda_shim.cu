@@ -187,7 +187,7 @@ size_t tm_cuda_weight_bytes(unsigned dtype, size_t N, size_t K) { return weight_
 // ---- device-pointer kernels ----------------------------------------------------
 bool tm_cuda_gemv_q_dev(const float* x, const void* W, float* y, unsigned N, unsigned K, unsigned dtype, void* stream) {
     if (!ensure_init(-1)) return false;
-    if (dtype == DT_F16 || dtype == DT_BF16) return launch_gemv_half(x, W, y, N, K, dtype == DT_BF16, (cudaStream_t)stream);
+    if (dtype == DT_F16 || dtype == DT_BF16) return launch_gemv_half(x, W, y, N, K, dtype == DT_BF16, false, (cudaStream_t)stream);
     return launch_gemv(x, (const uint8_t*)W, y, N, K, dtype, one_segment(N), (cudaStream_t)stream);
 }
 

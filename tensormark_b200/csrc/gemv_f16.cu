@@ -6,11 +6,17 @@
 // embed_h_row (2396-2407, tok_embed_h 3260-3271); bf16 has no GPU kernel in the reference (its loader keeps such
 // tensors on the CPU, tensormark/llama.h:4599-4606) and is served by the same kernel here.
 //
-// Bound: HBM, 2 bytes per weight. x is copied into shared memory once per CTA as fp32; LPR lanes (8, or 1 to 8 warps) share a
-// row and read it as 16-byte pieces (eight weights), eight independent loads in flight per lane, fp32 FMA, one shuffle
-// reduction per warp and row. A CTA's first loads do not depend on x: they are requested before it is waited for. Few rows take more
-// warps each, so that the machine is not left with one row per SM and a chain of loads (105 x 3584: 6.8 us a launch with one, now 3.4; 43913 x 4896: 82.7 us, now 78.6). Rows must be
-// 16-byte aligned for that form (K a multiple of 8 and an aligned base); anything else takes a scalar-load kernel.
+// Bound: HBM, 2 bytes per weight. x is copied into shared memory once per CTA as fp32; LPR lanes (8, or 1 to 8 warps) share
+// a row and read it as 16-byte pieces (eight weights), eight independent loads in flight per lane, fp32 FMA, one shuffle
+// reduction per warp and row (how many lanes share a row depends on N, and with it the last bits of its sum).
+//   * A CTA's first loads do not depend on x: where the weights are the lane's registered ones, they are requested before
+//     x is waited for. A caller's own device weights may come from the kernel before, as x may: before the wait they are
+//     only asked into L2, and requested while x is on its way into shared memory (2000 x 2048 3.9 us a launch with the
+//     early request, 4.1 so, 4.9 without the prefetch and behind x; 4096 x 4096 9.4, 9.8, 11.4).
+//   * Few rows take more warps each, so that the machine is not left with one row per SM and a chain of loads (105 x 3584:
+//     6.8 us a launch with one, now 3.4; 43913 x 4896: 82.7 us, now 78.6).
+// Rows must be 16-byte aligned for that form (K a multiple of 8 and an aligned base); anything else takes a scalar-load
+// kernel.
 #include "common.cuh"
 
 #include <cuda_fp16.h>
@@ -42,8 +48,7 @@ template <bool BF16> __device__ __forceinline__ float dot8(const uint4 w, const 
 }
 
 template <bool BF16, int LPR>
-__global__ void __launch_bounds__(256, 3) gemv_half_rows(const float* __restrict__ x, const uint16_t* __restrict__ W, float* __restrict__ y,
-                                                      uint32_t N, uint32_t K) {
+__global__ void __launch_bounds__(256, 3) gemv_half_rows(const float* x, const uint16_t* W, float* __restrict__ y, uint32_t N, uint32_t K, bool fixed) {
     constexpr uint32_t ROWS = 256 / LPR, STEP = LPR, U = 8, WPR = LPR / 32;    // WPR 0: several rows per warp
     extern __shared__ __align__(16) float xs[];
     __shared__ float sums[2][8];
@@ -53,13 +58,20 @@ __global__ void __launch_bounds__(256, 3) gemv_half_rows(const float* __restrict
         const uint4* wr = reinterpret_cast<const uint4*>(W + (size_t)row * K);
 #pragma unroll
         for (uint32_t u = 0; u < U; ++u)
-            if (i0 + u * STEP < k8) w[u] = __ldg(wr + i0 + u * STEP);
+            if (i0 + u * STEP < k8) w[u] = __ldcg(wr + i0 + u * STEP);
     };
     const uint32_t row0 = blockIdx.x * ROWS + threadIdx.x / LPR;
-    if (row0 < N) request(row0, first);
+    if (row0 < N) {
+        if (fixed) request(row0, first);
+        else if (first == 0)                                    // into L2 only, where a write that is still to come finds them
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(W + (size_t)row0 * K), "r"(min(k8, max(U * STEP, 256u)) * 16u) : "memory");
+    }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");          // x may come from the preceding kernel of the stream
-    for (uint32_t i = threadIdx.x; i < K / 4; i += blockDim.x) reinterpret_cast<float4*>(xs)[i] = __ldcg(reinterpret_cast<const float4*>(x) + i);
+    for (uint32_t i = threadIdx.x; i < K / 4; i += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + 4 * i)), "l"(x + 4 * i) : "memory");
+    if (!fixed && row0 < N) request(row0, first);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     uint32_t turn = 0;
     for (uint32_t base = blockIdx.x * ROWS; base < N; base += gridDim.x * ROWS, turn ^= 1u) {
@@ -135,7 +147,7 @@ __global__ void q4_split_to_interleaved_kernel(uint8_t* blocks, size_t nblocks) 
 
 }  // namespace
 
-bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsigned K, bool bf16, cudaStream_t st) {
+bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsigned K, bool bf16, bool fixed, cudaStream_t st) {
     if (!x || !W || !y) return fail("gemv_h: null pointer");
     if (N == 0) return true;
     if (K == 0) return fail("gemv_h: empty rows");
@@ -161,7 +173,7 @@ bool launch_gemv_half(const float* x, const void* W, float* y, unsigned N, unsig
             at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             at[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = at; cfg.numAttrs = 1;
-            cudaLaunchKernelEx(&cfg, kernel, x, w, y, (uint32_t)N, (uint32_t)K);
+            cudaLaunchKernelEx(&cfg, kernel, x, w, y, (uint32_t)N, (uint32_t)K, fixed);
             return true;
         };
         auto pick = [&](auto b) {

@@ -379,7 +379,7 @@ void tm_cuda_tok_gemv_h(int xslot, int wid, uint64_t woff, int yslot, size_t yof
     uint8_t* y = slot_ptr(yslot, yoff + (size_t)N * 4, "tok_gemv_h");
     const uint8_t* W = weight_ptr(wid, woff, (size_t)N * K * 2, "tok_gemv_h");
     if (!x || !y || !W) return;
-    if (!launch_gemv_half(x, W, (float*)(y + yoff), N, K, false, s.stream)) s.sticky = true;
+    if (!launch_gemv_half(x, W, (float*)(y + yoff), N, K, false, true, s.stream)) s.sticky = true;
 }
 void tm_cuda_tok_embed_h(int tokslot, unsigned idx, int wid, uint64_t woff, int xslot, unsigned D) {
     if (!ensure_init(-1)) return;

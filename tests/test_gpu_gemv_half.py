@@ -24,3 +24,20 @@ def test_row_shares(cuda, torch_mod, dt, n, k):
     y = gemv_dev(cuda, torch, dt, w, dev_f32(torch, x), n, k)
     wd = w.double().cpu().numpy()
     assert np.all(np.abs(y - wd @ x) <= 2e-6 * (np.abs(wd) @ np.abs(x)))
+
+
+@pytest.mark.parametrize("dt", [synth.F16, synth.BF16])
+def test_weights_from_the_kernel_before(cuda, torch_mod, dt):
+    """W may be the output of the launch right before, as x may: merged weights, for instance."""
+    torch = torch_mod
+    n, k, r = 1500, 2048, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    t = torch.float16 if dt == synth.F16 else torch.bfloat16
+    w, x = torch.empty(n, k, dtype=t, device="cuda"), torch.randn(k, generator=g, device="cuda")
+    for _ in range(20):
+        a, b = (torch.randn(*s, generator=g, device="cuda").to(t) for s in ((n, r), (r, k)))
+        w.zero_()
+        torch.cuda.synchronize()
+        torch.matmul(a, b, out=w)
+        y = gemv_dev(cuda, torch, dt, w, x, n, k)
+        assert np.array_equal(y, gemv_dev(cuda, torch, dt, w, x, n, k))
