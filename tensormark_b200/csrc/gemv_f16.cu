@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256, 3) gemv_half_rows(const float* x, const u
 
 // any K, any 2-byte aligned base: one warp per row, scalar loads
 template <bool BF16>
-__global__ void __launch_bounds__(256) gemv_half_generic(const float* __restrict__ x, const uint16_t* __restrict__ W, float* __restrict__ y,
+__global__ void __launch_bounds__(256) gemv_half_generic(const float* x, const uint16_t* __restrict__ W, float* __restrict__ y,
                                                          uint32_t N, uint32_t K) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x * 8 + warp;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) gemv_half_generic(const float* __restrict
 
 // x = row tok[idx] of a 16-bit table (sentinel 0xFFFFFFFF -> zeros), embed_h_row (metal.h:2396-2407)
 template <bool BF16>
-__global__ void embed_half_row(const uint32_t* __restrict__ tok, uint32_t idx, const uint16_t* __restrict__ W, float* __restrict__ x, uint32_t D) {
+__global__ void embed_half_row(const uint32_t* tok, uint32_t idx, const uint16_t* __restrict__ W, float* __restrict__ x, uint32_t D) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= D) return;

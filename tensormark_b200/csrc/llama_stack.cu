@@ -42,6 +42,7 @@ __device__ __forceinline__ float wsum(float v) {
     return v;
 }
 // Kernels of a layer follow each other closely: each may be set up while the one before it drains, and waits for it here.
+// What that one writes carries no __restrict__: the compiler must not load it through the read-only cache.
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -66,7 +67,7 @@ __device__ __forceinline__ float wmax(float v) {
 // OT = __half: the row goes straight into the next GEMM as its fp16 operand (the same value that GEMM's pre-pass would
 // make of the fp32 row: one rounding).
 template <typename OT>
-__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float* x, const float* __restrict__ w,
                                                            OT* __restrict__ out, uint32_t D, float eps) {
     __shared__ float part[8];
     __shared__ float inv_s;
@@ -396,8 +397,8 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 // A CTA's work grows with its token block, so the blocks of the last tokens start first (1499 tokens, 32 heads of 128: 139 us
 // in ascending order, where the longest CTAs of the last head were the tail, now 100; the MMAs alone take 66).
 template <int DH, typename OT>
-__global__ void __launch_bounds__(128, 3) prefill_attn_h_kernel(const float* __restrict__ qkv, uint32_t ld, const __half* __restrict__ kh,
-                                                                const __half* __restrict__ vh, OT* __restrict__ out, uint32_t QD,
+__global__ void __launch_bounds__(128, 3) prefill_attn_h_kernel(const float* qkv, uint32_t ld, const __half* kh,
+                                                                const __half* vh, OT* __restrict__ out, uint32_t QD,
                                                                 uint32_t T, uint32_t pos0, uint32_t ctx, uint32_t REP, float scale) {
     constexpr int RSH = DH + 8;                                 // halves per row in shared memory: 16-byte rows, conflict-free ldmatrix
     constexpr int KS = DH / 16;                                 // k-steps of q k^T

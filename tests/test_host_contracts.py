@@ -281,3 +281,23 @@ def test_gguf_index_is_read_natively(hc, tmp_path):
     i = over.rindex(struct.pack("<IQ", 0, 256))                                         # second tensor's (type, offset)
     over[i: i + 12] = struct.pack("<IQ", 0, 128)
     assert count(bytes(over)) == -1
+
+
+def test_programmatic_kernels_read_no_moving_data_as_constant():
+    """A kernel that is resident while its predecessor still writes (it waits with griddepcontrol.wait) must not have the
+    compiler load that data through the read-only path: const __restrict__ only on weights and tables."""
+    src = os.path.join(ROOT, "tensormark_b200", "csrc")
+    seen = 0
+    for f in sorted(os.listdir(src)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(src, f)).read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^;{]*?\)\s*)?(\w+)\(([^{;]*)\)\s*\{", text):
+            at, depth = m.end(), 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[at], 0)
+                at += 1
+            if not re.search(r"pdl_enter\(\)|griddepcontrol\.wait", text[m.end():at]):
+                continue
+            seen += 1
+            moving = [q for q in re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s+(\w+)", m.group(2)) if q not in ("W", "w", "tbl")]
+            assert not moving, (f, m.group(1), moving)
+    assert seen >= 15, seen
