@@ -147,11 +147,16 @@ __device__ __forceinline__ float stage_groups(uint32_t* units, uint32_t* fine, c
                 ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
                 v[j].x *= w2.x; v[j].y *= w2.y; v[j].z *= w2.z; v[j].w *= w2.w;
             } else if (x_op == 2u) {
-                // silu(x) * up with the hardware exponential and reciprocal: relative error 2^-21, inside what the
-                // fixed-point planes that follow keep
+                // silu(x) * up with the hardware exponential and reciprocal: relative error 2^-21, inside what the two
+                // fixed-point planes that follow keep; four planes keep more
                 const float4 w2 = w2s[j];
-                v[j].x = __fdividef(v[j].x, 1.0f + __expf(-v[j].x)) * w2.x; v[j].y = __fdividef(v[j].y, 1.0f + __expf(-v[j].y)) * w2.y;
-                v[j].z = __fdividef(v[j].z, 1.0f + __expf(-v[j].z)) * w2.z; v[j].w = __fdividef(v[j].w, 1.0f + __expf(-v[j].w)) * w2.w;
+                if constexpr (FINE) {
+                    v[j].x = v[j].x / (1.0f + expf(-v[j].x)) * w2.x; v[j].y = v[j].y / (1.0f + expf(-v[j].y)) * w2.y;
+                    v[j].z = v[j].z / (1.0f + expf(-v[j].z)) * w2.z; v[j].w = v[j].w / (1.0f + expf(-v[j].w)) * w2.w;
+                } else {
+                    v[j].x = __fdividef(v[j].x, 1.0f + __expf(-v[j].x)) * w2.x; v[j].y = __fdividef(v[j].y, 1.0f + __expf(-v[j].y)) * w2.y;
+                    v[j].z = __fdividef(v[j].z, 1.0f + __expf(-v[j].z)) * w2.z; v[j].w = __fdividef(v[j].w, 1.0f + __expf(-v[j].w)) * w2.w;
+                }
             }
             am[j] = max(max(__float_as_uint(fabsf(v[j].x)), __float_as_uint(fabsf(v[j].y))), max(__float_as_uint(fabsf(v[j].z)), __float_as_uint(fabsf(v[j].w))));
             s32[j] = (v[j].x + v[j].y) + (v[j].z + v[j].w);
