@@ -89,7 +89,7 @@ struct GemvFuse {                           // optional fusions of the decode ch
     bool accumulate;                        // y[row] += dot instead of y[row] = dot
     const Exchange* xchg;                   // nullptr: single GPU
     const uint32_t* xq;                     // x (after x_op) already in unit form for this dtype and K; the fp32 x is
-                                            // still passed: rows that are not 16-byte aligned take the plain kernel
+                                            // still passed: rows off the 16-byte grid stage four planes of it themselves
     uint32_t* share;                        // device scratch of xq_bytes(): x is far away (host memory), so the CTAs stage a part
     ShareCount* share_count;                // of it each and share the image, which this counts
 };

@@ -1263,7 +1263,8 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
 
     // Up to 512 tokens straight from the blocks: a weight is then converted at most twice, in the shadow of the copies. From
     // there on converting once for all token tiles is cheaper (4096 x 4096, blocks / fp16 copy: 512 tokens Q4_0 36 / 40,
-    // Q6_K 44 / 44 us; 1000 tokens Q4_0 54 / 48, Q6_K 75 / 52 us). The knobs of the fp16 kernels keep a call on them.
+    // Q6_K 44 / 44 us; 1000 tokens Q4_0 54 / 48, Q6_K 75 / 52 us: measured for these two formats, taken over for the
+    // others). The knobs of the fp16 kernels keep a call on them.
     // The kernels sum in different orders, so sizes choose and not what the caller's scratch has room for beyond its need.
     auto knob = [](const char* name, int unset) { const char* e = std::getenv(name); return e && *e ? std::atoi(e) : unset; };
     static const bool allow_fused = knob("TM_GEMM_FUSED", 0) == 1;
@@ -1272,8 +1273,8 @@ bool launch_gemm(const float* A, const uint8_t* W, float* C, unsigned ldc, unsig
         return launch_gemm_blocks(A, W, C, ldc, M, N, K, dtype, workspace, st);
 
     // Q4_0 with K a multiple of 256 and 16-byte aligned rows can be dequantized inside the GEMM (gemm_q4_tn).
-    // TM_GEMM_FUSED=1 selects it; the default is the pre-pass, which is the faster of the two today
-    // (2000 x 5632 x 2048: 72 us for pre-passes + TMA-fed kernel against 77 us for the producer-fed kernel,
+    // TM_GEMM_FUSED=1 selects it; the default is the pre-pass, which is the faster of the two
+    // (2000 x 5632 x 2048: 52 us for pre-pass + TMA-fed kernel against 78 us for the producer-fed kernel,
     // whose tensor pipe is 30 % busy with the producers stalled on their barriers).
     const uint32_t row_bytes = (K / be) * block_bytes(dtype);
     const bool fused = allow_fused && dtype == DT_Q4_0 && K % 256 == 0 && (uintptr_t)W % 16 == 0 && row_bytes % 16 == 0;

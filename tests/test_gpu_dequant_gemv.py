@@ -97,19 +97,20 @@ def test_config3_kquant_llama3_shapes(cuda, torch_mod, orc, dt, shape):
 def test_ragged_and_minimum_shapes(cuda, torch_mod, orc, dt):
     be = synth.BLOCK_ELEMS[dt]
     # one row, rows not a multiple of the warp row group, a single block per row, an odd block count,
-    # rows whose byte length is not a multiple of 16 (takes the byte-granular kernel)
+    # rows whose byte length is not a multiple of 16 (copied from the line they begin in)
     for n, k in [(1, 2048), (7, 4096), (3, be), (5, 3 * be), (301, 2048), (2, 11 * be), (1187, 2048)]:
         _check_gemv(cuda, torch_mod, orc, dt, n, k, seed=40 + n)
 
 
+@pytest.mark.parametrize("off", [6, 7])             # an even address rides the ring, an odd one takes the byte-granular kernel
 @pytest.mark.parametrize("dt", DTYPES)
-def test_unaligned_weight_base_uses_generic_kernel(cuda, torch_mod, orc, dt):
+def test_unaligned_weight_base(cuda, torch_mod, orc, dt, off):
     n, k = 19, 2048
     W = synth.make_weights(dt, n, k, seed=9)
     x = synth.make_activations(k, seed=9)
     buf = torch_mod.zeros(W.size + 64, dtype=torch_mod.uint8, device="cuda")
-    buf[6: 6 + W.size] = torch_mod.from_numpy(W.reshape(-1)).cuda()
-    view = buf[6:]
+    buf[off: off + W.size] = torch_mod.from_numpy(W.reshape(-1)).cuda()
+    view = buf[off:]
     y = gemv_dev(cuda, torch_mod, dt, view, dev_f32(torch_mod, x), n, k)
     y64, yabs = orc.gemv_f64(dt, W, x, n, k)
     assert np.all(np.abs(y - y64) <= TOL * yabs)
