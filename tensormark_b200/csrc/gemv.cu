@@ -16,8 +16,8 @@
 //     launches (the property tensormark/metal.h:504-510 requires).
 //   * Rows that start on any even address are served: a row's copy starts at the 16-byte boundary below it and the
 //     lanes read from the remainder on (AL = false). Such rows used to be multiplied by x in fp32; here x keeps four
-//     planes for them, which holds an fp32 x to its last bits. Odd addresses and TQ2 take gemv_generic, a plain byte-granular
-//     kernel with the same per-row arithmetic contract (tolerance-level, not bitwise, agreement).
+//     planes for them, which holds an fp32 x to its last bits. Odd addresses, TQ2 and an x of more than kMaxPlaneK take
+//     gemv_generic, a plain byte-granular kernel with the same per-row arithmetic contract (tolerance-level, not bitwise, agreement).
 #include "common.cuh"
 #include "gemv_tile.cuh"
 #include "share_count.h"
