@@ -13,7 +13,8 @@
 //   * The products of 4 loads x REP heads are summed over a row's lanes by a transposing butterfly (each step halves the
 //     values a lane keeps), after which a lane holds the scores it will exponentiate.
 //   * fp32 pairs in fma.rn.f32x2 for q k and p v.
-// Partials (max, sum, unnormalised output per split) are merged by a second kernel.
+// Partials (max, sum, unnormalised output per split) are merged by a second kernel or, where the calls are short, in the same
+// launch by the CTAs of a cluster.
 #include "common.cuh"
 #include "bulk.cuh"
 #include "glue.h"
@@ -45,6 +46,7 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // ---- the streaming kernel ------------------------------------------------------------------------------------------
+constexpr uint32_t kMaxCluster = 16;                        // splits that one launch merges
 constexpr int kLoads = 4;                                   // 16-byte loads per lane, of K and of V, per stage
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -95,7 +97,11 @@ template <int REP> struct Split {
     static constexpr uint32_t Half = Warps * kLoads * 512, Smem = Stages * 2 * Half;      // bytes of K (or V) per stage; of the ring
 };
 
-template <typename T, int DH, int REP>
+// CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
+// then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. Up to some thousand
+// positions the two launches and the way of the partials through L2 are most of the time: 32 / 8 heads of 128, 300 fp16
+// positions 8.3 us with the merging kernel, 6.4 us in one launch.
+template <typename T, int DH, int REP, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (Split<REP>::Warps + 1), 1)
 attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float* stat, uint32_t H, uint32_t ctx, uint32_t allow,
                    uint32_t chunk, float scale, const int* st, int* status) {
@@ -111,6 +117,9 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
     __shared__ __align__(16) float pbuf[NW][PW][REP];                        // a warp's weights of its positions
     __shared__ __align__(16) float cbuf[NW][REP];                            // its correction factors
     __shared__ float sm_m[NW][REP], sm_l[NW][REP];
+    __shared__ float2 cta_ml[REP];                                           // CLUSTER: this split's maximum and sum per head
+    float* const cta_o = reinterpret_cast<float*>(smem) + NW * REP * DH;     // and its output, behind those of its warps in the ring
+    static_assert((NW + 1) * REP * DH * sizeof(float) <= Split<REP>::Smem, "the outputs fit into the ring");
     __shared__ __align__(16) uint4 nothing;                                  // what a lane without a row multiplies its weight 0 by
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -329,9 +338,45 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
                 o = fmaf(f, out[((size_t)w * REP + r) * DH + d], o);
                 L = fmaf(f, sm_l[w][r], L);
             }
-            part[((size_t)split * H + head) * DH + d] = o;
-            if (d == 0) { stat[((size_t)split * H + head) * 2] = M; stat[((size_t)split * H + head) * 2 + 1] = L; }
+            if constexpr (CLUSTER) {
+                cta_o[i] = o;
+                if (d == 0) cta_ml[r] = make_float2(M, L);
+            } else {
+                part[((size_t)split * H + head) * DH + d] = o;
+                if (d == 0) { stat[((size_t)split * H + head) * 2] = M; stat[((size_t)split * H + head) * 2 + 1] = L; }
+            }
         }
+    }
+    if constexpr (CLUSTER) {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const uint32_t nsplit = gridDim.y, per = (uint32_t)(REP * DH) / nsplit;       // every CTA merges its share of the outputs: both are powers of two
+        for (uint32_t i = split * per + threadIdx.x; i < (split + 1u) * per; i += blockDim.x) {
+            const uint32_t at_o = smem_u32(cta_o) + 4u * i, at_ml = smem_u32(cta_ml) + 8u * (i / DH);
+            float2 ml[kMaxCluster];
+            float x[kMaxCluster], M = -CUDART_INF_F, o = 0.f, L = 0.f;
+#pragma unroll
+            for (uint32_t k = 0; k < kMaxCluster; ++k)
+                if (k < nsplit) {
+                    uint32_t a, b;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(at_ml), "r"(k));
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(at_o), "r"(k));
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(ml[k].x), "=f"(ml[k].y) : "r"(a) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[k]) : "r"(b) : "memory");
+                }
+#pragma unroll
+            for (uint32_t k = 0; k < kMaxCluster; ++k)
+                if (k < nsplit) M = fmaxf(M, ml[k].x);
+#pragma unroll
+            for (uint32_t k = 0; k < kMaxCluster; ++k)
+                if (k < nsplit) {
+                    const float f = ml[k].x == -CUDART_INF_F ? 0.f : __expf(ml[k].x - M);
+                    o = fmaf(f, x[k], o);
+                    L = fmaf(f, ml[k].y, L);
+                }
+            part[(size_t)kv * (REP * DH) + i] = o * (1.0f / L);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // nobody leaves while its shared memory is read
     }
 }
 
@@ -467,22 +512,79 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* part, co
 template <typename T, int DH, int REP>
 bool launch_stream(dim3 grid, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat, unsigned H, unsigned ctx,
                    unsigned allow, unsigned chunk, float scale, const int* state) {
-    static const cudaError_t attr = cudaFuncSetAttribute(attn_stream_kernel<T, DH, REP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem);
+    static const cudaError_t attr = cudaFuncSetAttribute(attn_stream_kernel<T, DH, REP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem);
     if (attr != cudaSuccess) return fail("attention: shared memory attribute: %s", cudaGetErrorString(attr));
-    launch_pdl(attn_stream_kernel<T, DH, REP>, grid, dim3(32 * (Split<REP>::Warps + 1)), Split<REP>::Smem, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state, device_status_word());
+    launch_pdl(attn_stream_kernel<T, DH, REP, false>, grid, dim3(32 * (Split<REP>::Warps + 1)), Split<REP>::Smem, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state, device_status_word());
     return true;
 }
 
+// One launch with a cluster of `cs` splits per K/V head; false (and no error) where the device cannot hold KVH of them at a time.
+template <typename T, int DH, int REP>
+bool launch_cluster(unsigned cs, unsigned KVH, cudaStream_t st, const float* q, const T* kc, const T* vc, float* out, unsigned H, unsigned ctx,
+                    unsigned allow, float scale, const int* state) {
+    auto* kernel = attn_stream_kernel<T, DH, REP, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(KVH, cs); cfg.blockDim = dim3(32 * (Split<REP>::Warps + 1)); cfg.dynamicSmemBytes = Split<REP>::Smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = cs; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    struct Fits { int clusters[5]; };
+    static const Fits fits = [&] {                          // clusters of 1, 2, 4, 8, 16 that run at a time
+        Fits f = {};
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem) != cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return f; }
+        cudaLaunchConfig_t c = cfg;
+        cudaLaunchAttribute a = at[0];
+        c.attrs = &a; c.numAttrs = 1;
+        for (int i = 0; i < 5; ++i) {
+            a.val.clusterDim.y = 1u << i;
+            c.gridDim = dim3(1, 1u << i);
+            if (cudaOccupancyMaxActiveClusters(&f.clusters[i], kernel, &c) != cudaSuccess) { cudaGetLastError(); f.clusters[i] = 0; }
+        }
+        return f;
+    }();
+    int i = 0;
+    while (1u << i < cs) ++i;
+    if (fits.clusters[i] < (int)KVH) return false;
+    static const bool pdl = [] { const char* e = std::getenv("TM_GLUE_PDL"); return !(e && *e == '0'); }();
+    cfg.numAttrs = pdl ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, q, kc, vc, out, (float*)nullptr, (uint32_t)H, (uint32_t)ctx, (uint32_t)allow, (uint32_t)cdiv(allow, cs), scale, state, device_status_word());
+    return true;
+}
 // One K/V head per grid column. The streaming kernel copies whole rows in bulk and wants the caches on 16-byte boundaries;
 // caches on any other address take the element-wise one.
 template <typename T, int DH>
-bool launch_splits(unsigned REP, unsigned KVH, unsigned nsplit, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat,
-                   unsigned H, unsigned ctx, unsigned allow, unsigned chunk, float scale, const int* state) {
+bool launch_splits(unsigned REP, unsigned KVH, unsigned nsplit, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat, float* out,
+                   unsigned H, unsigned ctx, unsigned allow, unsigned chunk, float scale, const int* state, bool* merged) {
+    static const bool one = [] { const char* e = std::getenv("TM_ATTN_CLUSTER"); return !(e && *e == '0'); }();   // A/B knob
     const dim3 grid(KVH, nsplit);
     const bool bulk = (uintptr_t)kc % 16 == 0 && (uintptr_t)vc % 16 == 0;
     bool ok = true;
+    *merged = false;
     auto go = [&](auto rep) {
         constexpr int R = decltype(rep)::value;
+        if (bulk && one) {
+            // A cluster has a power of two of CTAs, so fewer than the SMs allow: its CTAs read for longer by what their ranges are
+            // longer, and that is to cost less than the merging kernel (1.5-2.5 us; it takes 20 splits per round trip, and 40
+            // and more cost it 3-8 us). Measured, us for two launches / one, with the longer ranges' elements per head, fp16
+            // unless noted: 32/8 heads of 128 1500 positions (104 x 128 = 13k) 9.4 / 7.6, 5000 (347 x 128 = 44k) 12.0 / 13.3;
+            // 16/8 of 64 3500 (15.5k) 7.0 / 6.9, fp32 5000 (22k) 8.0 / 8.3; 40/40 of 128 fp32 700 (15k) 9.0 / 9.4, 500 (10.6k)
+            // 7.6 / 7.2. Eight heads per K/V head are more arithmetic: 64/8 of 128 700 (6.3k) 9.0 / 8.4, 1000 (8.8k) 9.1 / 9.7.
+            // Many splits: 28/7 of 128 fp32 (21) 4200 (13.7k) 15.4 / 10.6, 4/1 of 128 (148) 5000 (36k) 17.0 / 10.0, 20000 (143k)
+            // 19.3 / 20.8; eight heads 16/2 of 128 (74) 3500 (22k) 15.2 / 11.4, 5000 (31k) 13.8 / 13.9, fp32 12.8 / 15.0.
+            constexpr bool half = sizeof(T) == 2;
+            const unsigned more = R == 8 ? (nsplit > 40 ? 18432u : half ? 7168u : 6144u) : (nsplit > 20 ? 49152u : half ? 16384u : 12288u);
+            const unsigned longest = cdiv(allow, nsplit) + more / DH;
+            // 32 positions are a short stage; eight heads of 128 need the CTAs for the merge too (16/2, 140 fp32 positions: 6.4 us with 32, 6.1 with 8)
+            unsigned cs = kMaxCluster;
+            while (cs > 1 && (cs * KVH > (unsigned)device_sm_count() || (cs > 4 && cs > cdiv(allow, R * DH >= 1024 ? 8u : 32u)))) cs >>= 1;
+            for (; cs && cdiv(allow, cs) <= longest && !*merged; cs >>= 1)
+                *merged = launch_cluster<T, DH, R>(cs, KVH, st, q, kc, vc, out, H, ctx, allow, scale, state);
+            if (*merged) return;
+        }
         if (bulk) ok = launch_stream<T, DH, R>(grid, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state);
         else launch_pdl(attn_split_kernel<T, DH / 32, R>, grid, dim3(128), 0, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state);
     };
@@ -535,17 +637,17 @@ bool launch_attention(const float* q, const void* kc, const void* vc, bool half_
     }
     float* part = scratch;
     float* stat = scratch + pl.part_floats;
-    bool ok;
+    bool ok, merged;
     if (half_cache) {
         const __half *k = (const __half*)kc, *v = (const __half*)vc;
-        ok = dh == 128 ? launch_splits<__half, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, H, ctx, allow, chunk, scale, state)
-                       : launch_splits<__half, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, H, ctx, allow, chunk, scale, state);
+        ok = dh == 128 ? launch_splits<__half, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged)
+                       : launch_splits<__half, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged);
     } else {
         const float *k = (const float*)kc, *v = (const float*)vc;
-        ok = dh == 128 ? launch_splits<float, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, H, ctx, allow, chunk, scale, state)
-                       : launch_splits<float, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, H, ctx, allow, chunk, scale, state);
+        ok = dh == 128 ? launch_splits<float, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged)
+                       : launch_splits<float, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged);
     }
-    if (!ok) return false;
+    if (!ok || merged) return ok;
     launch_pdl(attn_combine_kernel, dim3(H), dim3(dh < 128 ? 64 : 128), 0, st, part, stat, out, H, dh, nsplit);
     note_launch();
     return check_launch("attn_combine");
