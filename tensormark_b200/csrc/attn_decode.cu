@@ -466,33 +466,46 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* q, const T
 }
 
 
-// out[head][d] = sum_s e^(m_s - M) part_s[d] / sum_s e^(m_s - M) l_s. One CTA per head, one thread per dim; the splits'
-// weights are worked out once, a lane per split, while the first partials are on their way (18 splits in three round trips
-// after the weights: 32 / 8 heads of 128, 8191 positions 15.9 us with the split kernel, now 15.6).
-__global__ void __launch_bounds__(128) attn_combine_kernel(const float* part, const float* stat, float* out, uint32_t H, uint32_t dh, uint32_t nsplit) {
-    constexpr uint32_t BATCH = 20;
-    __shared__ float wsum[256];
+// out[head][d] = sum_s e^(m_s - M) part_s[d] / sum_s e^(m_s - M) l_s. One CTA per head; bound by its chain of round trips to
+// L2. Four threads per dim take every fourth split, so 40 partials are on their way at a time, while a lane per split reads
+// its maximum and sum at once and works out the weights. With a thread per dim, 20 partials at a time and the maxima read
+// before the sums: 32 / 8 heads of 128, 8191 fp16 positions (18 splits) 15.1 us with the split kernel, now 13.4; 32 / 4 of 64
+// (37) 11.0 / 9.4; 8 / 1 of 128 (148) 22.6 / 11.8; 40 / 40 of 128 (3) 31.0 / 31.0.
+constexpr uint32_t kMergeGroups = 4;
+__global__ void __launch_bounds__(kMergeGroups * 128) attn_combine_kernel(const float* part, const float* stat, float* out, uint32_t H, uint32_t dh, uint32_t nsplit) {
+    constexpr uint32_t BATCH = 10, G = kMergeGroups, MOST = 256;
+    __shared__ float sums[G - 1][128];
+    __shared__ float wsum[MOST];
     __shared__ float inv;
     pdl_enter();
-    const uint32_t head = blockIdx.x, lane = threadIdx.x & 31u, d = threadIdx.x;
-    const bool mine = d < dh;                                  // dh <= 128
+    const uint32_t head = blockIdx.x, lane = threadIdx.x & 31u, d = threadIdx.x % dh, grp = threadIdx.x / dh;      // G * dh threads
     float v[BATCH];
     auto request = [&](uint32_t s0) {
 #pragma unroll
         for (uint32_t k = 0; k < BATCH; ++k)
-            if (mine && s0 + k < nsplit) v[k] = __ldcg(part + ((size_t)(s0 + k) * H + head) * dh + d);
+            if (s0 + G * k + grp < nsplit) v[k] = __ldcg(part + ((size_t)(s0 + G * k + grp) * H + head) * dh + d);
     };
     request(0);
     if (threadIdx.x < 32) {
+        float2 ml[MOST / 32];
         float M = -CUDART_INF_F, L = 0.f;
-        for (uint32_t s = lane; s < nsplit; s += 32) M = fmaxf(M, __ldcg(stat + ((size_t)s * H + head) * 2));
+#pragma unroll
+        for (uint32_t i = 0; i < MOST / 32; ++i) {
+            const uint32_t s = lane + 32u * i;
+            const float* at = stat + ((size_t)s * H + head) * 2;             // scratch is on 4 bytes
+            ml[i] = s < nsplit ? make_float2(__ldcg(at), __ldcg(at + 1)) : make_float2(-CUDART_INF_F, 0.f);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < MOST / 32; ++i) M = fmaxf(M, ml[i].x);
 #pragma unroll
         for (int o = 16; o; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        for (uint32_t s = lane; s < nsplit; s += 32) {
-            const float* ml = stat + ((size_t)s * H + head) * 2;
-            const float w = __ldcg(ml) == -CUDART_INF_F ? 0.f : __expf(__ldcg(ml) - M);
+#pragma unroll
+        for (uint32_t i = 0; i < MOST / 32; ++i) {
+            const uint32_t s = lane + 32u * i;
+            if (s >= nsplit) continue;
+            const float w = ml[i].x == -CUDART_INF_F ? 0.f : __expf(ml[i].x - M);
             wsum[s] = w;
-            L = fmaf(w, __ldcg(ml + 1), L);
+            L = fmaf(w, ml[i].y, L);
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
@@ -500,13 +513,18 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const float* part, co
     }
     __syncthreads();
     float o = 0.f;
-    for (uint32_t s0 = 0; s0 < nsplit; s0 += BATCH) {
+    for (uint32_t s0 = 0; s0 < nsplit; s0 += G * BATCH) {
         if (s0) request(s0);
 #pragma unroll
         for (uint32_t k = 0; k < BATCH; ++k)
-            if (s0 + k < nsplit) o = fmaf(wsum[s0 + k], v[k], o);
+            if (s0 + G * k + grp < nsplit) o = fmaf(wsum[s0 + G * k + grp], v[k], o);
     }
-    if (mine) out[(size_t)head * dh + d] = o * inv;
+    if (grp) sums[grp - 1][d] = o;
+    __syncthreads();
+    if (grp) return;
+#pragma unroll
+    for (uint32_t i = 0; i < G - 1; ++i) o += sums[i][d];
+    out[(size_t)head * dh + d] = o * inv;
 }
 
 template <typename T, int DH, int REP>
@@ -648,7 +666,7 @@ bool launch_attention(const float* q, const void* kc, const void* vc, bool half_
                        : launch_splits<float, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged);
     }
     if (!ok || merged) return ok;
-    launch_pdl(attn_combine_kernel, dim3(H), dim3(dh < 128 ? 64 : 128), 0, st, part, stat, out, H, dh, nsplit);
+    launch_pdl(attn_combine_kernel, dim3(H), dim3(kMergeGroups * dh), 0, st, part, stat, out, H, dh, nsplit);
     note_launch();
     return check_launch("attn_combine");
 }
