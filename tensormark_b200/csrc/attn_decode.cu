@@ -100,7 +100,7 @@ template <int REP> struct Split {
 // CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
 // then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. Up to some thousand
 // positions the two launches and the way of the partials through L2 are most of the time: 32 / 8 heads of 128, 300 fp16
-// positions 8.3 us with the merging kernel, 6.4 us in one launch.
+// positions 7.1 us with the merging kernel, 6.4 us in one launch.
 template <typename T, int DH, int REP, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (Split<REP>::Warps + 1), 1)
 attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float* stat, uint32_t H, uint32_t ctx, uint32_t allow,
@@ -586,15 +586,12 @@ bool launch_splits(unsigned REP, unsigned KVH, unsigned nsplit, cudaStream_t st,
         constexpr int R = decltype(rep)::value;
         if (bulk && one) {
             // A cluster has a power of two of CTAs, so fewer than the SMs allow: its CTAs read for longer by what their ranges are
-            // longer, and that is to cost less than the merging kernel (1.5-2.5 us; it takes 20 splits per round trip, and 40
-            // and more cost it 3-8 us). Measured, us for two launches / one, with the longer ranges' elements per head, fp16
-            // unless noted: 32/8 heads of 128 1500 positions (104 x 128 = 13k) 9.4 / 7.6, 5000 (347 x 128 = 44k) 12.0 / 13.3;
-            // 16/8 of 64 3500 (15.5k) 7.0 / 6.9, fp32 5000 (22k) 8.0 / 8.3; 40/40 of 128 fp32 700 (15k) 9.0 / 9.4, 500 (10.6k)
-            // 7.6 / 7.2. Eight heads per K/V head are more arithmetic: 64/8 of 128 700 (6.3k) 9.0 / 8.4, 1000 (8.8k) 9.1 / 9.7.
-            // Many splits: 28/7 of 128 fp32 (21) 4200 (13.7k) 15.4 / 10.6, 4/1 of 128 (148) 5000 (36k) 17.0 / 10.0, 20000 (143k)
-            // 19.3 / 20.8; eight heads 16/2 of 128 (74) 3500 (22k) 15.2 / 11.4, 5000 (31k) 13.8 / 13.9, fp32 12.8 / 15.0.
-            constexpr bool half = sizeof(T) == 2;
-            const unsigned more = R == 8 ? (nsplit > 40 ? 18432u : half ? 7168u : 6144u) : (nsplit > 20 ? 49152u : half ? 16384u : 12288u);
+            // longer, and that is to cost less than the merging kernel (1-1.5 us). Measured, us for two launches / one, with the
+            // longer ranges' elements per head, fp16 unless noted: 32/8 heads of 128 500 positions (4k) 7.3 / 6.5, 850 (7.5k) 7.3 /
+            // 7.5; 28/7 1250 (2.4k) 7.2 / 6.8, fp32 850 (1.7k) 6.5 / 6.7, 1250 (2.4k) 7.4 / 6.8, 2500 (4.7k) 8.3 / 8.3; 32/4 of 64 1250
+            // (2.9k) 7.8 / 7.0, 1800 (4.1k) 7.8 / 8.4, fp32 850 (1.4k) 6.2 / 5.6, 1250 6.2 / 6.4. One or two heads are less arithmetic per
+            // position: 16/8 of 64 1800 (8k) 6.6 / 5.8, 2500 (11k) 6.7 / 6.8; 40/40 of 128 fp32 500 (10.6k) 7.6 / 7.2, 850 (18k) 10.6 / 11.0.
+            const unsigned more = R <= 2 ? 10752u : sizeof(T) == 4 ? 2048u : R == 8 ? 3072u : 4608u;
             const unsigned longest = cdiv(allow, nsplit) + more / DH;
             // 32 positions are a short stage; eight heads of 128 need the CTAs for the merge too (16/2, 140 fp32 positions: 6.4 us with 32, 6.1 with 8)
             unsigned cs = kMaxCluster;

@@ -55,12 +55,14 @@ def test_ranges_around_a_stage(cuda, torch_mod, orc, KVH, rep, allow):
 
 @pytest.mark.parametrize("half", [False, True])
 @pytest.mark.parametrize("KVH,rep,dh,allow", [
-    (8, 4, 128, 3), (8, 4, 128, 1830), (8, 4, 128, 1900), (4, 8, 64, 3168), (4, 8, 64, 3190), (2, 4, 64, 15680), (2, 4, 64, 15700), (1, 8, 64, 17),
-    (1, 8, 128, 2816), (1, 8, 128, 2817), (5, 4, 128, 50), (3, 1, 64, 511), (37, 2, 64, 300), (74, 1, 128, 40), (148, 1, 64, 40), (149, 1, 64, 9),
+    (8, 4, 128, 3), (8, 4, 128, 500), (8, 4, 128, 620), (4, 8, 64, 1340), (4, 8, 64, 1380), (2, 4, 64, 1150), (2, 4, 64, 1500), (1, 8, 64, 17),
+    (1, 8, 128, 760), (1, 8, 128, 910), (5, 4, 128, 50), (3, 1, 64, 511), (37, 2, 64, 300), (74, 1, 128, 40), (148, 1, 64, 40), (149, 1, 64, 9),
+    (4, 4, 64, 9000), (3, 4, 128, 9000), (2, 2, 64, 20000), (1, 8, 128, 4800),
 ])
 def test_one_launch(cuda, torch_mod, orc, KVH, rep, dh, allow, half):
     """Around the lines between one launch and two: clusters of 16 down to 1, splits without a position, K/V heads that are no
-    power of two or more than fit at a time. The arithmetic is the same in both, and so is the bound."""
+    power of two or more than fit at a time; merges of 37, 49, 74 and 148 splits. The arithmetic is the same in both, and so is the
+    bound."""
     run(cuda, torch_mod, orc, KVH, rep, dh, allow + 3, allow, half)
 
 
