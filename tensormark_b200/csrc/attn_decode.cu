@@ -7,7 +7,8 @@
 // over a range of positions, one CTA per SM. The rows of a K/V head are contiguous, so a producer thread streams them
 // in 32 KB pieces (bulk copies into a ring of stages, some 190 KB in flight per SM) and nothing but the ring
 // limits the bytes in flight: the kernel this replaced read each row with a 2-byte-per-lane load, reduced every score
-// with five shuffles and waited for each position in turn (32 / 8 heads of 128, 8191 fp16 positions: 113.8 us against 15.9 us with the merge; the bytes alone take 5.1 us).
+// with five shuffles and waited for each position in turn (32 / 8 heads of 128, 8191 fp16
+// positions: 113.8 us against 15.9 us, with today's merge 12.9; the bytes alone take 5.1 us).
 //   * A warp takes 2 KB of K and of V of every stage (4 loads of 16 bytes per lane, the lanes of a row side by side) and
 //     keeps its own running maximum and sums: no barrier between warps until the range is finished.
 //   * The products of 4 loads x REP heads are summed over a row's lanes by a transposing butterfly (each step halves the
