@@ -1015,9 +1015,7 @@ __global__ void __launch_bounds__(256) prepass_f16(const uint8_t* __restrict__ W
     if (blockIdx.x >= blocks_w) return round_activations(A, Ah, n4, (size_t)(blockIdx.x - blocks_w) * (256 * kPrepItems) + threadIdx.x);
     constexpr uint32_t EN = Eight<DT>::N;                                  // weights per item
     const uint32_t per = K / EN;
-    // The last rows first: the GEMM starts with the first ones and finds in L2 what was written last (2000 x 5632 x 2048 Q4_0
-    // 60.3 -> 59.4 us).
-    const uint64_t total = (uint64_t)N * per, first = (uint64_t)(blocks_w - 1u - blockIdx.x) * (256 * kPrepItems) + threadIdx.x;
+    const uint64_t total = (uint64_t)N * per, first = (uint64_t)blockIdx.x * (256 * kPrepItems) + threadIdx.x;
     Eight<DT> e[kPrepItems];
 #pragma unroll
     for (int i = 0; i < kPrepItems; ++i) {
