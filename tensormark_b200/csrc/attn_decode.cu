@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "bulk.cuh"
 #include "glue.h"
+#include "per_device.h"
 
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -528,12 +529,23 @@ __global__ void __launch_bounds__(kMergeGroups * 128) attn_combine_kernel(const 
     out[(size_t)head * dh + d] = o * inv;
 }
 
+// Function attributes are a device's own: what the launches below prepare, they prepare for the device that is current.
+int current_device() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+    return dev;
+}
+
 template <typename T, int DH, int REP>
 bool launch_stream(dim3 grid, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat, unsigned H, unsigned ctx,
                    unsigned allow, unsigned chunk, float scale, const int* state) {
-    static const cudaError_t attr = cudaFuncSetAttribute(attn_stream_kernel<T, DH, REP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem);
-    if (attr != cudaSuccess) return fail("attention: shared memory attribute: %s", cudaGetErrorString(attr));
-    launch_pdl(attn_stream_kernel<T, DH, REP, false>, grid, dim3(32 * (Split<REP>::Warps + 1)), Split<REP>::Smem, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state, device_status_word());
+    auto* kernel = attn_stream_kernel<T, DH, REP, false>;
+    static PerDevice<bool> ready;
+    if (!ready.get(current_device(), [=](bool&) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem);
+            return e == cudaSuccess || fail("attention: shared memory attribute: %s", cudaGetErrorString(e));
+        })) return false;
+    launch_pdl(kernel, grid, dim3(32 * (Split<REP>::Warps + 1)), Split<REP>::Smem, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state, device_status_word());
     return true;
 }
 
@@ -550,11 +562,11 @@ bool launch_cluster(unsigned cs, unsigned KVH, cudaStream_t st, const float* q, 
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    struct Fits { int clusters[5]; };
-    static const Fits fits = [&] {                          // clusters of 1, 2, 4, 8, 16 that run at a time
-        Fits f = {};
+    struct Fits { int clusters[5]; };                       // of 1, 2, 4, 8, 16 CTAs, that run at a time
+    static PerDevice<Fits> device;
+    const Fits* fits = device.get(current_device(), [&](Fits& f) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem) != cudaSuccess ||
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return f; }
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return false; }
         cudaLaunchConfig_t c = cfg;
         cudaLaunchAttribute a = at[0];
         c.attrs = &a; c.numAttrs = 1;
@@ -563,11 +575,11 @@ bool launch_cluster(unsigned cs, unsigned KVH, cudaStream_t st, const float* q, 
             c.gridDim = dim3(1, 1u << i);
             if (cudaOccupancyMaxActiveClusters(&f.clusters[i], kernel, &c) != cudaSuccess) { cudaGetLastError(); f.clusters[i] = 0; }
         }
-        return f;
-    }();
+        return true;
+    });
     int i = 0;
     while (1u << i < cs) ++i;
-    if (fits.clusters[i] < (int)KVH) return false;
+    if (!fits || fits->clusters[i] < (int)KVH) return false;
     static const bool pdl = [] { const char* e = std::getenv("TM_GLUE_PDL"); return !(e && *e == '0'); }();
     cfg.numAttrs = pdl ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, q, kc, vc, out, (float*)nullptr, (uint32_t)H, (uint32_t)ctx, (uint32_t)allow, (uint32_t)cdiv(allow, cs), scale, state, device_status_word());

@@ -14,41 +14,33 @@
 #include "cuda_shim.h"
 #include "common.cuh"
 #include "glue.h"
+#include "per_device.h"
 
-#include <atomic>
 #include <cmath>
 
 namespace tmc {
 namespace {
 
 constexpr size_t kStaticScratchBytes = TM_CUDA_ATTN_STATIC_SCRATCH_BYTES;
-constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) float g_attn_scratch[kStaticScratchBytes / sizeof(float)];
 
-struct PerDevice {
-    std::atomic<float*> scratch{nullptr};   // device address of g_attn_scratch on this device; published last
-    int sms = 0;
+struct Device {
+    float* scratch;                         // address of g_attn_scratch on this device
+    int sms;
 };
-PerDevice g_dev[kMaxDevices];
 
-// Resolve the array's address on the current device (first call on that device only). Two host threads that make
-// their first call at once both look the address up and store the same two values; the address is stored last with
-// release order, so whoever reads it non-null also reads the SM count.
-PerDevice* current_device() {
+// nullptr (with the reason recorded): no current device, or the array's address or the SM count cannot be read.
+const Device* current_device() {
+    static PerDevice<Device> devices;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) { fail("attn_decode_static: no current CUDA device"); return nullptr; }
-    PerDevice& d = g_dev[dev];
-    if (!d.scratch.load(std::memory_order_acquire)) {
-        float* p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress((void**)&p, g_attn_scratch);
-        if (e != cudaSuccess || !p) { fail("attn_decode_static: cudaGetSymbolAddress: %s", cudaGetErrorString(e)); return nullptr; }
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) { fail("attn_decode_static: cannot read the SM count"); return nullptr; }
-        d.sms = sms;
-        d.scratch.store(p, std::memory_order_release);
-    }
-    return &d;
+    return devices.get(dev, [dev](Device& d) {
+        const cudaError_t e = cudaGetSymbolAddress((void**)&d.scratch, g_attn_scratch);
+        if (e != cudaSuccess || !d.scratch) return fail("attn_decode_static: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
+        if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || d.sms <= 0) return fail("attn_decode_static: cannot read the SM count");
+        return true;
+    });
 }
 
 }  // namespace
@@ -62,7 +54,7 @@ extern "C" bool tm_cuda_attn_decode_static_dev(const float* q, const void* kc, c
     if (!q || !kc || !vc || !out) return fail("attn_decode_static: null pointer");
     if (!H || !KVH || !dh || !ctx || !allow || allow > ctx || H % KVH || !std::isfinite(scale) || scale <= 0)
         return fail("attn_decode_static: invalid decode attention dimensions or scale");
-    PerDevice* d = current_device();
+    const Device* d = current_device();
     if (!d) return false;
     const unsigned REP = H / KVH;
     if (dh != 64 && dh != 128) return fail("attn_decode_static: head dimension %u (64 and 128 are built)", dh);
@@ -77,6 +69,6 @@ extern "C" bool tm_cuda_attn_decode_static_dev(const float* q, const void* kc, c
                     "use tm_cuda_attn_decode_dev with a buffer of your own", need, kStaticScratchBytes);
     // Nothing has to be cleared: every word the combine pass reads was written by the split
     // pass of this same call.
-    return launch_attention(q, kc, vc, kv_half != 0, d->scratch.load(std::memory_order_acquire), out, H, KVH, dh, ctx, allow, scale, REP, pl,
+    return launch_attention(q, kc, vc, kv_half != 0, d->scratch, out, H, KVH, dh, ctx, allow, scale, REP, pl,
                             (cudaStream_t)stream);
 }

@@ -134,3 +134,24 @@ extern "C" __attribute__((visibility("default"))) int hc_share_count_selftest() 
     c.total = device = ~0u - 1u;                     // and past the counter's end
     return launch(8) && c.total == 6u ? 0 : 4;
 }
+
+// What is prepared on one device is not taken for prepared on another, a preparation that failed is tried again, and threads
+// that arrive together prepare once. 0: so it is.
+#include "../../tensormark_b200/csrc/per_device.h"
+#include <thread>
+extern "C" __attribute__((visibility("default"))) int hc_per_device_selftest() {
+    tmc::PerDevice<int> p;
+    int made = 0;
+    auto get = [&](int device, bool works) { return p.get(device, [&](int& v) { ++made; v = 100 + device; return works; }); };
+    const int* a = get(0, true);
+    if (!a || *a != 100 || get(0, true) != a || made != 1) return 1;
+    if (get(1, false) || made != 2) return 2;
+    const int* b = get(1, true);
+    if (!b || *b != 101 || b == a || *a != 100 || made != 3) return 3;
+    if (get(-1, true) || get(tmc::kMaxDevices, true) || made != 3) return 4;
+    std::vector<std::thread> threads;
+    std::atomic<int> right{0};
+    for (int i = 0; i < 8; ++i) threads.emplace_back([&] { const int* c = get(tmc::kMaxDevices - 1, true); right += c && *c == 100 + tmc::kMaxDevices - 1; });
+    for (std::thread& t : threads) t.join();
+    return right == 8 && made == 4 ? 0 : 5;
+}

@@ -77,6 +77,21 @@ def test_failed_launch_is_not_counted(hc):
     assert hc.hc_share_count_selftest() == 0
 
 
+def test_devices_are_prepared_one_by_one(hc):
+    assert hc.hc_per_device_selftest() == 0
+
+
+def test_attention_sets_function_attributes_on_each_device():
+    """The attention entries serve the device that is current, so an attribute set once per process is missing on the next
+    device: no result of cudaFuncSetAttribute or of an occupancy query in a static of its own."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "tensormark_b200", "csrc", "attn_decode.cu")).read())
+    assert len(re.findall(r"cudaFuncSetAttribute\(|cudaOccupancyMaxActiveClusters\(", text)) == 4
+    statics = re.findall(r"static\s+const\s[^;]*?=[^;]*", text)
+    assert not [s for s in statics if re.search(r"cudaFuncSet|cudaOccupancy|Fits", s)]
+    for at in (m.start() for m in re.finditer(r"cudaFuncSetAttribute\(", text)):
+        assert ".get(current_device()," in text[max(0, at - 400):at]
+
+
 @pytest.mark.parametrize("dt", [synth.Q4_0, synth.Q5_K])
 def test_gemv_pool_rows(hc, orc, dt):
     n, k = 200, 512                         # 200 rows: three full 64-row chunks and a ragged one
