@@ -29,8 +29,6 @@
 namespace tmc {
 namespace {
 
-inline unsigned cdiv(unsigned a, unsigned b) { return (a + b - 1) / b; }
-
 template <typename... P, typename... A>
 void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     static const bool on = [] { const char* e = std::getenv("TM_GLUE_PDL"); return !(e && *e == '0'); }();
@@ -48,7 +46,6 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // ---- the streaming kernel ------------------------------------------------------------------------------------------
-constexpr uint32_t kMaxCluster = 16;                        // splits that one launch merges
 constexpr int kLoads = 4;                                   // 16-byte loads per lane, of K and of V, per stage
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -582,39 +579,29 @@ bool launch_cluster(unsigned cs, unsigned KVH, cudaStream_t st, const float* q, 
     if (!fits || fits->clusters[i] < (int)KVH) return false;
     static const bool pdl = [] { const char* e = std::getenv("TM_GLUE_PDL"); return !(e && *e == '0'); }();
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, kernel, q, kc, vc, out, (float*)nullptr, (uint32_t)H, (uint32_t)ctx, (uint32_t)allow, (uint32_t)cdiv(allow, cs), scale, state, device_status_word());
+    cudaLaunchKernelEx(&cfg, kernel, q, kc, vc, out, (float*)nullptr, (uint32_t)H, (uint32_t)ctx, (uint32_t)allow, (uint32_t)attn_cdiv(allow, cs), scale, state, device_status_word());
     return true;
 }
 // One K/V head per grid column. The streaming kernel copies whole rows in bulk and wants the caches on 16-byte boundaries;
 // caches on any other address take the element-wise one.
 template <typename T, int DH>
-bool launch_splits(unsigned REP, unsigned KVH, unsigned nsplit, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat, float* out,
-                   unsigned H, unsigned ctx, unsigned allow, unsigned chunk, float scale, const int* state, bool* merged) {
+bool launch_splits(unsigned sms, unsigned REP, unsigned KVH, AttnSplits sp, cudaStream_t st, const float* q, const T* kc, const T* vc, float* part, float* stat, float* out,
+                   unsigned H, unsigned ctx, unsigned allow, float scale, const int* state, bool* merged) {
     static const bool one = [] { const char* e = std::getenv("TM_ATTN_CLUSTER"); return !(e && *e == '0'); }();   // A/B knob
-    const dim3 grid(KVH, nsplit);
+    const dim3 grid(KVH, sp.nsplit);
     const bool bulk = (uintptr_t)kc % 16 == 0 && (uintptr_t)vc % 16 == 0;
     bool ok = true;
     *merged = false;
     auto go = [&](auto rep) {
         constexpr int R = decltype(rep)::value;
         if (bulk && one) {
-            // A cluster has a power of two of CTAs, so fewer than the SMs allow: its CTAs read for longer by what their ranges are
-            // longer, and that is to cost less than the merging kernel (1-1.5 us). Measured, us for two launches / one, with the
-            // longer ranges' elements per head, fp16 unless noted: 32/8 heads of 128 500 positions (4k) 7.3 / 6.5, 850 (7.5k) 7.3 /
-            // 7.5; 28/7 1250 (2.4k) 7.2 / 6.8, fp32 850 (1.7k) 6.5 / 6.7, 1250 (2.4k) 7.4 / 6.8, 2500 (4.7k) 8.3 / 8.3; 32/4 of 64 1250
-            // (2.9k) 7.8 / 7.0, 1800 (4.1k) 7.8 / 8.4, fp32 850 (1.4k) 6.2 / 5.6, 1250 6.2 / 6.4. One or two heads are less arithmetic per
-            // position: 16/8 of 64 1800 (8k) 6.6 / 5.8, 2500 (11k) 6.7 / 6.8; 40/40 of 128 fp32 500 (10.6k) 7.6 / 7.2, 850 (18k) 10.6 / 11.0.
-            const unsigned more = R <= 2 ? 10752u : sizeof(T) == 4 ? 2048u : R == 8 ? 3072u : 4608u;
-            const unsigned longest = cdiv(allow, nsplit) + more / DH;
-            // 32 positions are a short stage; eight heads of 128 need the CTAs for the merge too (16/2, 140 fp32 positions: 6.4 us with 32, 6.1 with 8)
-            unsigned cs = kMaxCluster;
-            while (cs > 1 && (cs * KVH > (unsigned)device_sm_count() || (cs > 4 && cs > cdiv(allow, R * DH >= 1024 ? 8u : 32u)))) cs >>= 1;
-            for (; cs && cdiv(allow, cs) <= longest && !*merged; cs >>= 1)
+            const AttnClusters c = attn_clusters(sms, KVH, R, DH, sizeof(T), allow, grid.y);
+            for (unsigned cs = c.cs; cs && attn_cdiv(allow, cs) <= c.longest && !*merged; cs >>= 1)
                 *merged = launch_cluster<T, DH, R>(cs, KVH, st, q, kc, vc, out, H, ctx, allow, scale, state);
             if (*merged) return;
         }
-        if (bulk) ok = launch_stream<T, DH, R>(grid, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state);
-        else launch_pdl(attn_split_kernel<T, DH / 32, R>, grid, dim3(128), 0, st, q, kc, vc, part, stat, H, ctx, allow, chunk, scale, state);
+        if (bulk) ok = launch_stream<T, DH, R>(grid, st, q, kc, vc, part, stat, H, ctx, allow, sp.chunk, scale, state);
+        else launch_pdl(attn_split_kernel<T, DH / 32, R>, grid, dim3(128), 0, st, q, kc, vc, part, stat, H, ctx, allow, sp.chunk, scale, state);
     };
     switch (REP) {
         case 1: go(std::integral_constant<int, 1>{}); break;
@@ -630,53 +617,29 @@ bool launch_splits(unsigned REP, unsigned KVH, unsigned nsplit, cudaStream_t st,
 
 }  // namespace
 
-AttnPlan plan_attention(unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t probs_bytes) {
-    return plan_attention_sms((unsigned)device_sm_count(), H, KVH, dh, ctx, allow, probs_bytes);
-}
-AttnPlan plan_attention_sms(unsigned sms, unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t probs_bytes) {
-    AttnPlan pl{};
-    // Enough (kv head, split) CTAs to cover the machine; every split at least 32
-    // positions; the partials must fit the caller's probs buffer.
-    unsigned nsplit = cdiv(sms, KVH);
-    nsplit = nsplit < cdiv(allow, 32u) ? nsplit : cdiv(allow, 32u);
-    const size_t per_split = (size_t)H * (dh + 2) * sizeof(float);
-    const unsigned fit = (unsigned)(probs_bytes / per_split);
-    if (fit == 0) { pl.nsplit = 0; return pl; }
-    if (nsplit > fit) nsplit = fit;
-    if (nsplit == 0) nsplit = 1;
-    pl.chunk = cdiv(allow, nsplit);
-    pl.nsplit = cdiv(allow, pl.chunk);
-    pl.part_floats = (size_t)pl.nsplit * H * dh;
-    (void)ctx;
-    return pl;
+AttnPlan plan_attention(unsigned H, unsigned KVH, unsigned dh, unsigned allow, size_t scratch_bytes) {
+    return plan_attention_sms((unsigned)device_sm_count(), H, KVH, dh, allow, scratch_bytes);
 }
 
 bool launch_attention(const float* q, const void* kc, const void* vc, bool half_cache, float* scratch, float* out,
                       unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, float scale, unsigned REP,
                       const AttnPlan& pl, cudaStream_t st, const int* state) {
     if (dh != 64 && dh != 128) return fail("attention: head dim %u unsupported (64 or 128)", dh);
-    // The plan's splits bound the scratch. No more CTAs than SMs: a CTA fills one, so one CTA over a whole wave would
-    // double the time (8 K/V heads on 148 SMs: 18 splits of the 19 planned).
-    unsigned nsplit = pl.nsplit, chunk = pl.chunk;
-    const unsigned most = (unsigned)device_sm_count() / KVH;
-    if (most && nsplit > most) {
-        nsplit = most; chunk = cdiv(allow, nsplit);
-        if (!state) nsplit = cdiv(allow, chunk);
-    }
+    const AttnSplits sp = attn_splits(pl, KVH, allow, state != nullptr);
     float* part = scratch;
     float* stat = scratch + pl.part_floats;
     bool ok, merged;
     if (half_cache) {
         const __half *k = (const __half*)kc, *v = (const __half*)vc;
-        ok = dh == 128 ? launch_splits<__half, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged)
-                       : launch_splits<__half, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged);
+        ok = dh == 128 ? launch_splits<__half, 128>(pl.sms, REP, KVH, sp, st, q, k, v, part, stat, out, H, ctx, allow, scale, state, &merged)
+                       : launch_splits<__half, 64>(pl.sms, REP, KVH, sp, st, q, k, v, part, stat, out, H, ctx, allow, scale, state, &merged);
     } else {
         const float *k = (const float*)kc, *v = (const float*)vc;
-        ok = dh == 128 ? launch_splits<float, 128>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged)
-                       : launch_splits<float, 64>(REP, KVH, nsplit, st, q, k, v, part, stat, out, H, ctx, allow, chunk, scale, state, &merged);
+        ok = dh == 128 ? launch_splits<float, 128>(pl.sms, REP, KVH, sp, st, q, k, v, part, stat, out, H, ctx, allow, scale, state, &merged)
+                       : launch_splits<float, 64>(pl.sms, REP, KVH, sp, st, q, k, v, part, stat, out, H, ctx, allow, scale, state, &merged);
     }
     if (!ok || merged) return ok;
-    launch_pdl(attn_combine_kernel, dim3(H), dim3(kMergeGroups * dh), 0, st, part, stat, out, H, dh, nsplit);
+    launch_pdl(attn_combine_kernel, dim3(H), dim3(kMergeGroups * dh), 0, st, part, stat, out, H, dh, sp.nsplit);
     note_launch();
     return check_launch("attn_combine");
 }

@@ -62,7 +62,7 @@ extern "C" bool tm_cuda_attn_decode_static_dev(const float* q, const void* kc, c
     // The allocating entry's split rule (one helper for both): enough (kv head, split) CTAs to cover the GPU, at
     // least 32 positions per split. The static array must hold all of them; a shape that needs more is refused rather
     // than run with fewer splits.
-    const AttnPlan pl = plan_attention_sms((unsigned)d->sms, H, KVH, dh, ctx, allow, (size_t)1 << 40);
+    const AttnPlan pl = plan_attention_sms((unsigned)d->sms, H, KVH, dh, allow, (size_t)1 << 40);
     const size_t need = (size_t)pl.nsplit * H * (dh + 2) * sizeof(float);
     if (need > kStaticScratchBytes)
         return fail("attn_decode_static: this shape needs %zu bytes of split-K scratch, the static array holds %zu; "

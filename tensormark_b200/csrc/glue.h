@@ -5,6 +5,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "attn_plan.h"
 #include "common.cuh"
 
 namespace tmc {
@@ -30,15 +31,8 @@ bool launch_choose_shard(const float* x, unsigned* out, unsigned lo, unsigned n,
 bool launch_choose(const float* x, unsigned* out, unsigned n, unsigned idx, float inv_temp, unsigned seed, bool sample,
                    unsigned long long* scratch, cudaStream_t st, const int* state = nullptr, const Exchange* xchg = nullptr);
 
-struct AttnPlan {
-    unsigned nsplit;        // 0: the scratch cannot hold even one split
-    unsigned chunk;         // positions per split
-    size_t part_floats;     // floats of partial outputs; the (max, sum) stats follow them
-};
-// scratch_bytes: size of the buffer that will receive partials and stats.
-AttnPlan plan_attention(unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t scratch_bytes);
-// The same rule for a caller that names the SM count itself (a scratch_bytes of 1 << 40 means: no limit from the buffer).
-AttnPlan plan_attention_sms(unsigned sms, unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, size_t scratch_bytes);
+// plan_attention_sms (attn_plan.h) for the device that the library is initialised on
+AttnPlan plan_attention(unsigned H, unsigned KVH, unsigned dh, unsigned allow, size_t scratch_bytes);
 bool launch_attention(const float* q, const void* kc, const void* vc, bool half_cache, float* scratch, float* out,
                       unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, float scale, unsigned REP,
                       const AttnPlan& pl, cudaStream_t st, const int* state = nullptr);

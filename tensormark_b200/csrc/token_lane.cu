@@ -493,7 +493,7 @@ void tm_cuda_tok_attn(int qslot, int kcslot, int vcslot, int probslot, int outsl
     // Split-K partials live in the probs slot, which the caller reserved for H*ctx floats.
     float* probs = (float*)slot_ptr(probslot, (size_t)H * (dh + 2) * 4, "tok_attn");
     if (!q || !kc || !vc || !out || !probs) return;
-    const AttnPlan pl = plan_attention(H, KVH, dh, ctx, (unsigned)allow, s.slots[probslot].bytes);
+    const AttnPlan pl = plan_attention(H, KVH, dh, (unsigned)allow, s.slots[probslot].bytes);
     if (!pl.nsplit) { latch("tok_attn: probs slot too small for one split"); return; }
     if (!launch_attention(q, kc, vc, s.kv_half, probs, out, H, KVH, dh, ctx, (unsigned)allow, scale, REP, pl, s.stream)) s.sticky = true;
 }
@@ -742,7 +742,7 @@ void tm_cuda_tok_attn_at(int qslot, int kcslot, int vcslot, int probslot, int ou
     const int* st = state_ptr(stateslot, "tok_attn_at");
     if (!q || !kc || !vc || !out || !probs || !st) return;
     // the split count is fixed for the whole chain (sized for a full context); the kernel derives its chunk from the state
-    const AttnPlan pl = plan_attention(H, KVH, dh, ctx, ctx, s.slots[probslot].bytes);
+    const AttnPlan pl = plan_attention(H, KVH, dh, ctx, s.slots[probslot].bytes);
     if (!pl.nsplit) { latch("tok_attn_at: probs slot too small for one split"); return; }
     if (!launch_attention(q, kc, vc, s.kv_half, probs, out, H, KVH, dh, ctx, ctx, scale, REP, pl, s.stream, st)) s.sticky = true;
 }
@@ -873,7 +873,7 @@ void tm_cuda_tok_graph_destroy(int id) {
 
 size_t tm_cuda_attn_decode_scratch(unsigned H, unsigned KVH, unsigned dh, unsigned ctx, unsigned allow) {
     if (!ensure_init(-1) || !H || !KVH || !dh || !allow) return 0;
-    const AttnPlan pl = plan_attention(H, KVH, dh, ctx, allow, (size_t)1 << 40);
+    const AttnPlan pl = plan_attention(H, KVH, dh, allow, (size_t)1 << 40);
     return (size_t)pl.nsplit * H * (dh + 2) * sizeof(float);
 }
 bool tm_cuda_attn_decode_dev(const float* q, const void* kc, const void* vc, float* scratch, size_t scratch_bytes,
@@ -883,7 +883,7 @@ bool tm_cuda_attn_decode_dev(const float* q, const void* kc, const void* vc, flo
     if (!q || !kc || !vc || !scratch || !out) return fail("attn_decode: null pointer");
     if (!H || !KVH || !dh || !ctx || !allow || allow > ctx || H % KVH || !std::isfinite(scale) || scale <= 0)
         return fail("attn_decode: invalid decode attention dimensions or scale");
-    const AttnPlan pl = plan_attention(H, KVH, dh, ctx, allow, scratch_bytes);
+    const AttnPlan pl = plan_attention(H, KVH, dh, allow, scratch_bytes);
     if (!pl.nsplit) return fail("attn_decode: scratch of %zu bytes cannot hold one split", scratch_bytes);
     return launch_attention(q, kc, vc, kv_half != 0, scratch, out, H, KVH, dh, ctx, allow, scale, H / KVH, pl,
                             (cudaStream_t)stream);

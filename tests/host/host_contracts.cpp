@@ -155,3 +155,15 @@ extern "C" __attribute__((visibility("default"))) int hc_per_device_selftest() {
     for (std::thread& t : threads) t.join();
     return right == 8 && made == 4 ? 0 : 5;
 }
+
+// The launch shape of decode attention on a device of `sms` SMs whose scratch is unlimited: {plan's splits, splits of two
+// launches, positions of each, first cluster size, longest range of one launch, SMs of the plan}.
+#include "../../tensormark_b200/csrc/attn_plan.h"
+extern "C" __attribute__((visibility("default"))) void hc_attn_shape(unsigned sms, unsigned KVH, unsigned rep, unsigned dh, unsigned elem_bytes,
+                                                                     unsigned allow, unsigned* out) {
+    const tmc::AttnPlan pl = tmc::plan_attention_sms(sms, KVH * rep, KVH, dh, allow, (size_t)1 << 40);
+    const tmc::AttnSplits sp = tmc::attn_splits(pl, KVH, allow, false);
+    const tmc::AttnClusters c = tmc::attn_clusters(pl.sms, KVH, rep, dh, elem_bytes, allow, sp.nsplit);
+    const unsigned v[6] = {pl.nsplit, sp.nsplit, sp.chunk, c.cs, c.longest, pl.sms};
+    std::memcpy(out, v, sizeof v);
+}

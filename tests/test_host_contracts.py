@@ -81,6 +81,28 @@ def test_devices_are_prepared_one_by_one(hc):
     assert hc.hc_per_device_selftest() == 0
 
 
+def test_attention_shape_follows_the_sms_that_the_caller_names(hc):
+    """Every split is there and none is empty; two launches take no more than a wave of CTAs, one launch no more than the SMs;
+    and nothing but the plan says how many SMs there are."""
+    shape = (C.c_uint * 6)()
+    for sms in (148, 132, 20, 1):
+        for kvh in (1, 2, 3, 5, 8, 32, 74, 149):
+            for rep in (1, 2, 4, 8):
+                for dh in (64, 128):
+                    for elem in (2, 4):
+                        for allow in (1, 31, 33, 97, 300, 500, 999, 1250, 8191, 32768):
+                            hc.hc_attn_shape(sms, kvh, rep, dh, elem, allow, shape)
+                            planned, nsplit, chunk, cs, longest, of = shape
+                            assert of == sms
+                            assert 1 <= nsplit <= planned and (nsplit * kvh <= sms or nsplit == planned == 1 or kvh > sms)
+                            assert (nsplit - 1) * chunk < allow <= nsplit * chunk
+                            assert cs in (1, 2, 4, 8, 16) and (cs * kvh <= sms or cs == 1) and longest >= chunk
+    hc.hc_attn_shape(148, 8, 4, 128, 2, 300, shape)
+    assert shape[3] * 8 <= 148 and shape[3] > 1 and -(-300 // shape[3]) <= shape[4]                  # one launch of a cluster
+    hc.hc_attn_shape(148, 8, 4, 128, 2, 8191, shape)
+    assert shape[1] == 18 and -(-8191 // shape[3]) > shape[4]                                        # two launches
+
+
 def test_attention_sets_function_attributes_on_each_device():
     """The attention entries serve the device that is current, so an attribute set once per process is missing on the next
     device: no result of cudaFuncSetAttribute or of an occupancy query in a static of its own."""

@@ -7,6 +7,10 @@ allocation on their token path; it must give what tm_cuda_attn_decode_dev gives,
 although both calls write the same array."""
 from __future__ import annotations
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -47,6 +51,38 @@ def test_static_scratch_attention_matches_twice_in_a_row(cuda, torch_mod, half):
         assert torch.cuda.memory_allocated() == before
         # the tolerance the attention parity tests use (1e-3 relative, 2e-5 absolute)
         assert np.allclose(got.cpu().numpy(), want.cpu().numpy(), rtol=1e-3, atol=2e-5)
+
+
+ALONE = """
+import ctypes as C
+import torch
+from tensormark_b200 import lib
+L = lib.load()
+torch.cuda.set_device(0)
+st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+P = lambda t: C.c_void_p(t.data_ptr())
+H, KVH, dh, ctx, scale = 32, 8, 128, 1024, 128 ** -0.5
+g = torch.Generator(device="cuda").manual_seed(5)
+q = torch.randn(H, dh, generator=g, device="cuda")
+k, v = (torch.randn(KVH, ctx, dh, generator=g, device="cuda").half() for _ in range(2))
+for allow, launches in ((300, 1), (1000, 2)):
+    out = torch.full((H, dh), float("nan"), device="cuda")
+    before = L.tm_cuda_launch_count()
+    assert L.tm_cuda_attn_decode_static_dev(P(q), P(k), P(v), P(out), H, KVH, dh, ctx, allow, scale, 1, st), lib.last_error()
+    torch.cuda.synchronize()
+    assert L.tm_cuda_launch_count() - before == launches, (allow, L.tm_cuda_launch_count() - before)
+    s = torch.einsum("grd,gpd->grp", q.double().view(KVH, H // KVH, dh), k[:, :allow].double()) * scale
+    want = torch.einsum("grp,gpd->grd", s.softmax(-1), v[:, :allow].double()).reshape(H, dh)
+    assert torch.allclose(out.double(), want, rtol=1e-3, atol=2e-5), (out - want).abs().max()
+"""
+
+
+def test_static_entry_alone_in_a_process(cuda):
+    """A host that calls nothing else: the library is not initialised, and the entry still takes the launches that the SMs of
+    the current device call for."""
+    r = subprocess.run([sys.executable, "-c", ALONE], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
 
 
 def test_static_scratch_refuses_what_does_not_fit(cuda, torch_mod):
