@@ -96,6 +96,11 @@ template <int REP> struct Split {
     static constexpr uint32_t Half = Warps * kLoads * 512, Smem = Stages * 2 * Half;      // bytes of K (or V) per stage; of the ring
 };
 
+// A wait ran out. status is null in a process that has not initialised the library: there the outputs, which are NaN, have to tell.
+__device__ __forceinline__ void note_gone(int* status) {
+    if (status) *(volatile int*)status = 1;
+}
+
 // CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
 // then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. Up to some thousand
 // positions the two launches and the way of the partials through L2 are most of the time: 32 / 8 heads of 128, 300 fp16
@@ -143,7 +148,7 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
             const uint8_t* vb = reinterpret_cast<const uint8_t*>(vc + ((size_t)kv * ctx + p0) * DH);
             uint32_t s = 0, par = 1;
             for (uint32_t t = 0; t < tiles; ++t) {
-                if (!mbar_wait(empty + 8u * s, par, &gone)) { *(volatile int*)status = 1; break; }
+                if (!mbar_wait(empty + 8u * s, par, &gone)) { note_gone(status); break; }
                 const uint32_t bytes = min((uint32_t)TP, p1 - p0 - t * TP) * ROW, bar = full + 8u * s, at = ring + s * 2u * HALF;
                 mbar_expect_tx(bar, 2u * bytes);
                 bulk_g2s(at, kb + (size_t)t * HALF, bytes, bar);
@@ -290,7 +295,6 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
             mbar_arrive_if(empty + 8u * s, lane == 0);
             if (++s == (uint32_t)kStages) { s = 0; par ^= 1u; }
         }
-        if (!ok && lane == 0) *(volatile int*)status = 1;
         // a head's sum lies over the lanes that do not name it and are not duplicates
         if constexpr (NVL > REP) {
 #pragma unroll
@@ -315,6 +319,11 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
                 for (int o = LR; o < 32; o <<= 1) { f.x += __shfl_xor_sync(0xffffffffu, f.x, o); f.y += __shfl_xor_sync(0xffffffffu, f.y, o); }
                 acc[r][j] = pack2(f.x, f.y);
             }
+        __syncwarp();
+        if (!ok) {                                                           // rows that never came were multiplied: no number may pass for the result
+            note_gone(status);
+            for (int r = 0; r < REP; ++r) sm_l[warp][r] = CUDART_NAN_F;
+        }
         // the ring is free once every warp is through with it: the warps' outputs go there
         asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
         float* out = reinterpret_cast<float*>(smem);                         // [NW][REP][DH]

@@ -103,6 +103,13 @@ def test_attention_shape_follows_the_sms_that_the_caller_names(hc):
     assert shape[1] == 18 and -(-8191 // shape[3]) > shape[4]                                        # two launches
 
 
+def test_attention_reports_a_wait_only_where_someone_listens():
+    """The static entry runs in processes that have no status word (null until the library is initialised)."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "tensormark_b200", "csrc", "attn_decode.cu")).read())
+    stores = [m.start() for m in re.finditer(r"\*\s*\((?:volatile )?int\s*\*\)\s*status\s*=[^=]|\*status\s*=[^=]|status\[\d\]\s*=[^=]", text)]
+    assert len(stores) == 1 and text[:stores[0]].rstrip().endswith("if (status)")
+
+
 def test_attention_sets_function_attributes_on_each_device():
     """The attention entries serve the device that is current, so an attribute set once per process is missing on the next
     device: no result of cudaFuncSetAttribute or of an occupancy query in a static of its own."""
