@@ -101,6 +101,16 @@ __device__ __forceinline__ void note_gone(int* status) {
     if (status) *(volatile int*)status = 1;
 }
 
+// The producer leaves when the copies of its last stages have landed, whether or not the warps that they are for still wait: what
+// a warp gives up on may come later, and the CTA's shared memory must be its own until then. The first copy that does not come
+// within the limit ends the waiting. Out of line and past the loop, where it costs nothing: the warps end no sooner.
+template <uint32_t STAGES>
+__device__ __noinline__ void land(uint32_t full, uint32_t issued) {
+    int late = 0;
+#pragma unroll 1
+    for (uint32_t i = issued > STAGES ? issued - STAGES : 0u; i < issued; ++i) (void)mbar_wait_slow(full + 8u * (i % STAGES), i / STAGES & 1u, &late, kWaitLimitNs);
+}
+
 // CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
 // then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. Up to some thousand
 // positions the two launches and the way of the partials through L2 are most of the time: 32 / 8 heads of 128, 300 fp16
@@ -146,20 +156,17 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
         if (lane == 0) {
             const uint8_t* kb = reinterpret_cast<const uint8_t*>(kc + ((size_t)kv * ctx + p0) * DH);
             const uint8_t* vb = reinterpret_cast<const uint8_t*>(vc + ((size_t)kv * ctx + p0) * DH);
-            uint32_t s = 0, par = 1;
+            uint32_t s = 0, par = 1, issued = 0;
             for (uint32_t t = 0; t < tiles; ++t) {
                 if (!mbar_wait(empty + 8u * s, par, &gone)) { note_gone(status); break; }
                 const uint32_t bytes = min((uint32_t)TP, p1 - p0 - t * TP) * ROW, bar = full + 8u * s, at = ring + s * 2u * HALF;
                 mbar_expect_tx(bar, 2u * bytes);
                 bulk_g2s(at, kb + (size_t)t * HALF, bytes, bar);
                 bulk_g2s(at + HALF, vb + (size_t)t * HALF, bytes, bar);
+                ++issued;
                 if (++s == (uint32_t)kStages) { s = 0; par ^= 1u; }
             }
-            if (*(volatile int*)&gone) {                                     // copies may be in flight: a last bounded chance to land
-                gone = 0;
-                for (uint32_t i = 0; i < (uint32_t)kStages; ++i)
-                    for (uint32_t b = 0; b < 2; ++b) (void)mbar_wait(full + 8u * i, b, &gone, 50000000ull);
-            }
+            land<(uint32_t)kStages>(full, issued);
         }
     } else {
         const uint32_t gl = (uint32_t)lane % LR, rg = (uint32_t)lane / LR;   // place in a row, row of the load
