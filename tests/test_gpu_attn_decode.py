@@ -28,14 +28,17 @@ def run(cuda, torch, orc, KVH, rep, dh, ctx, allow, half, off=0, last_v=None):
     need = cuda.tm_cuda_attn_decode_scratch(H, KVH, dh, ctx, allow)
     scratch = torch.empty(need // 4 + 1, dtype=torch.float32, device="cuda")
     out = torch.empty(H * dh, dtype=torch.float32, device="cuda")
+    launched = cuda.tm_cuda_launch_count()
     lib.check(cuda.tm_cuda_attn_decode_dev(ptr(qd), at[0], at[1], ptr(scratch), need, ptr(out), H, KVH, dh, ctx, allow, scale,
                                            int(half), stream_ptr(torch)), "attn_decode_dev")
+    launched = cuda.tm_cuda_launch_count() - launched
     torch.cuda.synchronize()
     got = out.cpu().numpy().reshape(H, dh)
     K, V = kv[0].astype(np.float32), kv[1].astype(np.float32)
     for g in range(KVH):
         want = orc.attn_group(q[g * rep:(g + 1) * rep], K[g, :allow], V[g, :allow], scale)
         assert np.allclose(got[g * rep:(g + 1) * rep], want, rtol=1e-3, atol=2e-5), (g, np.abs(got[g * rep:(g + 1) * rep] - want).max())
+    return launched
 
 
 @pytest.mark.parametrize("half", [False, True])
@@ -53,23 +56,25 @@ def test_ranges_around_a_stage(cuda, torch_mod, orc, KVH, rep, allow):
     run(cuda, torch_mod, orc, KVH, rep, 128, max(allow, 256), allow, True)
 
 
+# launches with fp32 and with fp16 caches on 148 SMs, which hold up to seven clusters of 16 CTAs that fill an SM each
 @pytest.mark.parametrize("half", [False, True])
-@pytest.mark.parametrize("KVH,rep,dh,allow", [
-    (8, 4, 128, 3), (8, 4, 128, 500), (8, 4, 128, 620), (4, 8, 64, 1340), (4, 8, 64, 1380), (2, 4, 64, 1150), (2, 4, 64, 1500), (1, 8, 64, 17),
-    (1, 8, 128, 760), (1, 8, 128, 910), (5, 4, 128, 50), (3, 1, 64, 511), (37, 2, 64, 300), (74, 1, 128, 40), (148, 1, 64, 40), (149, 1, 64, 9),
-    (4, 4, 64, 9000), (3, 4, 128, 9000), (2, 2, 64, 20000), (1, 8, 128, 4800),
+@pytest.mark.parametrize("KVH,rep,dh,allow,launches", [
+    (8, 4, 128, 3, (1, 1)), (8, 4, 128, 500, (2, 1)), (8, 4, 128, 620, (2, 2)), (4, 8, 64, 1340, (2, 1)), (4, 8, 64, 1380, (2, 2)),
+    (2, 4, 64, 1150, (2, 1)), (2, 4, 64, 1500, (2, 1)), (1, 8, 64, 17, (1, 1)), (1, 8, 128, 760, (1, 1)), (1, 8, 128, 910, (2, 2)),
+    (5, 4, 128, 50, (1, 1)), (3, 1, 64, 511, (1, 1)), (37, 2, 64, 300, (1, 1)), (74, 1, 128, 40, (1, 1)), (148, 1, 64, 40, (1, 1)),
+    (149, 1, 64, 9, (2, 2)), (4, 4, 64, 9000, (2, 2)), (3, 4, 128, 9000, (2, 2)), (2, 2, 64, 20000, (2, 2)), (1, 8, 128, 4884, (2, 2)),
 ])
-def test_one_launch(cuda, torch_mod, orc, KVH, rep, dh, allow, half):
+def test_one_launch(cuda, torch_mod, orc, KVH, rep, dh, allow, launches, half):
     """Around the lines between one launch and two: clusters of 16 down to 1, splits without a position, K/V heads that are no
     power of two or more than fit at a time; merges of 37, 49, 74 and 148 splits. The arithmetic is the same in both, and so is the
-    bound."""
-    run(cuda, torch_mod, orc, KVH, rep, dh, allow + 3, allow, half)
+    bound; the launches say which of the two it was."""
+    assert run(cuda, torch_mod, orc, KVH, rep, dh, allow + 3, allow, half) == launches[half]
 
 
 @pytest.mark.parametrize("half", [False, True])
 def test_caches_off_the_grid(cuda, torch_mod, orc, half):
-    run(cuda, torch_mod, orc, 2, 4, 128, 300, 257, half, off=1)
-    run(cuda, torch_mod, orc, 3, 8, 64, 300, 300, half, off=3)
+    assert run(cuda, torch_mod, orc, 2, 4, 128, 300, 257, half, off=1) == 2
+    assert run(cuda, torch_mod, orc, 3, 8, 64, 300, 300, half, off=3) == 2
 
 
 @pytest.mark.parametrize("half", [False, True])
