@@ -20,35 +20,40 @@ from tests.gpu_util import ptr, stream_ptr
 pytestmark = pytest.mark.gpu
 
 
-def _case(torch, Hn, KVH, dh, ctx, seed, half):
+def _case(torch, Hn, KVH, dh, ctx, seed, half, off=0):
+    """q, K, V; off: elements that the caches lie behind a 16-byte boundary."""
     g = torch.Generator(device="cuda").manual_seed(seed)
     q = torch.randn(Hn * dh, generator=g, device="cuda", dtype=torch.float32)
-    k = torch.randn(KVH * ctx * dh, generator=g, device="cuda", dtype=torch.float32)
-    v = torch.randn(KVH * ctx * dh, generator=g, device="cuda", dtype=torch.float32)
+    k = torch.randn(KVH * ctx * dh + 8, generator=g, device="cuda", dtype=torch.float32)
+    v = torch.randn(KVH * ctx * dh + 8, generator=g, device="cuda", dtype=torch.float32)
     if half:
         k, v = k.half(), v.half()
-    return q, k, v
+    return q, k[off:], v[off:]
 
 
 @pytest.mark.parametrize("half", [1, 0])
-def test_static_scratch_attention_matches_twice_in_a_row(cuda, torch_mod, half):
+def test_static_scratch_attention_matches_call_after_call(cuda, torch_mod, half):
+    """Calls in a row share the array, and only the form of two launches uses it: a long call, a shorter one with as many splits
+    (18), one with four (caches off the 16-byte grid are merged by a second launch at any length), one in a single launch, and
+    again a long one."""
     torch = torch_mod
     Hn, KVH, dh, ctx = 32, 8, 128, 1024          # the decode-chain head geometry
     scale = 1.0 / np.sqrt(dh)
     sp = stream_ptr(torch)
-    for call, allow in enumerate((640, 97)):      # two calls in a row share the array; the second is shorter
-        q, k, v = _case(torch, Hn, KVH, dh, ctx, 20 + call, half)
+    for call, (allow, off, launches) in enumerate([(1000, 0, 2), (640, 0, 2), (97, 1, 2), (97, 0, 1), (1024, 0, 2)]):
+        q, k, v = _case(torch, Hn, KVH, dh, ctx, 20 + call, half, off)
         need = cuda.tm_cuda_attn_decode_scratch(Hn, KVH, dh, ctx, allow)
         scratch = torch.empty(need // 4 + 4, dtype=torch.float32, device="cuda")
         want = torch.empty(Hn * dh, dtype=torch.float32, device="cuda")
         got = torch.full((Hn * dh,), float("nan"), dtype=torch.float32, device="cuda")
         lib.check(cuda.tm_cuda_attn_decode_dev(ptr(q), ptr(k), ptr(v), ptr(scratch), need, ptr(want), Hn, KVH, dh, ctx,
                                                allow, scale, half, sp), "tm_cuda_attn_decode_dev")
-        before = torch.cuda.memory_allocated()
+        before, launched = torch.cuda.memory_allocated(), cuda.tm_cuda_launch_count()
         lib.check(cuda.tm_cuda_attn_decode_static_dev(ptr(q), ptr(k), ptr(v), ptr(got), Hn, KVH, dh, ctx, allow, scale,
                                                       half, sp), "tm_cuda_attn_decode_static_dev")
         torch.cuda.synchronize()
         assert torch.cuda.memory_allocated() == before
+        assert cuda.tm_cuda_launch_count() - launched == launches
         # the tolerance the attention parity tests use (1e-3 relative, 2e-5 absolute)
         assert np.allclose(got.cpu().numpy(), want.cpu().numpy(), rtol=1e-3, atol=2e-5)
 
