@@ -103,12 +103,12 @@ __device__ __forceinline__ void note_gone(int* status) {
 
 // The producer leaves when the copies of its last stages have landed, whether or not the warps that they are for still wait: what
 // a warp gives up on may come later, and the CTA's shared memory must be its own until then. The first copy that does not come
-// within the limit ends the waiting. Out of line and past the loop, where it costs nothing: the warps end no sooner.
+// within the limit ends the waiting. Out of line, with its flag in shared memory and the count kept outside the loop, it costs nothing
+// (8191 fp16 positions of 32 / 8 heads 13.04 us without and with it; a counter in the loop and a flag on the stack: 13.13).
 template <uint32_t STAGES>
-__device__ __noinline__ void land(uint32_t full, uint32_t issued) {
-    int late = 0;
+__device__ __noinline__ void land(uint32_t full, uint32_t issued, int* late) {
 #pragma unroll 1
-    for (uint32_t i = issued > STAGES ? issued - STAGES : 0u; i < issued; ++i) (void)mbar_wait_slow(full + 8u * (i % STAGES), i / STAGES & 1u, &late, kWaitLimitNs);
+    for (uint32_t i = issued > STAGES ? issued - STAGES : 0u; i < issued; ++i) (void)mbar_wait_slow(full + 8u * (i % STAGES), i / STAGES & 1u, late, kWaitLimitNs);
 }
 
 // CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
@@ -127,7 +127,7 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
     static_assert(TP * ROW == HALF, "a stage is whole rows");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[2 * kStages];
-    __shared__ int gone;
+    __shared__ int gone, late;
     __shared__ __align__(16) float pbuf[NW][PW][REP];                        // a warp's weights of its positions
     __shared__ __align__(16) float cbuf[NW][REP];                            // its correction factors
     __shared__ float sm_m[NW][REP], sm_l[NW][REP];
@@ -139,7 +139,7 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
     if (threadIdx.x == 0) {
         nothing = make_uint4(0u, 0u, 0u, 0u);
         for (int s = 0; s < kStages; ++s) { mbar_init(smem_u32(&bars[s]), 1); mbar_init(smem_u32(&bars[kStages + s]), NW); }
-        gone = 0;
+        gone = 0; late = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_enter();
@@ -156,17 +156,16 @@ attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float*
         if (lane == 0) {
             const uint8_t* kb = reinterpret_cast<const uint8_t*>(kc + ((size_t)kv * ctx + p0) * DH);
             const uint8_t* vb = reinterpret_cast<const uint8_t*>(vc + ((size_t)kv * ctx + p0) * DH);
-            uint32_t s = 0, par = 1, issued = 0;
+            uint32_t s = 0, par = 1, issued = tiles;
             for (uint32_t t = 0; t < tiles; ++t) {
-                if (!mbar_wait(empty + 8u * s, par, &gone)) { note_gone(status); break; }
+                if (!mbar_wait(empty + 8u * s, par, &gone)) { note_gone(status); issued = t; break; }
                 const uint32_t bytes = min((uint32_t)TP, p1 - p0 - t * TP) * ROW, bar = full + 8u * s, at = ring + s * 2u * HALF;
                 mbar_expect_tx(bar, 2u * bytes);
                 bulk_g2s(at, kb + (size_t)t * HALF, bytes, bar);
                 bulk_g2s(at + HALF, vb + (size_t)t * HALF, bytes, bar);
-                ++issued;
                 if (++s == (uint32_t)kStages) { s = 0; par ^= 1u; }
             }
-            land<(uint32_t)kStages>(full, issued);
+            land<(uint32_t)kStages>(full, issued, &late);
         }
     } else {
         const uint32_t gl = (uint32_t)lane % LR, rg = (uint32_t)lane / LR;   // place in a row, row of the load
