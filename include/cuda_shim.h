@@ -150,7 +150,10 @@ bool tm_cuda_attn_decode_dev(const float* q, const void* kc, const void* vc, flo
  * fit are refused (false, tm_cuda_last_error() says how many bytes were needed). The first call on
  * a device looks up the array's device address: make that call before any stream capture starts.
  * Every call shares the one array, so calls that may overlap on the GPU (different streams,
- * different threads) race with each other; within one stream, back-to-back calls are safe. */
+ * different threads) race with each other; within one stream, back-to-back calls are safe.
+ * The call serves the device that is current, whichever the library was initialised on, and needs no
+ * tm_cuda_init. Without it there is no status word: should a bounded wait of the kernel run out,
+ * no later entry reports it, and the outputs are NaN. */
 #define TM_CUDA_ATTN_STATIC_SCRATCH_BYTES (512u * 1024u)
 bool tm_cuda_attn_decode_static_dev(const float* q, const void* kc, const void* vc, float* out, unsigned H,
                                     unsigned KVH, unsigned dh, unsigned ctx, unsigned allow, float scale,

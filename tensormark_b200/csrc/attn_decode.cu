@@ -7,8 +7,8 @@
 // over a range of positions, one CTA per SM. The rows of a K/V head are contiguous, so a producer thread streams them
 // in 32 KB pieces (bulk copies into a ring of stages, some 190 KB in flight per SM) and nothing but the ring
 // limits the bytes in flight: the kernel this replaced read each row with a 2-byte-per-lane load, reduced every score
-// with five shuffles and waited for each position in turn (32 / 8 heads of 128, 8191 fp16
-// positions: 113.8 us against 15.9 us, with today's merge 12.9; the bytes alone take 5.1 us).
+// with five shuffles and waited for each position in turn (32 / 8 heads of 128, 8191 fp16 positions: 113.8 us, now 14.0 with K and
+// V from HBM, whose bytes alone take 5.1, and 11.9 with K and V in L2).
 //   * A warp takes 2 KB of K and of V of every stage (4 loads of 16 bytes per lane, the lanes of a row side by side) and
 //     keeps its own running maximum and sums: no barrier between warps until the range is finished.
 //   * The products of 4 loads x REP heads are summed over a row's lanes by a transposing butterfly (each step halves the
@@ -112,9 +112,9 @@ __device__ __noinline__ void land(uint32_t full, uint32_t issued, int* late) {
 }
 
 // CLUSTER: the splits of a K/V head are one cluster (1, gridDim.y) whose CTAs merge through distributed shared memory; part is
-// then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. Up to some thousand
-// positions the two launches and the way of the partials through L2 are most of the time: 32 / 8 heads of 128, 300 fp16
-// positions 7.1 us with the merging kernel, 6.4 us in one launch.
+// then the output itself and stat is not used. Else every split leaves a partial for the merging kernel. In short calls the
+// two launches and the way of the partials through L2 are most of the time (32 / 8 heads of 128, 300 fp16 positions: 7.1 us with the
+// merging kernel, 6.3 us in one launch); attn_plan.h says where the line lies, some 500 positions for these heads.
 template <typename T, int DH, int REP, bool CLUSTER>
 __global__ void __launch_bounds__(32 * (Split<REP>::Warps + 1), 1)
 attn_stream_kernel(const float* q, const T* kc, const T* vc, float* part, float* stat, uint32_t H, uint32_t ctx, uint32_t allow,
@@ -482,9 +482,10 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* q, const T
 
 // out[head][d] = sum_s e^(m_s - M) part_s[d] / sum_s e^(m_s - M) l_s. One CTA per head; bound by its chain of round trips to
 // L2. Four threads per dim take every fourth split, so 40 partials are on their way at a time, while a lane per split reads
-// its maximum and sum at once and works out the weights. With a thread per dim, 20 partials at a time and the maxima read
-// before the sums: 32 / 8 heads of 128, 8191 fp16 positions (18 splits) 15.1 us with the split kernel, now 13.4; 32 / 4 of 64
-// (37) 11.0 / 9.4; 8 / 1 of 128 (148) 22.6 / 11.8; 40 / 40 of 128 (3) 31.0 / 31.0.
+// its maximum and sum at once and works out the weights. A thread per dim, 20 partials at a time and the maxima read
+// before the sums, against this, us with the split kernel, 8191 fp16 positions, K and V in L2 (from HBM): 32 / 8 heads of 128 (18 splits)
+// 13.5 / 11.9 (15.5 / 14.0); 32 / 4 of 64 (37) 11.0 / 9.4 (12.0 / 10.6); 8 / 1 of 128 (147) 22.4 / 11.7 (22.9 / 12.1); 40 / 40 of 128 (3)
+// 31.0 / 31.0 (31.1 / 31.0).
 constexpr uint32_t kMergeGroups = 4;
 __global__ void __launch_bounds__(kMergeGroups * 128) attn_combine_kernel(const float* part, const float* stat, float* out, uint32_t H, uint32_t dh, uint32_t nsplit) {
     constexpr uint32_t BATCH = 10, G = kMergeGroups, MOST = 256;

@@ -51,11 +51,19 @@ inline AttnSplits attn_splits(const AttnPlan& pl, unsigned KVH, unsigned allow, 
 // cdiv(allow, cs) are at most `longest` positions; two launches where none is.
 //
 // A cluster has a power of two of CTAs, so fewer than the SMs allow: its CTAs read for longer by what their ranges are
-// longer, and that is to cost less than the merging kernel (1-1.5 us). Measured, us for two launches / one, with the
-// longer ranges' elements per head, fp16 unless noted: 32/8 heads of 128 500 positions (4k) 7.3 / 6.5, 850 (7.5k) 7.3 /
-// 7.5; 28/7 1250 (2.4k) 7.2 / 6.8, fp32 850 (1.7k) 6.5 / 6.7, 1250 (2.4k) 7.4 / 6.8, 2500 (4.7k) 8.3 / 8.3; 32/4 of 64 1250
-// (2.9k) 7.8 / 7.0, 1800 (4.1k) 7.8 / 8.4, fp32 850 (1.4k) 6.2 / 5.6, 1250 6.2 / 6.4. One or two heads are less arithmetic per
-// position: 16/8 of 64 1800 (8k) 6.6 / 5.8, 2500 (11k) 6.7 / 6.8; 40/40 of 128 fp32 500 (10.6k) 7.6 / 7.2, 850 (18k) 10.6 / 11.0.
+// longer, and that is to cost less than the merging kernel (1-1.5 us). The line is a number of elements per head by which
+// the ranges are longer. Measured on both sides of it, us for two launches / one, K and V partly in L2:
+//   four heads, fp16 (4608): 4.0k 7.3 / 6.4 (32/8 heads of 128, 500 positions), 4.5k 7.5 / 6.8 (20/5, 1250); 6.4k 7.5 / 7.9 (20/5, 1800),
+//     7.6k 7.3 / 7.5 (32/8, 850)
+//   eight heads, fp16 (3072): 2.9k 7.8 / 6.9 (32/4 of 64, 1250), 3.0k 7.2 / 6.9 (16/2 of 64, 1250); 4.0k 8.1 / 8.4 (64/8 of 128, 500),
+//     4.1k 7.8 / 8.4 (32/4, 1800)
+//   four or eight heads, fp32 (2048): 1.0k 6.2 / 5.5 (32/8 of 128, 300), 1.4k 6.0 / 5.5 (32/4 of 64, 850), 1.7k 6.5 / 6.6 (28/7 of 128, 850);
+//     2.8k 6.1 / 6.5 (8/2 of 128, 850), 2.9k 6.0 / 6.4 (32/4, 1250)
+//   one or two heads, less arithmetic per position (10752): 8.0k 6.6 / 5.7 (16/8 of 64, 1800), 10.6k 7.4 / 6.3 and fp32 7.5 / 7.1 (40/40 of
+//     128, 500); 11.1k 6.7 / 6.8 (16/8, 2500), 18k fp32 10.6 / 10.7 (40/40, 850)
+// The elements are not all that counts: a range is read in whole stages, and the merge of more than 40 splits makes more than one trip.
+// Of 330 calls 24 are more than 2 % slower than the other form would be, the most 8/2 of 128, 2500 positions (two) 8.6 / 7.8 and 16/2
+// of 64, 2500 (two) 9.3 / 8.3; 28/7 of 128, 1800 (one) is the only one where the line lets ranges grow too long, 7.4 / 7.9.
 constexpr unsigned kMaxCluster = 16;                        // splits that one launch merges
 struct AttnClusters { unsigned cs, longest; };
 inline AttnClusters attn_clusters(unsigned sms, unsigned KVH, unsigned REP, unsigned dh, unsigned elem_bytes, unsigned allow, unsigned nsplit) {
