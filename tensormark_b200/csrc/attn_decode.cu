@@ -554,7 +554,9 @@ bool launch_stream(dim3 grid, cudaStream_t st, const float* q, const T* kc, cons
                    unsigned allow, unsigned chunk, float scale, const int* state) {
     auto* kernel = attn_stream_kernel<T, DH, REP, false>;
     static PerDevice<bool> ready;
-    if (!ready.get(current_device(), [=](bool&) {
+    const int dev = current_device();
+    if (dev < 0 || dev >= kMaxDevices) return fail("attention: no current CUDA device");
+    if (!ready.get(dev, [=](bool&) {
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Split<REP>::Smem);
             return e == cudaSuccess || fail("attention: shared memory attribute: %s", cudaGetErrorString(e));
         })) return false;

@@ -118,7 +118,7 @@ def test_attention_sets_function_attributes_on_each_device():
     statics = re.findall(r"static\s+const\s[^;]*?=[^;]*", text)
     assert not [s for s in statics if re.search(r"cudaFuncSet|cudaOccupancy|Fits", s)]
     for at in (m.start() for m in re.finditer(r"cudaFuncSetAttribute\(", text)):
-        assert ".get(current_device()," in text[max(0, at - 400):at]
+        assert re.search(r"\.get\((current_device\(\)|dev),", text[max(0, at - 400):at])
 
 
 @pytest.mark.parametrize("dt", [synth.Q4_0, synth.Q5_K])
